@@ -335,7 +335,9 @@ void prof_collect(mdgb_engine* e) {
 
 int pre_grid(const mdgb_engine* e) {
     const int maxg = std::min(4096, std::max(1, e->num_sms * e->pre_blocks_per_sm));  // bsum holds 4096
-    const int want = std::max({e->ntiles, (e->ncells + 1023) / 1024, (e->nrep + TILE - 1) / TILE, 1});
+    // reference order: one block per serial fold (six a replica at most)
+    const int folds = e->dev.refmode ? 6 * std::min(e->nrep, maxg) : 1;
+    const int want = std::max({e->ntiles, (e->ncells + 1023) / 1024, (e->nrep + TILE - 1) / TILE, folds});
     return std::min(maxg, want);
 }
 
@@ -1187,7 +1189,7 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
             (rc = dalloc(e, &d.cell_count, ncells)) ||
             (rc = dalloc(e, &d.cell_start, ncells + 1)) || (rc = dalloc(e, &d.cell_rep, ncells)) ||
             (rc = dalloc(e, &d.perm, N)) || (rc = dalloc(e, &d.tmp_pos, N)) ||
-            (rc = dalloc(e, &d.tmp_d, 8 * (size_t)N)) || (rc = dalloc(e, &d.tmp_i, 4 * (size_t)N)) ||
+            (rc = dalloc(e, &d.tmp_d, 8 * ((size_t)N + (d.refmode ? (size_t)SS_PAD * nrep : 0)))) || (rc = dalloc(e, &d.tmp_i, 4 * (size_t)N)) ||
             (rc = dalloc(e, &d.slot_of_rank, N)) || (rc = dalloc(e, &d.bsum, 4096)) ||
             (rc = dalloc(e, &d.lmask, 27 * (size_t)N)) || (rc = dalloc(e, &d.nbs, 27 * (size_t)ncells)) ||
             (rc = dalloc(e, &d.rb, 4 + 3 * (size_t)nrep)) ||

@@ -709,40 +709,268 @@ __device__ void phase_finalize_nh(const Dev& d, const StepParams& sp, int sel) {
     }
 }
 
-// Reference-order reductions: one thread per replica walks the atoms of type
-// `sel` in the reference's order and sums serially, exactly as the iterator
-// folds of macro_parameters/*.rs do.
-__device__ void phase_serial(const Dev& d, const StepParams& sp, int sel, bool coupling, bool nh_after_kick = false) {
+// ---------------------------------------------------------------------------
+// Reference-order reductions: the sums of macro_parameters/*.rs are serial
+// folds in the reference's atom order, s = RN(s + x_k), and keep its bits.
+//
+// A fold is cut into segments and every segment is run ahead of its turn, with
+// real FP64 additions, from an approximate start (a tree prefix sum).  Let the
+// true start be S, the simulated one Z, D = S - Z, and u the unit in the last
+// place of the largest binade the segment's running values reach.  When D is
+// a multiple of 2u and every running value of the simulation stays further
+// than |D| from a power of two, both runs round every addition alike (the
+// exact sums differ by a multiple of twice the rounding unit, so even ties go
+// the same way): the true end is the simulated end + D.  So a segment is run
+// once for each residue of S modulo 2u (S is a multiple of its own unit: 2
+// residues where the segment stays in S's binade, 4 or 8 where it climbs one
+// or two), and the segments are then stitched together one after the other in
+// integer arithmetic on the bit patterns.  A segment that climbs further, or
+// that comes too close to a power of two, is added term by term; so is
+// nothing else, whatever the values (a start that was exactly right is always
+// taken over).
+//
+// GB300's FP64 add takes 64 cycles of its scheduler's pipe, so one thread that
+// folds n terms needs n times that at the least; here 128 threads add at a
+// time, and the terms are computed and laid out by the whole grid before.
+// Against one thread per replica walking its atoms: a Berendsen T and P step
+// of 1,000 atoms 1.85 -> 0.13 ms, a frame of 111,360 atoms with its macro
+// parameters 188 -> 8.2 ms.
+constexpr int SS_SEGS = TILE;       // segments a round: one per thread
+constexpr int SS_KMAX = 8;          // residues a segment is run for at most
+constexpr long long SS_NEAR = 1ll << 30;   // |D| and distance to a power of two, in units
+
+// Terms per segment of a fold of n terms, and where term k lies in scratch:
+// rounds of SS_SEGS segments, inside a round [position][segment], so that a
+// round's threads read side by side.
+__host__ __device__ __forceinline__ int ss_len(long long n) {
+    const long long want = (n + SS_SEGS - 1) / SS_SEGS;
+    return want < 8 ? 8 : want > SS_PAD ? SS_PAD : (int)want;
+}
+__device__ __forceinline__ long long ss_place(long long k, long long n) {
+    const int len = ss_len(n);
+    const long long round = k / (SS_SEGS * len), base = round * (SS_SEGS * len);
+    const long long left = n - base;
+    const int segs = left >= SS_SEGS * len ? SS_SEGS : (int)((left + len - 1) / len);
+    const int i = (int)(k - base);
+    return base + (long long)(i % len) * segs + i / len;
+}
+
+struct SegRun {
+    long long base;       // bits of the simulated start, its low residue bits cleared
+    int mask;             // residues - 1
+    int ok;               // usable from a start that differs from the simulated one
+    int shift;            // exponent of the end - of the start
+    int deep;             // exponent of the start - smallest exponent reached
+    int flip;             // the sign changed on the way
+};
+
+// t + x_0 + x_1 + ... over one segment; lo/hi: smallest and largest exponent
+// field of the running values, near: one came within SS_NEAR units of a power
+// of two (or is zero, subnormal or not finite).
+template <bool LOOK>
+__device__ __forceinline__ double ss_run(const double* x, double c, int cnt, int stride, double t, int& lo, int& hi,
+                                         bool& near) {
+#pragma unroll 8
+    for (int q = 0; q < cnt; ++q) {
+        const double v = x ? __ldcg(x + (size_t)q * stride) : c;
+        t = __dadd_rn(t, v);
+        if (LOOK) {
+            const unsigned long long b = (unsigned long long)__double_as_longlong(t);
+            const int e = (int)((b >> 52) & 0x7FFull);
+            const long long f = (long long)(b & 0x000FFFFFFFFFFFFFull);
+            near |= e == 0 || e == 0x7FF || f <= SS_NEAR || f >= (1ll << 52) - SS_NEAR;
+            lo = min(lo, e);
+            hi = max(hi, e);
+        }
+    }
+    return t;
+}
+
+// ((0 + x_0) + x_1) + ... + x_(n-1), every addition rounded to nearest, by one
+// block of SS_SEGS threads; x in the ss_place order, or null: every term is c.
+// The result is valid in thread 0.
+__device__ double serial_sum(const double* x, long long n, double c) {
+    __shared__ SegRun seg[SS_SEGS];
+    __shared__ long long ends[SS_KMAX][SS_SEGS];   // bits of the simulated ends, by residue
+    __shared__ double wsum[SS_SEGS / 32], s_sum;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int len = ss_len(n);
+    if (tid == 0) s_sum = 0.0;
+    for (long long base = 0; base < n; base += SS_SEGS * len) {
+        const long long left = n - base;
+        const int segs = left >= SS_SEGS * len ? SS_SEGS : (int)((left + len - 1) / len);
+        const int cnt = (int)max(0ll, min((long long)len, left - (long long)tid * len));
+        const double* xs = x ? x + base + tid : nullptr;
+        int lo = 0x7FF, hi = 0;
+        bool near = false;
+        // approximate starts: the sum so far plus a tree prefix of the segments' own sums
+        double own = ss_run<false>(xs, c, cnt, segs, 0.0, lo, hi, near), incl = own;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const double y = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl = __dadd_rn(incl, y);
+        }
+        if (lane == 31) wsum[w] = incl;
+        __syncthreads();
+        double z = s_sum;
+        for (int k = 0; k < w; ++k) z = __dadd_rn(z, wsum[k]);
+        const double before = __shfl_up_sync(0xffffffffu, incl, 1);
+        if (lane) z = __dadd_rn(z, before);
+        // the runs
+        const double end = ss_run<true>(xs, c, cnt, segs, z, lo, hi, near);
+        const long long zb = __double_as_longlong(z), eb = __double_as_longlong(end);
+        const int ez = (int)((zb >> 52) & 0x7FF);
+        SegRun r;
+        const int climb = hi - ez + 1;       // log2 of the residues (0 or less: one)
+        r.ok = !near && ez > 0 && ez < 0x7FF && climb <= 3;
+        r.mask = r.ok && climb > 0 ? (1 << climb) - 1 : 0;
+        r.base = zb & ~(long long)r.mask;
+        r.shift = (int)((eb >> 52) & 0x7FF) - ez;
+        r.deep = max(0, ez - lo);
+        r.flip = (int)((unsigned long long)(zb ^ eb) >> 63);
+        ends[zb & r.mask][tid] = eb;
+        for (int j = 0; j <= r.mask; ++j)
+            if (j != (int)(zb & r.mask))
+                ends[j][tid] = __double_as_longlong(
+                    ss_run<false>(xs, c, cnt, segs, __longlong_as_double(r.base | j), lo, hi, near));
+        seg[tid] = r;
+        __syncthreads();
+        // the stitching
+        if (tid == 0) {
+            long long sb = __double_as_longlong(s_sum);
+            for (int g = 0; g < segs; ++g) {
+                const SegRun q = seg[g];
+                const int j = (int)(sb & q.mask);
+                const long long e = ends[j][g], dl = sb - (q.base | j);
+                if (dl == 0) {
+                    sb = e;
+                } else if (q.ok && (sb >> 52) == (q.base >> 52) && q.deep < 24 &&
+                           (dl < 0 ? -dl : dl) < (SS_NEAR >> q.deep)) {
+                    // same sign and exponent: dl is |S| - |Z| in units of S
+                    const long long du = q.flip ? -dl : dl;
+                    sb = e + (q.shift >= 0 ? du >> q.shift : du << -q.shift);
+                } else {
+                    const int m = (int)min((long long)len, left - (long long)g * len);
+                    sb = __double_as_longlong(ss_run<false>(x ? x + base + g : nullptr, c, m, segs,
+                                                            __longlong_as_double(sb), lo, hi, near));
+                }
+            }
+            s_sum = __longlong_as_double(sb);
+        }
+        __syncthreads();
+    }
+    return s_sum;
+}
+
+// Scratch row f of replica r (in the rebuild's tmp_d, which a reference-order
+// engine allocates with SS_PAD more per row and replica).
+__device__ __forceinline__ double* ss_row(const Dev& d, int f, int r, long long begin) {
+    return d.tmp_d + (size_t)f * ((size_t)d.ntot + (size_t)SS_PAD * d.nrep) + begin + (long long)SS_PAD * r;
+}
+
+// The folds' terms, in the reference's order (by rank), into the scratch rows.
+// Pass 1, rows 0-4: v m (3), kinetic energy, potential.
+__device__ void phase_serial_terms1(const Dev& d, int sel, bool coupling) {
+    const int N = d.ntot;
+    const double m = d.mass[sel];
+    for (int t = blockIdx.x; t < d.ntiles; t += gridDim.x) {
+        const int4 tl = d.tiles[t];
+        const RepDev& R = tile_rep(d, tl.x);
+        const int i = tl.y + threadIdx.x;
+        const long long k = i - R.begin - R.type_off[sel], n = R.type_off[sel + 1] - R.type_off[sel];
+        if ((int)threadIdx.x >= tl.z || k < 0 || k >= n) continue;
+        int s = __ldcg(d.slot_of_rank + i);
+        if (s < 0 || s >= N) { atomicOr(d.err, E_BOUNDS); s = i; }
+        const double vx = __ldcg(d.vel + s), vy = __ldcg(d.vel + N + s), vz = __ldcg(d.vel + 2 * N + s);
+        const long long at = ss_place(k, n);
+        ss_row(d, 0, tl.x, R.begin)[at] = vx * m;                                                  // mod.rs:12-25
+        ss_row(d, 1, tl.x, R.begin)[at] = vy * m;
+        ss_row(d, 2, tl.x, R.begin)[at] = vz * m;
+        if (coupling) continue;
+        ss_row(d, 3, tl.x, R.begin)[at] = m * (vx * vx + vy * vy + vz * vz) / 2.0;                 // energy.rs:14-22
+        ss_row(d, 4, tl.x, R.begin)[at] = __ldcg(d.epot + s);                                      // energy.rs:40-49
+    }
+}
+
+// Centre-of-mass velocity of replica r from the pass-1 folds.
+__device__ __forceinline__ void serial_vcm(const Dev& d, const RepDev& R, double vc[3]) {
+    const double* S = d.part + (size_t)R.tile_begin * 8;
+    const double sw = __ldcg(S + 3);
+    for (int a = 0; a < 3; ++a) vc[a] = __ldcg(S + a) / sw;
+}
+
+// Pass 2: row 0 thermal energy, rows 1-3 (as one) the pressure's three terms
+// of every atom, row 4 the negated virial.
+__device__ void phase_serial_terms2(const Dev& d, int sel) {
+    const int N = d.ntot;
+    const double m = d.mass[sel];
+    __shared__ double vc[3];
+    int vc_rep = -1;                  // replica vc[] belongs to (block-uniform)
+    for (int t = blockIdx.x; t < d.ntiles; t += gridDim.x) {
+        const int4 tl = d.tiles[t];
+        const RepDev& R = tile_rep(d, tl.x);
+        if (tl.x != vc_rep) {
+            __syncthreads();
+            if (threadIdx.x == 0) serial_vcm(d, R, vc);
+            __syncthreads();
+            vc_rep = tl.x;
+        }
+        const int i = tl.y + threadIdx.x;
+        const long long k = i - R.begin - R.type_off[sel], n = R.type_off[sel + 1] - R.type_off[sel];
+        if ((int)threadIdx.x >= tl.z || k < 0 || k >= n) continue;
+        int s = __ldcg(d.slot_of_rank + i);
+        if (s < 0 || s >= N) { atomicOr(d.err, E_BOUNDS); s = i; }
+        const double dx = __ldcg(d.vel + s) - vc[0], dy = __ldcg(d.vel + N + s) - vc[1],
+                     dz = __ldcg(d.vel + 2 * N + s) - vc[2];
+        const long long at = ss_place(k, n);
+        ss_row(d, 0, tl.x, R.begin)[at] = m * (dx * dx + dy * dy + dz * dz) / 2.0;                 // energy.rs:25-37
+        double* r1 = ss_row(d, 1, 3 * tl.x, 3 * R.begin);                                          // pressure.rs:13-18
+        r1[ss_place(3 * k, 3 * n)] = m * dx * dx;
+        r1[ss_place(3 * k + 1, 3 * n)] = m * dy * dy;
+        r1[ss_place(3 * k + 2, 3 * n)] = m * dz * dz;
+        ss_row(d, 4, tl.x, R.begin)[at] = -__ldcg(d.evir + s);
+    }
+}
+
+// One block per fold.  Pass 1 folds land in the replica's
+// first row of d.part (three momentum components, mass, kinetic energy,
+// potential), pass 2 folds in its first row of d.cpart (thermal energy, the
+// pressure's kinetic and virial sums).  Only the folds somebody reads run:
+// a coupled step needs neither energy, and the pressure only with a barostat.
+__device__ void phase_serial_folds(const Dev& d, int sel, int pass, bool coupling, bool nh_after_kick) {
+    const int nf = pass == 1 ? (coupling || nh_after_kick ? 4 : 6) : (nh_after_kick ? 1 : 3);
+    for (int w = blockIdx.x; w < d.nrep * nf; w += gridDim.x) {
+        const int r = w / nf, f = w % nf;
+        const RepDev* R = d.rep + r;
+        if (pass == 2 && f > 0 && coupling && !__ldcg(&R->baro_on)) continue;
+        const long long b = __ldcg(&R->begin);
+        const long long n = __ldcg(&R->type_off[sel + 1]) - __ldcg(&R->type_off[sel]);
+        const double* x;
+        if (pass == 1) x = f == 3 ? nullptr : ss_row(d, f < 3 ? f : f - 1, r, b);
+        else x = f == 0 ? ss_row(d, 0, r, b) : f == 1 ? ss_row(d, 1, 3 * r, 3 * b) : ss_row(d, 4, r, b);
+        const double s = serial_sum(x, pass == 2 && f == 1 ? 3 * n : n, 1.0 * d.mass[sel]);
+        if (threadIdx.x == 0)
+            (pass == 1 ? d.part + (size_t)__ldcg(&R->tile_begin) * 8
+                       : d.cpart + (size_t)__ldcg(&R->chunk_begin) * 8)[f] = s;
+        __syncthreads();
+    }
+}
+
+// What the folds give, per replica: the macro parameters (k_macro), or T, P
+// and the coupling factors, or (nh_after_kick) the second psi update.
+__device__ void phase_serial_finalize(const Dev& d, const StepParams& sp, int sel, bool coupling, bool nh_after_kick) {
     const int gt = blockIdx.x * blockDim.x + threadIdx.x;
     const int nt = gridDim.x * blockDim.x;
-    const int N = d.ntot;
     for (int r = gt; r < d.nrep; r += nt) {
         const RepDev R = load_rep(d.rep + r);
         RepDev* W = d.rep + r;
-        const long long b = R.begin + R.type_off[sel], e = R.begin + R.type_off[sel + 1];
-        const double m = d.mass[sel];
-        double sx = 0, sy = 0, sz = 0, sw = 0, ke = 0, pe = 0;
-        for (long long k = b; k < e; ++k) {
-            const int s = __ldcg(d.slot_of_rank + k);
-            if (s < 0 || s >= N) { atomicOr(d.err, E_BOUNDS); continue; }
-            const double vx = __ldcg(d.vel + s), vy = __ldcg(d.vel + N + s), vz = __ldcg(d.vel + 2 * N + s);
-            sx += vx * m; sy += vy * m; sz += vz * m; sw += 1.0 * m;   // mod.rs:12-25
-            ke += m * (vx * vx + vy * vy + vz * vz) / 2.0;              // energy.rs:14-22
-            pe += __ldcg(d.epot + s);                                    // energy.rs:40-49
-        }
-        const double vc[3] = {sx / sw, sy / sw, sz / sw};
-        double th = 0, r1 = 0, r2 = 0;
-        for (long long k = b; k < e; ++k) {
-            const int s = __ldcg(d.slot_of_rank + k);
-            if (s < 0 || s >= N) continue;
-            const double dx = __ldcg(d.vel + s) - vc[0], dy = __ldcg(d.vel + N + s) - vc[1],
-                         dz = __ldcg(d.vel + 2 * N + s) - vc[2];
-            th += m * (dx * dx + dy * dy + dz * dz) / 2.0;             // energy.rs:25-37
-            r1 += m * dx * dx; r1 += m * dy * dy; r1 += m * dz * dz;   // pressure.rs:13-18
-            r2 -= __ldcg(d.evir + s);
-        }
+        const double* A = d.part + (size_t)R.tile_begin * 8;
+        const double* B = d.cpart + (size_t)R.chunk_begin * 8;
+        const long long n = R.type_off[sel + 1] - R.type_off[sel];
+        const double th = __ldcg(B);
+        const double T = temperature_of(th, n);
         if (nh_after_kick) {
-            nh_update_psi(W, R, temperature_of(th, e - b), sp.dt);
+            nh_update_psi(W, R, T, sp.dt);
             continue;
         }
         double box[3] = {R.box[0], R.box[1], R.box[2]};
@@ -751,25 +979,41 @@ __device__ void phase_serial(const Dev& d, const StepParams& sp, int sel, bool c
                 for (int a = 0; a < 3; ++a) box[a] *= R.pending;
             for (int a = 0; a < 3; ++a) { W->box[a] = box[a]; W->cs[a] = box[a] / (double)R.nc[a]; }
         }
-        const double volume = box[0] * box[1] * box[2];
-        const double T = temperature_of(th, e - b);
-        const double P = (r1 + r2 * 0.5) / volume / 3.0;
-        W->vcm[0] = vc[0]; W->vcm[1] = vc[1]; W->vcm[2] = vc[2];
-        W->mom[0] = sx; W->mom[1] = sy; W->mom[2] = sz;
-        W->msum = sw; W->ke = ke; W->pe = pe / 2.0; W->thermal = th; W->virsum = -r2;
-        W->count = e - b; W->T = T; W->P = P;
+        double P = 0.0;
+        if (!coupling || R.baro_on) {
+            const double volume = box[0] * box[1] * box[2];
+            P = (__ldcg(B + 1) + __ldcg(B + 2) * 0.5) / volume / 3.0;
+            W->virsum = -__ldcg(B + 2);
+            W->P = P;
+        }
+        serial_vcm(d, R, W->vcm);
+        for (int a = 0; a < 3; ++a) W->mom[a] = __ldcg(A + a);
+        W->msum = __ldcg(A + 3);
+        if (!coupling) { W->ke = __ldcg(A + 4); W->pe = __ldcg(A + 5) / 2.0; }
+        W->thermal = th; W->count = n; W->T = T;
         if (coupling) coupling_factors(W, R, T, P, sp.dt);
     }
+}
+
+// Returns true when the launch must stop.
+__device__ bool phase_serial(const Dev& d, const StepParams& sp, int sel, bool coupling, bool nh_after_kick = false) {
+    phase_serial_terms1(d, sel, coupling || nh_after_kick);
+    if (grid_barrier(d)) return true;
+    phase_serial_folds(d, sel, 1, coupling, nh_after_kick);
+    if (grid_barrier(d)) return true;
+    phase_serial_terms2(d, sel);
+    if (grid_barrier(d)) return true;
+    phase_serial_folds(d, sel, 2, coupling, nh_after_kick);
+    if (grid_barrier(d)) return true;
+    phase_serial_finalize(d, sp, sel, coupling, nh_after_kick);
+    return false;
 }
 
 // psi += psi_dot(T_t) * dt/2 with T_t the temperature of the atoms of type t
 // (thermostat.rs:35-39 before the kick, :59-65 after it), per replica with a
 // Nose-Hoover thermostat.  Returns true when the launch must stop.
 __device__ __forceinline__ bool nh_psi_of_type(const Dev& d, const StepParams& sp, int t) {
-    if (d.refmode) {
-        phase_serial(d, sp, t, false, true);
-        return grid_barrier(d);
-    }
+    if (d.refmode) return phase_serial(d, sp, t, false, true) || grid_barrier(d);
     phase_partials1(d, t);
     if (grid_barrier(d)) return true;
     phase_chunk_sums<7>(d);
@@ -1546,7 +1790,7 @@ __global__ void __launch_bounds__(TILE, 6) k_pre(Dev d, StepParams sp) {
             for (int t = 0; t < sel; ++t)
                 if (nh_psi_of_type(d, sp, t)) return;
         if (d.refmode) {
-            phase_serial(d, sp, sel, true);
+            if (phase_serial(d, sp, sel, true)) return;
             if (grid_barrier(d)) return;
         } else if (d.mixed && d.ntot >= FX_MIN_ATOMS) {
             phase_partials_fx(d, sel);
@@ -1637,7 +1881,8 @@ __device__ __forceinline__ void k_pre_rebuild(const Dev& d, const StepParams& sp
 
 // Macro parameters of type `sel` (solver/src/macro_parameters): results land
 // in the replica records (vcm, mom, ke, pe, thermal, T, P, count).
-__global__ void __launch_bounds__(TILE) k_macro(Dev d, StepParams sp, int sel) {
+// 6 blocks per SM, as k_pre: the engine launches both on one grid size.
+__global__ void __launch_bounds__(TILE, 6) k_macro(Dev d, StepParams sp, int sel) {
     barrier_setup(sp);
     tile_rep_reset();
     if (d.refmode) {

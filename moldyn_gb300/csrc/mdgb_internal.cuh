@@ -37,6 +37,7 @@ constexpr int IDX_BITS = 27;
 constexpr uint32_t IDX_MASK = (1u << IDX_BITS) - 1u;
 constexpr int CODE_ZERO = 13;  // (0,0,0)
 constexpr int CHUNK_TILES = 256;  // tiles per reduction chunk
+constexpr int SS_PAD = 64;        // longest segment of a reference-order fold: padding of its scratch rows
 
 // error bits (device word, read by the host after each chunk)
 enum : int {
