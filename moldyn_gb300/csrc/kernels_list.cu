@@ -39,6 +39,7 @@
 // rlist (1 + 1e-5) -- far outside r_cut -- is listed on both sides or on
 // neither, where the direct build decides each side on its own.
 #include <algorithm>
+#include <type_traits>
 
 #include "mdgb_internal.cuh"
 
@@ -269,6 +270,65 @@ __global__ void __launch_bounds__(LM_WARPS * 32, 10) k_list_masks(Dev d) {
     }
 }
 
+// Lists of a reference-order engine into the reference's order (ascending
+// rank; one thread per atom there, so entry k of atom s lies rn words after
+// entry k - 1).  The warp takes its 32 atoms (lane = atom s0 + lane with n
+// entries) one after the other: lane l holds entries l, l + 32, ... of the
+// list, finds each one's place by counting the smaller keys, broadcast one
+// after the other, and stores it there.  An insertion sort per lane in global
+// memory took 1.5 ms for 6,912 atoms (a dependent load, rank gather and store
+// per move); this one is bound by its instructions (7 per key and round of
+// 32): a frame of 111,360 atoms 8.2 -> 5.0 ms, ten saved steps of 23,256 atoms
+// 9.4 -> 7.6 ms.  Lists of more than 128 entries keep the insertion sort.
+constexpr int SORT_PER_LANE = 4;
+
+__device__ __noinline__ void sort_lists_by_rank(const Dev& d, int s0, int n, long long rbeg, int rn) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    if (n > 32 * SORT_PER_LANE) sort_list_by_rank(d, s0 + lane, n, 1, rbeg, rn);
+    __syncwarp();   // the lists are written by the lane of their atom
+    unsigned todo = __ballot_sync(FULL, n > 1 && n <= 32 * SORT_PER_LANE);
+    while (todo) {
+        const int a = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        const int na = __shfl_sync(FULL, n, a);
+        uint32_t* list = d.nbr + list_index(s0 + a, 0, 1, rbeg, rn, d.cap);
+        uint32_t e[SORT_PER_LANE];
+        int key[SORT_PER_LANE], place[SORT_PER_LANE];
+#pragma unroll
+        for (int q = 0; q < SORT_PER_LANE; ++q) {
+            const int k = lane + 32 * q;
+            e[q] = k < na ? list[(size_t)k * rn] : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < SORT_PER_LANE; ++q) {
+            key[q] = lane + 32 * q < na ? __ldcg(d.rank + (e[q] & IDX_MASK)) : 0x7FFFFFFF;
+            place[q] = 0;
+        }
+        __syncwarp();   // every entry is read before any is stored
+        auto rounds = [&](auto nq_) {
+            constexpr int NQ = decltype(nq_)::value;
+#pragma unroll
+            for (int p = 0; p < NQ; ++p) {
+                const int m = min(32, na - 32 * p);
+                for (int k = 0; k < m; ++k) {
+                    const int other = __shfl_sync(FULL, key[p], k);
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) place[q] += other < key[q] ? 1 : 0;
+                }
+            }
+        };
+        if (na <= 32) rounds(std::integral_constant<int, 1>{});
+        else if (na <= 64) rounds(std::integral_constant<int, 2>{});
+        else if (na <= 96) rounds(std::integral_constant<int, 3>{});
+        else rounds(std::integral_constant<int, 4>{});
+#pragma unroll
+        for (int q = 0; q < SORT_PER_LANE; ++q)
+            if (lane + 32 * q < na) list[(size_t)place[q] * rn] = e[q];
+        __syncwarp();
+    }
+}
+
 // The direct build: every cell against the stream of its 27 neighbour cells.
 // all: every rebuilding replica (else those the paired build does not take).
 template <bool SINGLE>
@@ -449,13 +509,13 @@ __device__ __forceinline__ void list_direct(const Dev& d, uint32_t* lb_smem, boo
             }
             if (own) {
                 const int nfill = min(cnt, cap);
-                if (d.refmode) sort_list_by_rank(d, s, nfill, tpa, rbeg, rn);
                 d.nn[s] = nfill;
                 if (cnt > cap) {
                     atomicOr(d.err, E_NLIST);
                     atomicMax(d.max_needed, cnt);
                 }
             }
+            if (d.refmode) sort_lists_by_rank(d, ib + g, own ? min(cnt, cap) : 0, rbeg, rn);
             cmax = max(cmax, cnt);
         }
 #pragma unroll
@@ -557,13 +617,13 @@ __device__ __forceinline__ void list_expand(const Dev& d, uint32_t* lb_smem) {
             }
         }
         if (own) {
-            if (d.refmode) sort_list_by_rank(d, s, lim, tpa, rbeg, rn);
             d.nn[s] = lim;
             if (tot > cap) {
                 atomicOr(d.err, E_NLIST);
                 atomicMax(d.max_needed, tot);
             }
         }
+        if (d.refmode) sort_lists_by_rank(d, tl.y + sub, own ? lim : 0, rbeg, rn);
         int cmax = own ? tot : 0;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) cmax = max(cmax, __shfl_xor_sync(FULL, cmax, off));

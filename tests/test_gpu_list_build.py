@@ -135,3 +135,26 @@ def test_paired_build_ensemble_equals_direct(Engine):
     for k in FIELDS:
         assert np.array_equal(outs[0][k], outs[1][k]), k
     assert stats[0].direct_list_builds == 0 and stats[1].direct_list_builds > 0
+
+
+@pytest.mark.parametrize("rho,skin", [(0.1, 0.3), (0.3, 0.3), (0.8442, 0.05), (0.8442, 0.3), (0.8442, 0.55),
+                                      (0.8442, 0.8), (0.8442, 1.1)])
+@pytest.mark.parametrize("direct", [False, True])
+def test_reference_order_lists_of_every_length(Engine, oracle, rho, skin, direct):
+    """Lists of about 8, 25, 60, 78, 100, 127 and 165 entries sorted into the
+    reference's order (the sort takes up to 32, 64, 96 and 128 entries by
+    rounds of 32 and longer lists another way): the sums over them carry the
+    oracle's bits."""
+    pos, vel, box = gs.fcc((12, 12, 12) if rho > 0.5 else (9, 9, 9), rho=rho, jitter=0.05, seed=17)
+    perm = np.random.default_rng(3).permutation(len(pos))
+    pos, vel = pos[perm], vel[perm]
+    st = oracle.OracleState([len(pos)], pos, vel, [1.0], box, oracle.pot_table(1, default=(1.0, 1.0)))
+    st.update_force()
+    e = Engine(precision="fp64", reference_order=True, skin=skin, direct_list=direct)
+    e.set_potential(0, 0, 1.0, 1.0)
+    e.upload(np.zeros(len(pos), dtype=np.uint16), pos, vel, [1.0], box)
+    e.compute_forces()
+    out = e.download()
+    e.close()
+    assert np.array_equal(out["force"], st.force)
+    assert np.array_equal(out["potential"], st.potential) and np.array_equal(out["temp"], st.temp)
