@@ -717,24 +717,25 @@ __device__ void phase_finalize_nh(const Dev& d, const StepParams& sp, int sel) {
 // real FP64 additions, from an approximate start (a tree prefix sum).  Let the
 // true start be S, the simulated one Z, D = S - Z, and u the unit in the last
 // place of the largest binade the segment's running values reach.  When D is
-// a multiple of 2u and every running value of the simulation stays further
+// a multiple of u and every running value of the simulation stays further
 // than |D| from a power of two, both runs round every addition alike (the
-// exact sums differ by a multiple of twice the rounding unit, so even ties go
-// the same way): the true end is the simulated end + D.  So a segment is run
-// once for each residue of S modulo 2u (S is a multiple of its own unit: 2
-// residues where the segment stays in S's binade, 4 or 8 where it climbs one
-// or two), and the segments are then stitched together one after the other in
-// integer arithmetic on the bit patterns.  A segment that climbs further, or
-// that comes too close to a power of two, is added term by term; so is
-// nothing else, whatever the values (a start that was exactly right is always
-// taken over).
+// exact sums differ by a multiple of the rounding unit): the true end is the
+// simulated end + D.  Where a term may make a tie, D must be a multiple of 2u
+// (ties then go the same way).  So a segment is run once for each residue of
+// S modulo u or 2u (S is a multiple of its own unit: one residue, or two with
+// ties, where the segment stays in S's binade; 2, 4 or 8 where it climbs), and
+// the segments are then stitched together in integer arithmetic on the bit
+// patterns -- a run of segments that change neither binade nor sign as a
+// prefix sum, others one by one.  A segment that climbs further, or comes too
+// close to a power of two, is added term by term (a start that was exactly
+// right is always taken over).
 //
 // GB300's FP64 add takes 64 cycles of its scheduler's pipe, so one thread that
 // folds n terms needs n times that at the least; here 128 threads add at a
 // time, and the terms are computed and laid out by the whole grid before.
 // Against one thread per replica walking its atoms: a Berendsen T and P step
-// of 1,000 atoms 1.85 -> 0.13 ms, a frame of 111,360 atoms with its macro
-// parameters 188 -> 8.2 ms.
+// of 1,000 atoms 1.85 -> 0.10 ms, a frame of 111,360 atoms with its macro
+// parameters (the folds alone) 179 -> 1.2 ms.
 constexpr int SS_SEGS = TILE;       // segments a round: one per thread
 constexpr int SS_KMAX = 8;          // residues a segment is run for at most
 constexpr long long SS_NEAR = 1ll << 30;   // |D| and distance to a power of two, in units
@@ -744,7 +745,7 @@ constexpr long long SS_NEAR = 1ll << 30;   // |D| and distance to a power of two
 // round's threads read side by side.
 __host__ __device__ __forceinline__ int ss_len(long long n) {
     const long long want = (n + SS_SEGS - 1) / SS_SEGS;
-    return want < 8 ? 8 : want > SS_PAD ? SS_PAD : (int)want;
+    return want < 16 ? 16 : want > SS_PAD ? SS_PAD : (int)want;
 }
 __device__ __forceinline__ long long ss_place(long long k, long long n) {
     const int len = ss_len(n);
@@ -758,41 +759,75 @@ __device__ __forceinline__ long long ss_place(long long k, long long n) {
 struct SegRun {
     long long base;       // bits of the simulated start, its low residue bits cleared
     int mask;             // residues - 1
-    int ok;               // usable from a start that differs from the simulated one
+    int lim;              // |D| a start may differ by, in units of the start (0: not at all)
     int shift;            // exponent of the end - of the start
-    int deep;             // exponent of the start - smallest exponent reached
     int flip;             // the sign changed on the way
 };
 
-// t + x_0 + x_1 + ... over one segment; lo/hi: smallest and largest exponent
-// field of the running values, near: one came within SS_NEAR units of a power
-// of two (or is zero, subnormal or not finite).
+// t + x_0 + x_1 + ... over one segment.  LOOK: lo/hi the smallest and largest
+// exponent field of the running values; near: one came within SS_NEAR units of
+// a power of two (or is zero, subnormal or not finite); tie: an addition may
+// have been a tie -- its term has no bits below half the result's unit (t is
+// then a multiple of that half, too, unless the exponent jumped by two).
 template <bool LOOK>
 __device__ __forceinline__ double ss_run(const double* x, double c, int cnt, int stride, double t, int& lo, int& hi,
-                                         bool& near) {
-#pragma unroll 8
-    for (int q = 0; q < cnt; ++q) {
-        const double v = x ? __ldcg(x + (size_t)q * stride) : c;
-        t = __dadd_rn(t, v);
-        if (LOOK) {
-            const unsigned long long b = (unsigned long long)__double_as_longlong(t);
-            const int e = (int)((b >> 52) & 0x7FFull);
-            const long long f = (long long)(b & 0x000FFFFFFFFFFFFFull);
-            near |= e == 0 || e == 0x7FF || f <= SS_NEAR || f >= (1ll << 52) - SS_NEAR;
-            lo = min(lo, e);
-            hi = max(hi, e);
+                                         bool& near, bool& tie) {
+    int ep = LOOK ? (int)(((unsigned long long)__double_as_longlong(t) >> 52) & 0x7FFull) : 0;
+    // eight terms at a time, the next eight in flight (+ 0 past the end: no change)
+    double nx[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) nx[u] = u < cnt ? (x ? __ldcg(x + (size_t)u * stride) : c) : 0.0;
+    for (int q = 0; q < cnt; q += 8) {
+        double cur[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) cur[u] = nx[u];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int k = q + 8 + u;
+            nx[u] = k < cnt ? (x ? __ldcg(x + (size_t)k * stride) : c) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const double v = cur[u];
+            t = __dadd_rn(t, v);
+            if (LOOK) {
+                const unsigned long long b = (unsigned long long)__double_as_longlong(t);
+                const int e = (int)((b >> 52) & 0x7FFull);
+                const long long f = (long long)(b & 0x000FFFFFFFFFFFFFull);
+                near |= e == 0 || e == 0x7FF || f <= SS_NEAR || f >= (1ll << 52) - SS_NEAR;
+                lo = min(lo, e);
+                hi = max(hi, e);
+                const unsigned long long vb = (unsigned long long)__double_as_longlong(v) << 1;
+                const int r = e - (int)(vb >> 53);
+                tie |= vb != 0ull && (ep + 1 < e || r <= 1 || (r <= 54 && (vb << (64 - r)) == 0ull));
+                ep = e;
+            }
         }
     }
     return t;
 }
 
+// One segment taken over from the true start sb (bits); the sum's bits after it.
+__device__ __forceinline__ bool ss_take(const SegRun& q, long long end, long long sb, int j, long long& out) {
+    const long long dl = sb - (q.base | j);
+    if (dl == 0) { out = end; return true; }
+    if ((dl < 0 ? -dl : dl) >= q.lim || (sb >> 52) != (q.base >> 52)) return false;
+    // same sign and exponent: dl is |S| - |Z| in units of S
+    const long long du = q.flip ? -dl : dl;
+    out = end + (q.shift >= 0 ? du >> q.shift : du << -q.shift);
+    return true;
+}
+
 // ((0 + x_0) + x_1) + ... + x_(n-1), every addition rounded to nearest, by one
 // block of SS_SEGS threads; x in the ss_place order, or null: every term is c.
-// The result is valid in thread 0.
+// The result is valid in every thread.
 __device__ double serial_sum(const double* x, long long n, double c) {
     __shared__ SegRun seg[SS_SEGS];
     __shared__ long long ends[SS_KMAX][SS_SEGS];   // bits of the simulated ends, by residue
     __shared__ double wsum[SS_SEGS / 32], s_sum;
+    __shared__ int wruns[SS_SEGS / 32];
+    __shared__ unsigned short todo[SS_SEGS * (SS_KMAX - 1)];   // runs to do: segment and residue
+    const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int len = ss_len(n);
     if (tid == 0) s_sum = 0.0;
@@ -802,60 +837,98 @@ __device__ double serial_sum(const double* x, long long n, double c) {
         const int cnt = (int)max(0ll, min((long long)len, left - (long long)tid * len));
         const double* xs = x ? x + base + tid : nullptr;
         int lo = 0x7FF, hi = 0;
-        bool near = false;
+        bool near = false, tie = false;
         // approximate starts: the sum so far plus a tree prefix of the segments' own sums
-        double own = ss_run<false>(xs, c, cnt, segs, 0.0, lo, hi, near), incl = own;
+        double own = ss_run<false>(xs, c, cnt, segs, 0.0, lo, hi, near, tie), incl = own;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            const double y = __shfl_up_sync(0xffffffffu, incl, off);
+            const double y = __shfl_up_sync(FULL, incl, off);
             if (lane >= off) incl = __dadd_rn(incl, y);
         }
         if (lane == 31) wsum[w] = incl;
         __syncthreads();
         double z = s_sum;
         for (int k = 0; k < w; ++k) z = __dadd_rn(z, wsum[k]);
-        const double before = __shfl_up_sync(0xffffffffu, incl, 1);
+        const double before = __shfl_up_sync(FULL, incl, 1);
         if (lane) z = __dadd_rn(z, before);
         // the runs
-        const double end = ss_run<true>(xs, c, cnt, segs, z, lo, hi, near);
+        const double end = ss_run<true>(xs, c, cnt, segs, z, lo, hi, near, tie);
         const long long zb = __double_as_longlong(z), eb = __double_as_longlong(end);
         const int ez = (int)((zb >> 52) & 0x7FF);
         SegRun r;
-        const int climb = hi - ez + 1;       // log2 of the residues (0 or less: one)
-        r.ok = !near && ez > 0 && ez < 0x7FF && climb <= 3;
-        r.mask = r.ok && climb > 0 ? (1 << climb) - 1 : 0;
+        const int climb = hi - ez + (tie ? 1 : 0);       // log2 of the residues (0 or less: one)
+        const int deep = max(0, ez - lo);
+        const bool ok = !near && ez > 0 && ez < 0x7FF && climb <= 3 && deep < 24;
+        r.mask = ok && climb > 0 ? (1 << climb) - 1 : 0;
         r.base = zb & ~(long long)r.mask;
+        r.lim = ok ? (int)(SS_NEAR >> deep) : 0;
         r.shift = (int)((eb >> 52) & 0x7FF) - ez;
-        r.deep = max(0, ez - lo);
         r.flip = (int)((unsigned long long)(zb ^ eb) >> 63);
         ends[zb & r.mask][tid] = eb;
-        for (int j = 0; j <= r.mask; ++j)
-            if (j != (int)(zb & r.mask))
-                ends[j][tid] = __double_as_longlong(
-                    ss_run<false>(xs, c, cnt, segs, __longlong_as_double(r.base | j), lo, hi, near));
         seg[tid] = r;
+        // the other residues' runs, shared out over the block's threads
+        int at = r.mask;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int y = __shfl_up_sync(FULL, at, off);
+            if (lane >= off) at += y;
+        }
+        if (lane == 31) wruns[w] = at;
         __syncthreads();
-        // the stitching
-        if (tid == 0) {
+        int runs = 0;
+        for (int k = 0; k < SS_SEGS / 32; ++k) {
+            if (k < w) at += wruns[k];
+            runs += wruns[k];
+        }
+        for (int k = 1; k <= r.mask; ++k)
+            todo[at - k] = (unsigned short)(tid * SS_KMAX + ((int)(zb & r.mask) ^ k));
+        __syncthreads();
+        for (int k = tid; k < runs; k += SS_SEGS) {
+            const int g = todo[k] / SS_KMAX, j = todo[k] % SS_KMAX;
+            const int cg = (int)min((long long)len, left - (long long)g * len);
+            ends[j][g] = __double_as_longlong(ss_run<false>(x ? x + base + g : nullptr, c, cg, segs,
+                                                            __longlong_as_double(seg[g].base | j), lo, hi, near, tie));
+        }
+        __syncthreads();
+        // the stitching, by the first warp (every lane carries the sum)
+        if (w == 0) {
             long long sb = __double_as_longlong(s_sum);
-            for (int g = 0; g < segs; ++g) {
-                const SegRun q = seg[g];
-                const int j = (int)(sb & q.mask);
-                const long long e = ends[j][g], dl = sb - (q.base | j);
-                if (dl == 0) {
-                    sb = e;
-                } else if (q.ok && (sb >> 52) == (q.base >> 52) && q.deep < 24 &&
-                           (dl < 0 ? -dl : dl) < (SS_NEAR >> q.deep)) {
-                    // same sign and exponent: dl is |S| - |Z| in units of S
-                    const long long du = q.flip ? -dl : dl;
-                    sb = e + (q.shift >= 0 ? du >> q.shift : du << -q.shift);
-                } else {
-                    const int m = (int)min((long long)len, left - (long long)g * len);
-                    sb = __double_as_longlong(ss_run<false>(x ? x + base + g : nullptr, c, m, segs,
-                                                            __longlong_as_double(sb), lo, hi, near));
+            for (int g0 = 0; g0 < segs; g0 += 32) {
+                const SegRun q = seg[g0 + lane];
+                const bool plain = q.lim > 0 && q.mask == 0 && q.shift == 0 && !q.flip;
+                const long long gain = plain ? ends[0][g0 + lane] - q.base : 0;
+                const unsigned plains = __ballot_sync(FULL, plain);
+                const int m = min(32, segs - g0);
+                int f = 0;
+                while (f < m) {
+                    if (plains >> f & 1u) {
+                        // a run of plain segments from f on
+                        long long sum = lane >= f ? gain : 0;
+#pragma unroll
+                        for (int off = 1; off < 32; off <<= 1) {
+                            const long long y = __shfl_up_sync(FULL, sum, off);
+                            if (lane >= off) sum += y;
+                        }
+                        const long long start = sb + sum - (lane >= f ? gain : 0);
+                        long long out;
+                        const bool good = plain && ss_take(q, start + gain, start, 0, out);
+                        const unsigned stop = __ballot_sync(FULL, !good) & (0xFFFFFFFFu << f);
+                        const int g = stop ? min(__ffs(stop) - 1, m) : m;
+                        if (g > f) sb = __shfl_sync(FULL, start + gain, g - 1);
+                        f = g;
+                        if (f >= m) break;
+                    }
+                    const SegRun qf = seg[g0 + f];
+                    const int j = (int)(sb & qf.mask);
+                    if (!ss_take(qf, ends[j][g0 + f], sb, j, sb)) {
+                        const int cf = (int)min((long long)len, left - (long long)(g0 + f) * len);
+                        sb = __double_as_longlong(ss_run<false>(x ? x + base + g0 + f : nullptr, c, cf, segs,
+                                                                __longlong_as_double(sb), lo, hi, near, tie));
+                    }
+                    ++f;
                 }
             }
-            s_sum = __longlong_as_double(sb);
+            if (lane == 0) s_sum = __longlong_as_double(sb);
         }
         __syncthreads();
     }
