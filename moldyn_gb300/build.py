@@ -30,6 +30,7 @@ NVCC_COMMON = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-ff
 UNITS = [
     ("kernels_step.cu", ["-fmad=false"]),
     ("kernels_force.cu", []),
+    ("kernels_pairs.cu", []),
     ("kernels_list.cu", []),
     ("engine.cu", []),
     ("host_util.cpp", []),
@@ -45,7 +46,7 @@ def nvcc() -> str:
 
 def _sources():
     return [os.path.join(CSRC, u) for u, _ in UNITS] + [
-        os.path.join(CSRC, "mdgb_internal.cuh"), os.path.join(INCLUDE, "mdgb.h"), __file__]
+        os.path.join(CSRC, "mdgb_internal.cuh"), os.path.join(CSRC, "force_common.cuh"), os.path.join(INCLUDE, "mdgb.h"), __file__]
 
 
 def up_to_date() -> bool:

@@ -110,6 +110,8 @@ struct mdgb_engine {
     // allocations
     std::vector<void*> allocs;
     void* nbr_alloc = nullptr;
+    void* pair_alloc = nullptr;      // the FP64 path's pair records (Dev::pairs)
+    int pair_single = 0;             // Dev::single_type they were sized for
     // snapshot buffers (chunk retry)
     double4_32a* snap_pos = nullptr;
     double* snap_d = nullptr;   // [8][N]
@@ -202,6 +204,8 @@ void free_state(mdgb_engine* e) {
     for (void* p : e->allocs) cudaFree(p);
     e->allocs.clear();
     if (e->nbr_alloc) { cudaFree(e->nbr_alloc); e->nbr_alloc = nullptr; }
+    if (e->pair_alloc) { cudaFree(e->pair_alloc); e->pair_alloc = nullptr; }
+    e->dev.pairs = 0;
     e->dev.nn = nullptr;
     e->has_state = false;
     e->forces_valid = false;
@@ -259,6 +263,7 @@ std::vector<PairDev> pair_table(mdgb_engine* e) {
             q.rc2f_lo = (float)(rc2 * (1.0 - 1e-5));
             q.rc2f_hi = (float)(rc2 * (1.0 + 1e-5));
             q.rc2_cut = sqrt_cut(p.rc);
+            q.sig2 = p.sigma * p.sigma;
             tab[a * MAX_TYPES + b] = q;
             if (a < e->ntypes && b < e->ntypes) {
                 e->rcmax = std::max(e->rcmax, p.rc);
@@ -287,6 +292,48 @@ int upload_pairs(mdgb_engine* e) {
     return MDGB_OK;
 }
 
+// The FP64 path's pair records for the current list capacity.  From
+// PAIR_MIN_ATOMS atoms on the pairs are computed once (kernels_pairs.cu);
+// below, where a step is a few launches of latency, and with several threads
+// per atom, k_force_fp64 evaluates both sides.  About 4 KB an atom in a
+// liquid: where the device has no room for that (a tenth of its memory is
+// left to others), the records are left out as well.
+constexpr int PAIR_MIN_ATOMS = 4096;
+
+void alloc_pairs(mdgb_engine* e) {
+    Dev& d = e->dev;
+    d.pairs = 0;
+    e->pair_single = d.single_type;
+    if (e->pair_alloc) { cudaFree(e->pair_alloc); e->pair_alloc = nullptr; }
+    if (e->cfg.precision != MDGB_PRECISION_FP64 || e->ntot < PAIR_MIN_ATOMS || e->cfg.threads_per_atom > 1) return;
+    const size_t N = e->ntot, room = pair_room(N, d.cap, d.single_type);
+    if (room >= (size_t)PAIR_NEG) return;
+    // sizes in whole 256 bytes, so that every array starts aligned
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t s_rec = up(room * sizeof(PairRec)), s_ij = up(room * sizeof(uint2)),
+                 s_vir = up(room * sizeof(double)), s_of = up((size_t)d.cap * N * sizeof(uint32_t)), s_in = up(room),
+                 s_tile = up(e->ntiles * sizeof(int2)), s_cnt = up(e->nrep * sizeof(int));
+    const size_t total = s_rec + s_ij + s_vir + s_of + s_in + s_tile + s_cnt;
+    size_t free_b = 0, all_b = 0;
+    if (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess || total + all_b / 10 > free_b ||
+        cudaMalloc(&e->pair_alloc, total) != cudaSuccess) {
+        cudaGetLastError();
+        e->pair_alloc = nullptr;
+        return;
+    }
+    char* q = static_cast<char*>(e->pair_alloc);
+    d.pair_rec = reinterpret_cast<PairRec*>(q); q += s_rec;
+    d.pair_ij = reinterpret_cast<uint2*>(q); q += s_ij;
+    d.pair_vir = reinterpret_cast<double*>(q); q += s_vir;
+    d.pair_of = reinterpret_cast<uint32_t*>(q); q += s_of;
+    d.pair_in = reinterpret_cast<unsigned char*>(q); q += s_in;
+    d.pair_tile = reinterpret_cast<int2*>(q); q += s_tile;
+    d.pair_count = reinterpret_cast<int*>(q);
+    // no records until the next rebuild
+    cudaMemsetAsync(d.pair_tile, 0, s_tile + s_cnt, e->stream);
+    d.pairs = 1;
+}
+
 int alloc_nbr(mdgb_engine* e, int cap) {
     // the tpa-interleaved layout (nbr_index) needs cap to be a multiple of every tpa
     cap = std::max(8, (cap + 7) & ~7);
@@ -302,6 +349,7 @@ int alloc_nbr(mdgb_engine* e, int cap) {
     e->dev.cap = cap;
     e->cap = cap;
     e->lists_fresh = false;
+    alloc_pairs(e);
     return MDGB_OK;
 }
 
@@ -362,7 +410,7 @@ int launch_pre(mdgb_engine* e, const StepParams& sp) {
     }
     CU(launch_list_build(e->dev, e->lb_grid, e->lm_grid, e->stream));
     prof_end(e, pe);
-    e->st.kernel_launches += 3;
+    e->st.kernel_launches += e->dev.pairs ? 5 : 3;
     return MDGB_OK;
 }
 
@@ -403,9 +451,22 @@ int launch_force_class(mdgb_engine* e, const StepParams& sp, bool kick, int c, c
 int launch_force(mdgb_engine* e, const StepParams& sp_in, bool kick) {
     cudaEvent_t pe;
     prof_begin(e, 0, &pe);
-    if (e->cfg.flags & MDGB_FLAG_PERSISTENT)
+    if ((e->cfg.flags & MDGB_FLAG_PERSISTENT) && !e->dev.pairs)
         CU(cudaMemsetAsync(e->dev.queue, 0, mdgb_engine::NCLASS * sizeof(unsigned int), e->stream));
     const StepParams& sp = sp_in;
+    if (e->dev.pairs) {
+        Dev d = e->dev;
+        d.pos_next = e->pos_alt;
+        d.mir_next = e->mir_alt;
+        CU(launch_pair_forces(d, sp, kick, e->num_sms, e->stream));
+        e->st.kernel_launches += 2;
+        prof_end(e, pe);
+        if (kick && sp.fused) {
+            std::swap(e->dev.pos, e->pos_alt);
+            std::swap(e->dev.mir, e->mir_alt);
+        }
+        return MDGB_OK;
+    }
     band_fn bk = band_kernel(e->cfg.precision);
     if (bk) CU(cudaMemsetAsync(e->dev.band_count, 0, sizeof(int), e->stream));
     // classes touch disjoint atoms, tiles and queue counters: the second and
@@ -919,8 +980,8 @@ int autotune_skin(mdgb_engine* e, double dt) {
 int autotune_tpa(mdgb_engine* e) {
     e->tuned = true;
     const int NC = mdgb_engine::NCLASS;
-    if (e->dev.refmode || e->cfg.threads_per_atom > 0) {
-        const int t = e->dev.refmode ? 1 : e->cfg.threads_per_atom;
+    if (e->dev.refmode || e->dev.pairs || e->cfg.threads_per_atom > 0) {
+        const int t = e->dev.refmode || e->dev.pairs ? 1 : e->cfg.threads_per_atom;
         for (int c = 0; c < NC; ++c) e->class_tpa[c] = t;
         e->tpa = t;
         int rc = apply_class_tpa(e);
@@ -1217,6 +1278,8 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
     if (!e->nbr_alloc || cap > e->cap) {
         rc = alloc_nbr(e, cap);
         if (rc) return rc;
+    } else if (e->pair_single != d.single_type) {
+        alloc_pairs(e);   // as many records as list entries with several types
     }
     e->st = mdgb_stats{};
     e->st.neighbor_capacity = e->cap;

@@ -644,6 +644,7 @@ __global__ void __launch_bounds__(LB_WARPS * 32, 11) k_build_list(Dev d) {
     const bool direct = d.direct_list || *(volatile const unsigned int*)(d.bar + 4) != 0u;
     list_direct<SINGLE>(d, lb_smem, direct);
     if (!direct) list_expand(d, lb_smem);
+    if (d.pairs) return;   // k_pair_link closes the rebuild
     // The last block to finish closes the rebuild of every replica.
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -653,20 +654,7 @@ __global__ void __launch_bounds__(LB_WARPS * 32, 11) k_build_list(Dev d) {
     __syncthreads();
     if (s_last) {
         __threadfence();
-        for (int r = threadIdx.x; r < d.nrep; r += blockDim.x) {
-            RepDev* W = d.rep + r;
-            if (W->rebuild) {
-                W->rebuild = 0;
-                W->nrebuilds += 1;
-            }
-        }
-        if (threadIdx.x == 0) {
-            if (d.trace) atomicAdd(d.trace + TR_LIST, global_ns() - d.trace[TR_STAMP]);
-            if (direct) d.bar[5] += 1u;   // direct builds, for the engine's counters
-            d.bar[4] = 0u;
-            d.bar[3] = 0u;
-            atomicExch(d.bar + 2, 0u);
-        }
+        close_rebuild(d, direct);
     }
 }
 
@@ -706,7 +694,8 @@ cudaError_t launch_list_build(const Dev& d, int grid, int mgrid, cudaStream_t st
         k_list_masks<false><<<mgrid, LM_WARPS * 32, 0, st>>>(d);
         k_build_list<false><<<grid, LB_WARPS * 32, LB_SMEM, st>>>(d);
     }
-    return cudaGetLastError();
+    const cudaError_t err = cudaGetLastError();
+    return err != cudaSuccess || !d.pairs ? err : launch_pair_build(d, st);
 }
 
 }  // namespace mdgb

@@ -1,0 +1,444 @@
+// kernels_pairs.cu -- the FP64 path's force pass over pair records: every pair
+// computed once (update_force, solver/src/solver/potential.rs:158-216).
+//
+// GB300's FP64 pipe takes 64 cycles of a scheduler per warp instruction,
+// however few lanes are active, so k_force_fp64 (a thread per atom, both sides
+// of every pair, about 86 FP64 instructions each, lanes idle where a candidate
+// is outside r_cut) is bound by it.  Here a force pass is two kernels:
+//
+//   k_pair_terms  one thread per pair record: the pair's force, potential and
+//                 virial terms once, from the side of its owner.  Candidates
+//                 outside r_cut (FP32 prefilter) are dropped before the FP64
+//                 work: a warp queues what passes and computes 32 at a time.
+//   k_pair_sums   one thread per atom: walks its list in list order and adds
+//                 the records (the partner's with the force negated), then the
+//                 second half kick and, on NVE chunks, the next step's kick
+//                 and drift.
+//
+// r_ji = -r_ij, |r|, U and F . r are the same bits from either side, so the
+// per-atom sums are those of the one-sided loop, term by term and in the same
+// order; with MDGB_FLAG_REFERENCE_ORDER they stay bit-identical to the
+// reference.
+//
+// After every list build k_pair_rows gives each list entry its record -- the
+// entry of the atom that comes first in device order, or of the only atom that
+// lists the pair (several types) -- and k_pair_link finds the partner's entry
+// by binary search in its (ascending) list.  A pair listed by the later atom
+// only (within rounding of the list radius, far outside r_cut) has none.
+//
+// 256,000 atoms, one NVE pass: 3.66 ms with k_force_fp64; 0.42 + 0.23 ms in
+// tree order here, and 0.41 ms more at a rebuild (every ninth step).  23,256
+// atoms in reference order: 0.53 -> 0.18 ms.  k_pair_terms keeps the FP64 pipe
+// busy 82 % of the time; k_pair_sums waits for its record gathers (FP64 43 %).
+#include <algorithm>
+
+#include "force_common.cuh"
+
+namespace mdgb {
+
+// Atom i owns its entry for j: j lists the pair too and comes later, or does
+// not list it (the reference's t1 <= t2 loop, potential.rs:171-172).
+__device__ __forceinline__ bool pair_owned(const Dev& d, int i, int ti, int j) {
+    return j > i || (!d.single_type && type_of(__ldg(d.mir + j)) > ti);
+}
+
+// One block per tile: records for the tile's owned entries, numbered by a
+// warp's 32 atoms together -- list position by list position, so that stores
+// here, and the loads of a warp that walks its atoms' lists in k_pair_sums,
+// lie side by side.
+__global__ void __launch_bounds__(TILE) k_pair_rows(Dev d) {
+    if (*(volatile const unsigned int*)(d.bar + 2) == 0u) return;   // no rebuild this step
+    if (chunk_failed(d)) return;
+    __shared__ int wsum[TILE / 32];
+    __shared__ int s_base;
+    const unsigned FULL = 0xffffffffu;
+    const int4 tl = d.tiles[blockIdx.x];
+    const RepDev* R = d.rep + tl.x;
+    if (!R->rebuild) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long rbeg = R->begin;
+    const int rn = R->n;
+    const int s = tl.y + threadIdx.x;
+    const int n = (int)threadIdx.x < tl.z ? d.nn[s] : 0;
+    const int nmax = __reduce_max_sync(FULL, n);
+    const int ty = n ? type_of(d.mir[s]) : 0;
+    const size_t li = list_index(s, 0, 1, rbeg, rn, d.cap);
+    int own = 0;
+    for (int k = 0; k < n; ++k) {
+        const uint32_t e = d.nbr[li + (size_t)k * rn];
+        own += pair_owned(d, s, ty, (int)(e & IDX_MASK)) ? 1 : 0;
+    }
+    own = __reduce_add_sync(FULL, own);
+    if (lane == 0) wsum[w] = own;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int total = 0;
+        for (int k = 0; k < TILE / 32; ++k) { const int t = wsum[k]; wsum[k] = total; total += t; }
+        const int room = (int)pair_room(rn, d.cap, d.single_type);
+        const int first = (int)pair_room((size_t)rbeg, d.cap, d.single_type);
+        const int base = atomicAdd(d.pair_count + tl.x, total);
+        s_base = first + base;
+        if (base + total > room) {   // lists nearly full everywhere: a longer list makes room
+            atomicOr(d.err, E_NLIST);
+            atomicMax(d.max_needed, d.cap + 1);
+            total = 0;
+            s_base = -1;
+        }
+        d.pair_tile[blockIdx.x] = make_int2(max(s_base, 0), total);
+    }
+    __syncthreads();
+    const bool fits = s_base >= 0;
+    uint32_t rec = (uint32_t)(s_base + wsum[w]);
+    for (int k = 0; k < nmax; ++k) {
+        const uint32_t e = k < n ? d.nbr[li + (size_t)k * rn] : 0u;
+        const bool mine = fits && k < n && pair_owned(d, s, ty, (int)(e & IDX_MASK));
+        const unsigned got = __ballot_sync(FULL, mine);
+        const uint32_t at = rec + __popc(got & ((1u << lane) - 1u));
+        if (k < n) d.pair_of[li + (size_t)k * rn] = mine ? at : PAIR_NONE;
+        if (mine) d.pair_ij[at] = make_uint2((uint32_t)s, e);
+        rec += __popc(got);
+    }
+}
+
+// One thread per record: the partner's list entry of the pair, by binary
+// search -- by rank in the reference's order; else the lists ascend as 32-bit
+// words (shift code, then index) and the partner sees the pair at the opposite
+// code.  The last block closes the rebuild.
+__global__ void __launch_bounds__(TILE) k_pair_link(Dev d) {
+    if (*(volatile const unsigned int*)(d.bar + 2) == 0u) return;
+    if (chunk_failed(d)) return;
+    __shared__ int s_last;
+    for (int t = blockIdx.x; t < d.ntiles; t += gridDim.x) {
+        const int4 tl = d.tiles[t];
+        const RepDev* R = d.rep + tl.x;
+        if (!R->rebuild) continue;
+        const long long rbeg = R->begin;
+        const int rn = R->n;
+        const int2 pt = d.pair_tile[t];
+        for (int q = threadIdx.x; q < pt.y; q += blockDim.x) {
+            const uint2 ij = d.pair_ij[pt.x + q];
+            const int i = (int)ij.x, j = (int)(ij.y & IDX_MASK);
+            if (!d.single_type && type_of(__ldg(d.mir + j)) > type_of(__ldg(d.mir + i))) continue;
+            const size_t lj = list_index(j, 0, 1, rbeg, rn, d.cap);
+            const uint32_t want = (uint32_t)i | ((uint32_t)(26 - (int)(ij.y >> IDX_BITS)) << IDX_BITS);
+            const int ri = d.refmode ? d.rank[i] : 0;
+            int lo = 0, hi = d.nn[j];
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                const uint32_t e = __ldg(d.nbr + lj + (size_t)mid * rn);
+                if (d.refmode ? d.rank[e & IDX_MASK] < ri : e < want) lo = mid + 1; else hi = mid;
+            }
+            if (lo < d.nn[j] && (d.nbr[lj + (size_t)lo * rn] & IDX_MASK) == (uint32_t)i)
+                d.pair_of[lj + (size_t)lo * rn] = (uint32_t)(pt.x + q) | PAIR_NEG;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(d.bar + 3, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (s_last) {
+        __threadfence();
+        close_rebuild(d, d.direct_list || *(volatile const unsigned int*)(d.bar + 4) != 0u);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Pair terms.
+
+// The reference's operation sequence (potential.rs:57-75, :201-211) with the
+// library's square root and divisions.  False: |r| > r_cut.
+struct PairTerms {
+    double gx, gy, gz, u, t;
+};
+
+__device__ __noinline__ bool ref_terms_plain(double rx, double ry, double rz, double r2, const PairDev& P,
+                                             PairTerms& o) {
+    const double r = __dsqrt_rn(r2);
+    if (r > P.rc) return false;                                          // :202-204
+    const double sr = __ddiv_rn(P.sigma, r);
+    const double s2 = __dmul_rn(sr, sr);
+    const double s4 = __dmul_rn(s2, s2);
+    const double s6 = __dmul_rn(s2, s4);
+    const double s12 = __dmul_rn(s6, s6);
+    o.u = __dsub_rn(__dmul_rn(P.eps4, __dsub_rn(s12, s6)), P.ucut);
+    const double dudr = __dmul_rn(__ddiv_rn(P.eps24, r), __dsub_rn(s6, __dmul_rn(2.0, s12)));
+    o.gx = __dmul_rn(__ddiv_rn(rx, r), dudr);                            // :207-211
+    o.gy = __dmul_rn(__ddiv_rn(ry, r), dudr);
+    o.gz = __dmul_rn(__ddiv_rn(rz, r), dudr);
+    o.t = __dadd_rn(__dadd_rn(__dmul_rn(o.gx, rx), __dmul_rn(o.gy, ry)), __dmul_rn(o.gz, rz));
+    return true;
+}
+
+__device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7FF; }
+
+// An approximation of 1/sqrt(x) or 1/x to about 2^-22, from FP32; x in the
+// FP32 range.
+__device__ __forceinline__ double seed_rsqrt(double x) { return flt_to_dbl(rsqrtf(dbl_to_flt_rn(x))); }
+__device__ __forceinline__ double seed_rcp(double x) { return flt_to_dbl(__fdividef(1.0f, dbl_to_flt_rn(x))); }
+
+// a / r correctly rounded, from y = 1/r within half a unit in the last place
+// (and a rounding of 2^-104) and yl = 1/r - y: q0 is within half a unit plus
+// 2^-50 of the quotient, its remainder is exact, and one correction rounds
+// correctly (Markstein 1990: a quotient lies at least 2^-106 r^-1 from the
+// middle of two doubles, further than the correction's own error; the one
+// exception is an r within a few units below a power of two).
+__device__ __forceinline__ double div_by(double a, double r, double y, double yl) {
+    const double q0 = __fma_rn(a, y, __dmul_rn(a, yl));
+    return __fma_rn(__fma_rn(-r, q0, a), y, q0);
+}
+
+// The same terms, bit for bit, with one square root and one reciprocal for the
+// five divisions by r: 1/sqrt(r2) by Newton's iteration (third order, from the
+// FP32 seed), r from it by one correction step whose remainder is checked (a
+// correctly rounded root has -u r < r2 - r^2 <= u r, u its unit in the last
+// place), 1/r in two words, and div_by.  58 FP64 instructions against about 78
+// with the library's divisions.  Values outside a range that keeps every
+// intermediate normal take the plain form.
+// FORCE: only the force is wanted (50).
+template <bool FORCE>
+__device__ __forceinline__ bool ref_terms(double rx, double ry, double rz, double r2, const PairDev& P, PairTerms& o) {
+    const int e2 = exp_field(r2);
+    const auto tame = [](double x) { const int e = exp_field(x); return e > 1023 - 400 || x == 0.0; };
+    bool ok = e2 > 1023 - 100 && e2 < 1023 + 100;
+    ok = ok && tame(rx) && tame(ry) && tame(rz);
+    double r = 0.0, y = 0.0;
+    if (ok) {
+        // r2 is below r_cut^2 exactly when its rounded root is at most r_cut
+        if (__double_as_longlong(r2) >= __double_as_longlong(P.rc2_cut)) return false;
+        const double y0 = seed_rsqrt(r2);
+        const double e = __fma_rn(-__dmul_rn(r2, y0), y0, 1.0);
+        y = __fma_rn(__dmul_rn(y0, e), __fma_rn(0.375, e, 0.5), y0);
+        const double g = __dmul_rn(r2, y);
+        const double h = __longlong_as_double(__double_as_longlong(y) - (1ll << 52));   // y / 2
+        r = __fma_rn(__fma_rn(-g, g, r2), h, g);
+        const double rem = __fma_rn(-r, r, r2);
+        const long long rb = __double_as_longlong(rem), mag = rb & 0x7FFFFFFFFFFFFFFFll;
+        // bits of u r, u = 2^(exponent of r - 52)
+        const long long lim = __double_as_longlong(r) + ((long long)(exp_field(r) - 1023 - 52) << 52);
+        ok = mag < lim || rb == lim;
+        // 1/r of an r just below a power of two does not round from y
+        ok = ok && (__double_as_longlong(r) & 0xFFFFFFFFFFFFFll) < 0xFFFFFFFFFFF00ll;
+    }
+    if (!ok) return ref_terms_plain(rx, ry, rz, r2, P, o);
+    y = __fma_rn(__fma_rn(-r, y, 1.0), y, y);
+    const double yl = __dmul_rn(__fma_rn(-r, y, 1.0), y);
+    const double sr = div_by(P.sigma, r, y, yl);
+    const double s2 = __dmul_rn(sr, sr);
+    const double s4 = __dmul_rn(s2, s2);
+    const double s6 = __dmul_rn(s2, s4);
+    const double s12 = __dmul_rn(s6, s6);
+    if (!FORCE) o.u = __dsub_rn(__dmul_rn(P.eps4, __dsub_rn(s12, s6)), P.ucut);
+    const double dudr = __dmul_rn(div_by(P.eps24, r, y, yl), __fma_rn(-2.0, s12, s6));   // 2 s12 is exact
+    o.gx = __dmul_rn(div_by(rx, r, y, yl), dudr);
+    o.gy = __dmul_rn(div_by(ry, r, y, yl), dudr);
+    o.gz = __dmul_rn(div_by(rz, r, y, yl), dudr);
+    if (!FORCE)
+        o.t = __dadd_rn(__dadd_rn(__dmul_rn(o.gx, rx), __dmul_rn(o.gy, ry)), __dmul_rn(o.gz, rz));
+    return true;
+}
+
+// Tree order (no MDGB_FLAG_REFERENCE_ORDER): the same functions of r^2 without
+// the root and the divisions by r -- sigma^2 / r^2 by one Newton step, F . r =
+// r dU/dr -- 24 FP64 instructions, 21 for the force alone.  Fewer roundings than the reference's form
+// ((sigma / r)^6 carries six times the rounding of r and of the quotient).
+template <bool FORCE>
+__device__ __forceinline__ bool r2_terms(double rx, double ry, double rz, double r2, const PairDev& P, PairTerms& o) {
+    const int e2 = exp_field(r2);
+    if (!(e2 > 1023 - 100 && e2 < 1023 + 100)) return ref_terms_plain(rx, ry, rz, r2, P, o);
+    if (__double_as_longlong(r2) >= __double_as_longlong(P.rc2_cut)) return false;
+    const double y0 = seed_rcp(r2);
+    const double e = __fma_rn(-r2, y0, 1.0);
+    const double y = __fma_rn(__fma_rn(e, e, e), y0, y0);
+    const double s2 = __dmul_rn(P.sig2, y);
+    const double s6 = __dmul_rn(__dmul_rn(s2, s2), s2);
+    if (!FORCE) o.u = __fma_rn(__dmul_rn(P.eps4, s6), __dsub_rn(s6, 1.0), -P.ucut);
+    o.t = __dmul_rn(__dmul_rn(P.eps24, s6), __fma_rn(-2.0, s6, 1.0));
+    const double f = __dmul_rn(o.t, y);
+    o.gx = __dmul_rn(rx, f);
+    o.gy = __dmul_rn(ry, f);
+    o.gz = __dmul_rn(rz, f);
+    return true;
+}
+
+// `parts` blocks per tile, each a share of the tile's records; a warp walks
+// its part 32 candidates at a time.
+template <bool REF, bool FORCE>
+__global__ void __launch_bounds__(TILE) k_pair_terms(Dev d, int parts) {
+    if (chunk_failed(d)) return;
+    __shared__ float4 tab[27];
+    __shared__ uint32_t queue[TILE / 32][64];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int t = blockIdx.x / parts, part = blockIdx.x % parts;
+    const int4 tl = d.tiles[t];
+    const int2 pt = d.pair_tile[t];
+    const RepDev* R = d.rep + tl.x;
+    shift_table(tab, R);
+    __syncthreads();
+    const int per = ((pt.y + parts * TILE - 1) / (parts * TILE)) * 32;   // a warp's share, whole 32s
+    const int begin = pt.x + (part * (TILE / 32) + w) * per;
+    const int end = min(pt.x + pt.y, begin + per);
+    const double box[3] = {R->box[0], R->box[1], R->box[2]};
+    const float Lf[3] = {(float)box[0], (float)box[1], (float)box[2]};
+    const bool brute = R->mode == MODE_BRUTE;
+    uint32_t* qu = queue[w];
+    int held = 0;
+    auto compute = [&](int at) {
+        const uint32_t rec = qu[at];
+        const uint2 ij = d.pair_ij[rec];
+        const int j = (int)(ij.y & IDX_MASK);
+        const double4_32a pi = d.pos[ij.x], pj = d.pos[j];
+        const PairDev& P = d.pair[type_of(pi) * MAX_TYPES + type_of(pj)];
+        const double rx = min_image_ref(__dsub_rn(pj.x, pi.x), box[0]);   // potential.rs:181-200
+        const double ry = min_image_ref(__dsub_rn(pj.y, pi.y), box[1]);
+        const double rz = min_image_ref(__dsub_rn(pj.z, pi.z), box[2]);
+        const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), __dmul_rn(rz, rz));
+        PairTerms o;
+        o.u = 0.0;
+        const bool in = REF ? ref_terms<FORCE>(rx, ry, rz, r2, P, o) : r2_terms<FORCE>(rx, ry, rz, r2, P, o);
+        if (in) {
+            double2* dst = reinterpret_cast<double2*>(d.pair_rec + rec);
+            dst[0] = make_double2(o.gx, o.gy);
+            dst[1] = make_double2(o.gz, o.u);
+            if (!FORCE) d.pair_vir[rec] = o.t;
+        }
+        d.pair_in[rec] = in ? 1 : 0;
+    };
+    for (int b = begin; b < end; b += 32) {
+        const int rec = b + lane;
+        bool pass = false;
+        if (rec < end) {
+            // certainly outside r_cut in FP32: no FP64 work
+            const uint2 ij = d.pair_ij[rec];
+            const float4 mi = __ldg(d.mir + ij.x), mj = __ldg(d.mir + (ij.y & IDX_MASK));
+            const float4 sh = tab[ij.y >> IDX_BITS];
+            float ex = mj.x - mi.x + sh.x, ey = mj.y - mi.y + sh.y, ez = mj.z - mi.z + sh.z;
+            if (brute) {
+                if (ex < -0.5f * Lf[0]) ex += Lf[0]; else if (ex > 0.5f * Lf[0]) ex -= Lf[0];
+                if (ey < -0.5f * Lf[1]) ey += Lf[1]; else if (ey > 0.5f * Lf[1]) ey -= Lf[1];
+                if (ez < -0.5f * Lf[2]) ez += Lf[2]; else if (ez > 0.5f * Lf[2]) ez -= Lf[2];
+            }
+            const PairDev& P = d.pair[type_of(mi) * MAX_TYPES + type_of(mj)];
+            pass = !(ex * ex + ey * ey + ez * ez > P.rc2f_hi * 1.0001f);
+            if (!pass) d.pair_in[rec] = 0;
+        }
+        const unsigned got = __ballot_sync(0xffffffffu, pass);
+        if (pass) qu[held + __popc(got & ((1u << lane) - 1u))] = (uint32_t)rec;
+        held += __popc(got);
+        __syncwarp();
+        if (held >= 32) {
+            held -= 32;
+            compute(held + lane);
+            __syncwarp();
+        }
+    }
+    if (lane < held) compute(lane);
+}
+
+// ---------------------------------------------------------------------------
+// Per-atom sums in list order.  FORCE: a fused NVE pass, whose potential and
+// virial nobody reads (the chunk's last pass writes them) -- no record is then
+// read but its one sector, and neither forces nor sums are stored.
+template <bool KICK, bool FORCE>
+__global__ void __launch_bounds__(TILE) k_pair_sums(Dev d, StepParams sp) {
+    if (chunk_failed(d)) return;
+    __shared__ float tcs[8];
+    const int N = d.ntot;
+    const int4 tl = d.tiles[blockIdx.x];
+    const RepDev* R = d.rep + tl.x;
+    const long long rbeg = R->begin;
+    const int rn = R->n;
+    if (KICK && sp.fused && threadIdx.x == 0) drift_consts(*R, tcs);
+    __syncthreads();
+    const int s = tl.y + threadIdx.x;
+    const bool act = (int)threadIdx.x < tl.z;
+    double fx = 0.0, fy = 0.0, fz = 0.0, pe = 0.0, vr = 0.0;
+    const int n = act ? d.nn[s] : 0;
+    const uint32_t* row = d.pair_of + list_index(s, 0, 1, rbeg, rn, d.cap);
+    // 32 entries at a time: which of them lie inside r_cut, then their records
+    // in order, four loaded before any is added
+    constexpr int NB = 4;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const int m = min(32, n - k0);
+        uint32_t in = 0u;
+#pragma unroll 8
+        for (int q = 0; q < m; ++q) {
+            const uint32_t r = __ldg(row + (size_t)(k0 + q) * rn);
+            if (r != PAIR_NONE && __ldg(d.pair_in + (r & ~PAIR_NEG))) in |= 1u << q;
+        }
+        while (in) {
+            uint32_t r[NB];
+            double2 a[NB], b[NB];
+            double v[NB];
+#pragma unroll
+            for (int u = 0; u < NB; ++u) {
+                r[u] = PAIR_NONE;
+                if (in) r[u] = __ldg(row + (size_t)(k0 + __ffs(in) - 1) * rn);
+                in &= in - 1u;
+            }
+#pragma unroll
+            for (int u = 0; u < NB; ++u)
+                if (r[u] != PAIR_NONE) {
+                    const double2* p = reinterpret_cast<const double2*>(d.pair_rec + (r[u] & ~PAIR_NEG));
+                    a[u] = __ldg(p);
+                    b[u] = __ldg(p + 1);
+                    if (!FORCE) v[u] = __ldg(d.pair_vir + (r[u] & ~PAIR_NEG));
+                }
+#pragma unroll
+            for (int u = 0; u < NB; ++u)
+                if (r[u] != PAIR_NONE) {
+                    const unsigned long long neg = (unsigned long long)(r[u] & PAIR_NEG) << 32;
+                    auto sgn = [&](double x) {
+                        return __longlong_as_double((long long)((unsigned long long)__double_as_longlong(x) ^ neg));
+                    };
+                    fx = __dadd_rn(fx, sgn(a[u].x));
+                    fy = __dadd_rn(fy, sgn(a[u].y));
+                    fz = __dadd_rn(fz, sgn(b[u].x));
+                    if (!FORCE) {
+                        pe = __dadd_rn(pe, b[u].y);
+                        vr = __dadd_rn(vr, v[u]);
+                    }
+                }
+        }
+    }
+    float disp = 0.f;
+    if (act) {
+        if (!FORCE) {
+            d.frc[s] = fx; d.frc[N + s] = fy; d.frc[2 * N + s] = fz;
+            d.epot[s] = pe; d.evir[s] = vr;
+        }
+        if (KICK) disp = kick_and_drift<false>(d, sp, R, tcs, s, type_of(d.pos[s]), fx, fy, fz);
+    }
+    if (KICK && sp.fused) note_displacement(d, tl.x, disp);
+}
+
+// ---------------------------------------------------------------------------
+// Host side.
+cudaError_t launch_pair_build(const Dev& d, cudaStream_t st) {
+    k_pair_rows<<<d.ntiles, TILE, 0, st>>>(d);
+    k_pair_link<<<std::min(d.ntiles, 4096), TILE, 0, st>>>(d);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pair_forces(const Dev& d, const StepParams& sp, bool kick, int num_sms, cudaStream_t st) {
+    // Blocks per tile: four blocks (four warps a scheduler) keep an SM's FP64
+    // pipe busy, and more would cut a warp's share to a few batches of 32, the
+    // last of them partly empty.
+    const int parts = std::max(1, std::min(16, (4 * num_sms + d.ntiles - 1) / d.ntiles));
+    const bool force = kick && sp.fused;
+    const int grid = d.ntiles * parts;
+    if (d.refmode) {
+        if (force) k_pair_terms<true, true><<<grid, TILE, 0, st>>>(d, parts);
+        else k_pair_terms<true, false><<<grid, TILE, 0, st>>>(d, parts);
+    } else {
+        if (force) k_pair_terms<false, true><<<grid, TILE, 0, st>>>(d, parts);
+        else k_pair_terms<false, false><<<grid, TILE, 0, st>>>(d, parts);
+    }
+    if (force) k_pair_sums<true, true><<<d.ntiles, TILE, 0, st>>>(d, sp);
+    else if (kick) k_pair_sums<true, false><<<d.ntiles, TILE, 0, st>>>(d, sp);
+    else k_pair_sums<false, false><<<d.ntiles, TILE, 0, st>>>(d, sp);
+    return cudaGetLastError();
+}
+
+}  // namespace mdgb

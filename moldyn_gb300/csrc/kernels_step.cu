@@ -1306,6 +1306,9 @@ __device__ void phase_zero_cells(const Dev& d) {
         const int r = d.cell_rep[c];
         if (__ldcg(&d.rep[r].rebuild)) d.cell_count[c] = 0;
     }
+    if (d.pairs)
+        for (int r = gt; r < d.nrep; r += nt)
+            if (__ldcg(&d.rep[r].rebuild)) d.pair_count[r] = 0;
 }
 
 // Cell of every atom, and its slot among the cell's atoms in arrival order

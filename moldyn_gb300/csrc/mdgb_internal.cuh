@@ -60,6 +60,7 @@ struct PairDev {
     float rc2f_lo, rc2f_hi;  // band around rc^2 decided exactly in FP64
     int pad0, pad1;
     double rc2_cut;          // smallest double whose rounded square root exceeds rc
+    double sig2;             // sigma^2
 };
 
 struct RepDev {
@@ -124,6 +125,15 @@ struct StepParams {
     long long barrier_cycles;  // > 0: the grid barrier's wait limit in clock cycles (0: the default, ~2 s)
 };
 
+// The FP64 path's pair records (kernels_pairs.cu): force and potential of one
+// pair, each pair computed once -- one 32-byte sector.  The virial term F . r
+// lies in an array of its own (passes nobody reads it from skip it).
+struct __align__(32) PairRec {
+    double gx, gy, gz, u;
+};
+constexpr uint32_t PAIR_NONE = 0xFFFFFFFFu;   // a list entry without a record
+constexpr uint32_t PAIR_NEG = 0x80000000u;    // the record is the partner's: negate the force
+
 // Everything a kernel needs, passed by value.
 struct Dev {
     int ntot, ntiles, nrep, ntypes, cap, tpa, ncells;
@@ -182,6 +192,16 @@ struct Dev {
     float4* mir_next;           //   and mirrors (the other buffer of each pair)
     int2* band_list;            // mixed path: atoms (index, replica) left to k_force_band
     int* band_count;
+    // FP64 pair records (pairs != 0): replica r owns records pair_first(r) ..
+    // of pair_room(r), handed out tile by tile at a rebuild
+    int pairs, pad_pr;
+    uint32_t* pair_of;          // [cap][N], list order: record of each list entry, PAIR_NEG, PAIR_NONE
+    uint2* pair_ij;             // per record: atom i, its list entry (j | code << IDX_BITS)
+    PairRec* pair_rec;          // per record: the terms of the last force pass
+    double* pair_vir;
+    unsigned char* pair_in;     // per record: 1 if within r_cut at the last force pass
+    int2* pair_tile;            // [ntiles] first record, record count
+    int* pair_count;            // [nrep] records handed out since the rebuild
     FxRow* fx_part;             // [ntiles] exact tile sums (mixed path, coupled steps)
     FxRow* fx_cpart;            // [nchunks] exact chunk sums
 };
@@ -230,6 +250,33 @@ cudaError_t list_build_init();
 int list_build_grid(const Dev& d, int num_sms);
 int list_masks_grid(const Dev& d, int num_sms);
 cudaError_t launch_list_build(const Dev& d, int grid, int mgrid, cudaStream_t st);
+
+// FP64 pair records (kernels_pairs.cu).
+// Records a replica's region holds: half its list entries when both sides of
+// every pair list it (one type), else all of them.
+__host__ __device__ __forceinline__ size_t pair_room(size_t n, int cap, int single_type) {
+    return single_type ? n * (size_t)(cap / 2) : n * (size_t)cap;
+}
+cudaError_t launch_pair_build(const Dev& d, cudaStream_t st);
+cudaError_t launch_pair_forces(const Dev& d, const StepParams& sp, bool kick, int num_sms, cudaStream_t st);
+
+// Closes the rebuild k_pre started (one block, every thread).
+__device__ __forceinline__ void close_rebuild(const Dev& d, bool direct) {
+    for (int r = threadIdx.x; r < d.nrep; r += blockDim.x) {
+        RepDev* W = d.rep + r;
+        if (W->rebuild) {
+            W->rebuild = 0;
+            W->nrebuilds += 1;
+        }
+    }
+    if (threadIdx.x == 0) {
+        if (d.trace) atomicAdd(d.trace + TR_LIST, global_ns() - d.trace[TR_STAMP]);
+        if (direct) d.bar[5] += 1u;   // direct builds, for the engine's counters
+        d.bar[4] = 0u;
+        d.bar[3] = 0u;
+        atomicExch(d.bar + 2, 0u);
+    }
+}
 
 __device__ __forceinline__ int type_of(double4_32a p) { return (int)__double_as_longlong(p.w); }
 __device__ __forceinline__ int type_of(float4 p) { return __float_as_int(p.w); }

@@ -24,3 +24,16 @@ def test_sqrt_cut_matches_the_square_root_test(tmp_path):
     out = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
     assert "0 failures" in out.stdout
+
+
+def test_shared_reciprocal_gives_the_rounded_root_and_quotients(tmp_path):
+    """The FP64 pair kernel's square root and its five divisions by it through
+    one reciprocal carry the bits of sqrt and of the division operator."""
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    exe = str(tmp_path / "shared_reciprocal_check")
+    subprocess.check_call([cxx, "-O2", "-std=c++17", "-ffp-contract=off",
+                           os.path.join(ROOT, "tests", "cpp", "shared_reciprocal_check.cpp"), "-o", exe])
+    out = subprocess.run([exe, "2000000"], capture_output=True, text=True, timeout=120)
+    assert out.returncode == 0, out.stdout + out.stderr
