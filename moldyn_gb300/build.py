@@ -46,7 +46,8 @@ def nvcc() -> str:
 
 def _sources():
     return [os.path.join(CSRC, u) for u, _ in UNITS] + [
-        os.path.join(CSRC, "mdgb_internal.cuh"), os.path.join(CSRC, "force_common.cuh"), os.path.join(INCLUDE, "mdgb.h"), __file__]
+        os.path.join(CSRC, "mdgb_internal.cuh"), os.path.join(CSRC, "force_common.cuh"),
+        os.path.join(CSRC, "force_mixed.cuh"), os.path.join(CSRC, "list_direct.cuh"), os.path.join(INCLUDE, "mdgb.h"), __file__]
 
 
 def up_to_date() -> bool:

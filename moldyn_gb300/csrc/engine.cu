@@ -77,7 +77,7 @@ struct mdgb_engine {
     // the GPU reads the caller's pageable arrays itself (Grace: address
     // translation through the host's page tables), so uploads skip the copy
     bool host_direct = false;
-    int pre_blocks_per_sm = 0;
+    int pre_blocks_per_sm = 0, steps_blocks_per_sm = 0;
     int force_blocks_per_sm[4] = {0, 0, 0, 0};
     LJ pot[MAX_TYPES][MAX_TYPES];
     LJ pot_default;
@@ -683,12 +683,41 @@ int compute_forces_impl(mdgb_engine* e) {
     return fail(e, MDGB_ERR_NEIGHBOR_OVERFLOW, "neighbour list kept overflowing");
 }
 
+// Whether a chunk of this state's steps runs as one launch (k_steps): few
+// enough atoms that the step is launch latency and a mostly idle chip, one
+// thread per atom in the list layout, and nothing that looks at single
+// launches.  us a step, one launch / launches, mixed path: NVE 20 / 55 at 2,016
+// atoms, 29 / 58 at 8,788, 43 / 60 at 23,328, 66 / 59 at 32,000; Berendsen T
+// and P 58 / 83, 75 / 83, 105 / 97 at 23,328 (the same crossing with
+// Nose-Hoover).
+constexpr int SMALL_MAX_ATOMS = 24576, SMALL_MAX_COUPLED = 12288;
+bool small_size(const mdgb_engine* e) {
+    return e->ntot <= SMALL_MAX_ATOMS && !e->dev.pairs && e->cfg.rebuild_every == 0 && e->steps_blocks_per_sm > 0 &&
+           e->cfg.threads_per_atom <= 1 &&
+           !(e->cfg.flags & (MDGB_FLAG_PROFILE | MDGB_FLAG_TRACE | MDGB_FLAG_PERSISTENT));
+}
+bool small_system(const mdgb_engine* e, const StepParams& sp) {
+    if (!small_size(e) || ((sp.coupled || sp.thermo_nh) && e->ntot > SMALL_MAX_COUPLED)) return false;
+    for (int c = 0; c < mdgb_engine::NCLASS; ++c)
+        if (e->class_ntiles[c] && e->class_tpa[c] != 1) return false;
+    return true;
+}
+
 // n steps.  NVE chunks fuse each step's first kick and drift into the force
 // pass of the step before (steps 2..nf+1); nf is even, so the position/mirror
 // buffer pair ends the chunk the way round it started (a captured graph stays
 // valid), and the chunk's last step is unfused, leaving the state at a whole
 // step.
 int run_chunk_kernels(mdgb_engine* e, const StepParams& sp, int n) {
+    if (small_system(e, sp)) {
+        Dev d = e->dev;
+        d.pos_next = e->pos_alt;
+        d.mir_next = e->mir_alt;
+        CU(launch_steps(d, sp, n, e->cfg.precision == MDGB_PRECISION_FP32_NAIVE, e->num_sms * e->steps_blocks_per_sm,
+                        e->stream));
+        e->st.kernel_launches++;
+        return MDGB_OK;
+    }
     const bool fusable = sp.do_drift && !sp.coupled && !sp.thermo_nh;
     const int nf = fusable ? ((n - 1) & ~1) : 0;
     for (int i = 0; i < n; ++i) {
@@ -980,8 +1009,8 @@ int autotune_skin(mdgb_engine* e, double dt) {
 int autotune_tpa(mdgb_engine* e) {
     e->tuned = true;
     const int NC = mdgb_engine::NCLASS;
-    if (e->dev.refmode || e->dev.pairs || e->cfg.threads_per_atom > 0) {
-        const int t = e->dev.refmode || e->dev.pairs ? 1 : e->cfg.threads_per_atom;
+    if (e->dev.refmode || e->dev.pairs || e->cfg.threads_per_atom > 0 || small_size(e)) {
+        const int t = e->cfg.threads_per_atom > 0 && !e->dev.refmode ? e->cfg.threads_per_atom : 1;
         for (int c = 0; c < NC; ++c) e->class_tpa[c] = t;
         e->tpa = t;
         int rc = apply_class_tpa(e);
@@ -1543,6 +1572,7 @@ MDGB_API int mdgb_create(const mdgb_config* cfg, mdgb_engine** out) {
     int bps2 = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps2, (const void*)k_macro, TILE, 0);
     e->pre_blocks_per_sm = std::max(1, std::min(bps, bps2));
+    if (steps_init(&e->steps_blocks_per_sm) != cudaSuccess) { delete e; return MDGB_ERR_CUDA; }
     if (list_build_init() != cudaSuccess) { cudaGetLastError(); delete e; return MDGB_ERR_CUDA; }
     lj_finish(e->pot_default);
     *out = e;

@@ -1,5 +1,5 @@
 // force_common.cuh -- device helpers of the force kernels (kernels_force.cu,
-// kernels_pairs.cu).
+// kernels_pairs.cu, the whole-chunk kernel in kernels_step.cu).
 #pragma once
 #include "mdgb_internal.cuh"
 
@@ -42,6 +42,122 @@ __device__ __forceinline__ double min_image_ref(double r, double L) {
         return dadd_nospec(r, __longlong_as_double((long long)((unsigned long long)__double_as_longlong(L) ^ s)));
     }
     return r;
+}
+
+// The terms of one pair, from the side of the atom the displacement starts at.
+struct PairTerms {
+    double gx, gy, gz, u, t;
+};
+
+// The reference's operation sequence (potential.rs:57-75, :201-211) with the
+// library's square root and divisions.  False: |r| > r_cut.
+static __device__ __noinline__ bool ref_terms_plain(double rx, double ry, double rz, double r2, const PairDev& P,
+                                             PairTerms& o) {
+    const double r = __dsqrt_rn(r2);
+    if (r > P.rc) return false;                                          // :202-204
+    const double sr = __ddiv_rn(P.sigma, r);
+    const double s2 = __dmul_rn(sr, sr);
+    const double s4 = __dmul_rn(s2, s2);
+    const double s6 = __dmul_rn(s2, s4);
+    const double s12 = __dmul_rn(s6, s6);
+    o.u = __dsub_rn(__dmul_rn(P.eps4, __dsub_rn(s12, s6)), P.ucut);
+    const double dudr = __dmul_rn(__ddiv_rn(P.eps24, r), __dsub_rn(s6, __dmul_rn(2.0, s12)));
+    o.gx = __dmul_rn(__ddiv_rn(rx, r), dudr);                            // :207-211
+    o.gy = __dmul_rn(__ddiv_rn(ry, r), dudr);
+    o.gz = __dmul_rn(__ddiv_rn(rz, r), dudr);
+    o.t = __dadd_rn(__dadd_rn(__dmul_rn(o.gx, rx), __dmul_rn(o.gy, ry)), __dmul_rn(o.gz, rz));
+    return true;
+}
+
+__device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7FF; }
+
+// An approximation of 1/sqrt(x) or 1/x to about 2^-22, from FP32; x in the
+// FP32 range.
+__device__ __forceinline__ double seed_rsqrt(double x) { return flt_to_dbl(rsqrtf(dbl_to_flt_rn(x))); }
+__device__ __forceinline__ double seed_rcp(double x) { return flt_to_dbl(__fdividef(1.0f, dbl_to_flt_rn(x))); }
+
+// a / r correctly rounded, from y = 1/r within half a unit in the last place
+// (and a rounding of 2^-104) and yl = 1/r - y: q0 is within half a unit plus
+// 2^-50 of the quotient, its remainder is exact, and one correction rounds
+// correctly (Markstein 1990: a quotient lies at least 2^-106 r^-1 from the
+// middle of two doubles, further than the correction's own error; the one
+// exception is an r within a few units below a power of two).
+__device__ __forceinline__ double div_by(double a, double r, double y, double yl) {
+    const double q0 = __fma_rn(a, y, __dmul_rn(a, yl));
+    return __fma_rn(__fma_rn(-r, q0, a), y, q0);
+}
+
+// The same terms, bit for bit, with one square root and one reciprocal for the
+// five divisions by r: 1/sqrt(r2) by Newton's iteration (third order, from the
+// FP32 seed), r from it by one correction step whose remainder is checked (a
+// correctly rounded root has -u r < r2 - r^2 <= u r, u its unit in the last
+// place), 1/r in two words, and div_by.  58 FP64 instructions against about 78
+// with the library's divisions.  Values outside a range that keeps every
+// intermediate normal take the plain form.
+// FORCE: only the force is wanted (50).
+template <bool FORCE>
+__device__ __forceinline__ bool ref_terms(double rx, double ry, double rz, double r2, const PairDev& P, PairTerms& o) {
+    const int e2 = exp_field(r2);
+    const auto tame = [](double x) { const int e = exp_field(x); return e > 1023 - 400 || x == 0.0; };
+    bool ok = e2 > 1023 - 100 && e2 < 1023 + 100;
+    ok = ok && tame(rx) && tame(ry) && tame(rz);
+    double r = 0.0, y = 0.0;
+    if (ok) {
+        // r2 is below r_cut^2 exactly when its rounded root is at most r_cut
+        if (__double_as_longlong(r2) >= __double_as_longlong(P.rc2_cut)) return false;
+        const double y0 = seed_rsqrt(r2);
+        const double e = __fma_rn(-__dmul_rn(r2, y0), y0, 1.0);
+        y = __fma_rn(__dmul_rn(y0, e), __fma_rn(0.375, e, 0.5), y0);
+        const double g = __dmul_rn(r2, y);
+        const double h = __longlong_as_double(__double_as_longlong(y) - (1ll << 52));   // y / 2
+        r = __fma_rn(__fma_rn(-g, g, r2), h, g);
+        const double rem = __fma_rn(-r, r, r2);
+        const long long rb = __double_as_longlong(rem), mag = rb & 0x7FFFFFFFFFFFFFFFll;
+        // bits of u r, u = 2^(exponent of r - 52)
+        const long long lim = __double_as_longlong(r) + ((long long)(exp_field(r) - 1023 - 52) << 52);
+        ok = mag < lim || rb == lim;
+        // 1/r of an r just below a power of two does not round from y
+        ok = ok && (__double_as_longlong(r) & 0xFFFFFFFFFFFFFll) < 0xFFFFFFFFFFF00ll;
+    }
+    if (!ok) return ref_terms_plain(rx, ry, rz, r2, P, o);
+    y = __fma_rn(__fma_rn(-r, y, 1.0), y, y);
+    const double yl = __dmul_rn(__fma_rn(-r, y, 1.0), y);
+    const double sr = div_by(P.sigma, r, y, yl);
+    const double s2 = __dmul_rn(sr, sr);
+    const double s4 = __dmul_rn(s2, s2);
+    const double s6 = __dmul_rn(s2, s4);
+    const double s12 = __dmul_rn(s6, s6);
+    if (!FORCE) o.u = __dsub_rn(__dmul_rn(P.eps4, __dsub_rn(s12, s6)), P.ucut);
+    const double dudr = __dmul_rn(div_by(P.eps24, r, y, yl), __fma_rn(-2.0, s12, s6));   // 2 s12 is exact
+    o.gx = __dmul_rn(div_by(rx, r, y, yl), dudr);
+    o.gy = __dmul_rn(div_by(ry, r, y, yl), dudr);
+    o.gz = __dmul_rn(div_by(rz, r, y, yl), dudr);
+    if (!FORCE)
+        o.t = __dadd_rn(__dadd_rn(__dmul_rn(o.gx, rx), __dmul_rn(o.gy, ry)), __dmul_rn(o.gz, rz));
+    return true;
+}
+
+// Tree order (no MDGB_FLAG_REFERENCE_ORDER): the same functions of r^2 without
+// the root and the divisions by r -- sigma^2 / r^2 by one Newton step, F . r =
+// r dU/dr -- 24 FP64 instructions, 21 for the force alone.  Fewer roundings than the reference's form
+// ((sigma / r)^6 carries six times the rounding of r and of the quotient).
+template <bool FORCE>
+__device__ __forceinline__ bool r2_terms(double rx, double ry, double rz, double r2, const PairDev& P, PairTerms& o) {
+    const int e2 = exp_field(r2);
+    if (!(e2 > 1023 - 100 && e2 < 1023 + 100)) return ref_terms_plain(rx, ry, rz, r2, P, o);
+    if (__double_as_longlong(r2) >= __double_as_longlong(P.rc2_cut)) return false;
+    const double y0 = seed_rcp(r2);
+    const double e = __fma_rn(-r2, y0, 1.0);
+    const double y = __fma_rn(__fma_rn(e, e, e), y0, y0);
+    const double s2 = __dmul_rn(P.sig2, y);
+    const double s6 = __dmul_rn(__dmul_rn(s2, s2), s2);
+    if (!FORCE) o.u = __fma_rn(__dmul_rn(P.eps4, s6), __dsub_rn(s6, 1.0), -P.ucut);
+    o.t = __dmul_rn(__dmul_rn(P.eps24, s6), __fma_rn(-2.0, s6, 1.0));
+    const double f = __dmul_rn(o.t, y);
+    o.gx = __dmul_rn(rx, f);
+    o.gy = __dmul_rn(ry, f);
+    o.gz = __dmul_rn(rz, f);
+    return true;
 }
 
 // Second half kick v += F dt/2m (integrator.rs:49-55).  With sp.fused (NVE

@@ -35,7 +35,10 @@
 // This file is compiled with -fmad=false: its FP64 arithmetic (kick, drift,
 // wrap, reductions, coupling factors) keeps the reference's unfused
 // multiply-then-add rounding unless a fused operation is written out.
-#include "mdgb_internal.cuh"
+#include <algorithm>
+
+#include "force_mixed.cuh"
+#include "list_direct.cuh"
 
 namespace mdgb {
 
@@ -78,9 +81,11 @@ __device__ __forceinline__ double4_32a ldcg4(const double4_32a* p) {
 // block's verdict after the last barrier.
 __shared__ long long g_bar_limit;
 __shared__ int g_bar_abort;
+__shared__ int g_bar_spin;    // poll without sleeping in between (k_steps: short phases)
 
-__device__ __forceinline__ void barrier_setup(const StepParams& sp) {
+__device__ __forceinline__ void barrier_setup(const StepParams& sp, bool spin = false) {
     if (threadIdx.x == 0) {
+        g_bar_spin = spin ? 1 : 0;
         g_bar_limit = sp.barrier_cycles > 0 ? sp.barrier_cycles : BARRIER_LIMIT_CYCLES;
         g_bar_abort = 0;
     }
@@ -105,13 +110,60 @@ __device__ __forceinline__ bool grid_barrier(const Dev& d) {
         } else {
             const long long t0 = clock64();
             while (*gen == g) {
-                __nanosleep(100);
+                if (!g_bar_spin) __nanosleep(100);
                 if (clock64() - t0 > g_bar_limit) {
                     atomicOr(d.err, E_TIMEOUT);
                     break;
                 }
             }
         }
+        __threadfence();
+        g_tile_rep_id = -1;
+        g_bar_abort = (*(volatile int*)d.err & E_TIMEOUT) ? 1 : 0;
+    }
+    __syncthreads();
+    return g_bar_abort != 0;
+}
+
+// A grid barrier whose last block to arrive runs f() before it lets the others
+// go: f sees everything written before the barrier, and every block everything
+// f wrote (k_steps: reductions' last stages and the rebuild decision, which
+// would otherwise take a phase and a barrier of their own).
+template <class F>
+__device__ __forceinline__ bool grid_barrier_then(const Dev& d, F f) {
+    __shared__ int s_last_block, s_failed;
+    __syncthreads();
+    volatile unsigned int* gen = d.bar + 1;
+    unsigned int g = 0;
+    if (threadIdx.x == 0) {
+        g = *gen;
+        __threadfence();
+        s_last_block = atomicAdd(d.bar, 1u) == gridDim.x - 1 ? 1 : 0;
+        s_failed = chunk_failed(d) ? 1 : 0;
+        __threadfence();
+        g_tile_rep_id = -1;
+    }
+    __syncthreads();
+    if (s_last_block) {
+        if (!s_failed) f();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicExch(d.bar, 0u);
+            __threadfence();
+            atomicAdd(d.bar + 1, 1u);
+        }
+    } else if (threadIdx.x == 0) {
+        const long long t0 = clock64();
+        while (*gen == g) {
+            if (!g_bar_spin) __nanosleep(100);
+            if (clock64() - t0 > g_bar_limit) {
+                atomicOr(d.err, E_TIMEOUT);
+                break;
+            }
+        }
+    }
+    if (threadIdx.x == 0) {
         __threadfence();
         g_tile_rep_id = -1;
         g_bar_abort = (*(volatile int*)d.err & E_TIMEOUT) ? 1 : 0;
@@ -217,10 +269,10 @@ __device__ __forceinline__ void warp_sum_rows(const double* rows, int n, double 
 }
 
 template <int NS>
-__device__ void phase_chunk_sums(const Dev& d) {
+__device__ void phase_chunk_sums(const Dev& d, int block, int blocks) {
     const int lane = threadIdx.x & 31;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
+    const int gw = (block * blockDim.x + threadIdx.x) >> 5;
+    const int nw = (blocks * blockDim.x) >> 5;
     for (int c = gw; c < d.nchunks; c += nw) {
         const int4 ch = d.chunks[c];
         double s[NS];
@@ -294,9 +346,9 @@ __device__ void phase_partials1(const Dev& d, int sel) {
 
 // One warp per replica: COM velocity, momentum, kinetic and potential energy
 // (mod.rs:12-34, energy.rs:14-49).
-__device__ void phase_finalize1(const Dev& d, int sel) {
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ void phase_finalize1(const Dev& d, int sel, int block, int blocks) {
+    const int warps = (blocks * blockDim.x) >> 5;
+    const int gw = (block * blockDim.x + threadIdx.x) >> 5;
     const double m = d.mass[sel];
     for (int r = gw; r < d.nrep; r += warps) {
         const RepDev R = load_rep(d.rep + r);
@@ -364,9 +416,9 @@ __device__ __forceinline__ void coupling_factors(RepDev* W, const RepDev& R, dou
 // Finalize pass 2.  coupling: first apply the box part of the pending
 // barostat update (box *= mu once per type, barostat.rs:45), then T, P and
 // the coupling factors.
-__device__ void phase_finalize2(const Dev& d, const StepParams& sp, bool coupling, int sel) {
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ void phase_finalize2(const Dev& d, const StepParams& sp, bool coupling, int sel, int block, int blocks) {
+    const int warps = (blocks * blockDim.x) >> 5;
+    const int gw = (block * blockDim.x + threadIdx.x) >> 5;
     for (int r = gw; r < d.nrep; r += warps) {
         const RepDev R = load_rep(d.rep + r);
         double S1[1];
@@ -395,9 +447,9 @@ __device__ void phase_finalize2(const Dev& d, const StepParams& sp, bool couplin
 // n |vcm|^2 (as sum v_i = n vcm), so pass 2 and its barriers fold into the
 // finalize of pass 1; then what phase_finalize2 does (box, T, P, coupling).
 // The FP64 path keeps the reference's explicit second pass.
-__device__ void phase_finalize_single(const Dev& d, const StepParams& sp, int sel) {
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ void phase_finalize_single(const Dev& d, const StepParams& sp, int sel, int block, int blocks) {
+    const int warps = (blocks * blockDim.x) >> 5;
+    const int gw = (block * blockDim.x + threadIdx.x) >> 5;
     const double m = d.mass[sel];
     for (int r = gw; r < d.nrep; r += warps) {
         const RepDev R = load_rep(d.rep + r);
@@ -697,9 +749,9 @@ __device__ __forceinline__ void nh_update_psi(RepDev* W, const RepDev& R, double
     W->psi = R.psi + psi_dot * (dt / 2.0);
 }
 
-__device__ void phase_finalize_nh(const Dev& d, const StepParams& sp, int sel) {
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ void phase_finalize_nh(const Dev& d, const StepParams& sp, int sel, int block, int blocks) {
+    const int warps = (blocks * blockDim.x) >> 5;
+    const int gw = (block * blockDim.x + threadIdx.x) >> 5;
     for (int r = gw; r < d.nrep; r += warps) {
         const RepDev R = load_rep(d.rep + r);
         double S1[1];
@@ -1039,7 +1091,7 @@ __device__ void phase_serial_finalize(const Dev& d, const StepParams& sp, int se
         RepDev* W = d.rep + r;
         const double* A = d.part + (size_t)R.tile_begin * 8;
         const double* B = d.cpart + (size_t)R.chunk_begin * 8;
-        const long long n = R.type_off[sel + 1] - R.type_off[sel];
+        const long long n = __ldcg(&W->type_off[sel + 1]) - __ldcg(&W->type_off[sel]);
         const double th = __ldcg(B);
         const double T = temperature_of(th, n);
         if (nh_after_kick) {
@@ -1082,23 +1134,35 @@ __device__ bool phase_serial(const Dev& d, const StepParams& sp, int sel, bool c
     return false;
 }
 
+// The stages that follow a pass over the tiles: chunk sums, then a finalize
+// step.  With a few chunks (a few replicas of at most some ten thousand atoms)
+// the last block to arrive at the barrier does both; otherwise they are phases
+// of their own.  Returns true when the launch must stop.
+constexpr int THEN_MAX_CHUNKS = 16;
+template <int NS, class F>
+__device__ __forceinline__ bool sums_then(const Dev& d, F finalize) {
+    if (d.nchunks <= THEN_MAX_CHUNKS)
+        return grid_barrier_then(d, [&] {
+            phase_chunk_sums<NS>(d, 0, 1);
+            __syncthreads();
+            finalize(0, 1);
+        });
+    if (grid_barrier(d)) return true;
+    phase_chunk_sums<NS>(d, blockIdx.x, gridDim.x);
+    if (grid_barrier(d)) return true;
+    finalize(blockIdx.x, gridDim.x);
+    return grid_barrier(d);
+}
+
 // psi += psi_dot(T_t) * dt/2 with T_t the temperature of the atoms of type t
 // (thermostat.rs:35-39 before the kick, :59-65 after it), per replica with a
 // Nose-Hoover thermostat.  Returns true when the launch must stop.
 __device__ __forceinline__ bool nh_psi_of_type(const Dev& d, const StepParams& sp, int t) {
     if (d.refmode) return phase_serial(d, sp, t, false, true) || grid_barrier(d);
     phase_partials1(d, t);
-    if (grid_barrier(d)) return true;
-    phase_chunk_sums<7>(d);
-    if (grid_barrier(d)) return true;
-    phase_finalize1(d, t);
-    if (grid_barrier(d)) return true;
+    if (sums_then<7>(d, [&](int b, int n) { phase_finalize1(d, t, b, n); })) return true;
     phase_partials2(d, t);
-    if (grid_barrier(d)) return true;
-    phase_chunk_sums<1>(d);
-    if (grid_barrier(d)) return true;
-    phase_finalize_nh(d, sp, t);
-    return grid_barrier(d);
+    return sums_then<1>(d, [&](int b, int n) { phase_finalize_nh(d, sp, t, b, n); });
 }
 
 // ---------------------------------------------------------------------------
@@ -1225,9 +1289,9 @@ __device__ void phase_drift(const Dev& d, const StepParams& sp, bool kicked) {
 }
 
 // Per replica: consume the pending barostat factor, decide on a rebuild.
-__device__ void phase_decide(const Dev& d, const StepParams& sp) {
-    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nt = gridDim.x * blockDim.x;
+__device__ void phase_decide(const Dev& d, const StepParams& sp, int block, int blocks) {
+    const int gt = block * blockDim.x + threadIdx.x;
+    const int nt = blocks * blockDim.x;
     for (int r = gt; r < d.nrep; r += nt) decide_replica(d, sp, r);
 }
 
@@ -1299,9 +1363,9 @@ __device__ void phase_work_list(const Dev& d) {
     }
 }
 
-__device__ void phase_zero_cells(const Dev& d) {
-    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nt = gridDim.x * blockDim.x;
+__device__ void phase_zero_cells(const Dev& d, int block, int blocks) {
+    const int gt = block * blockDim.x + threadIdx.x;
+    const int nt = blocks * blockDim.x;
     for (int c = gt; c < d.ncells; c += nt) {
         const int r = d.cell_rep[c];
         if (__ldcg(&d.rep[r].rebuild)) d.cell_count[c] = 0;
@@ -1395,12 +1459,11 @@ __device__ void phase_scan_b(const Dev& d) {
     }
 }
 
-__device__ void phase_scan_c(const Dev& d, int chunk) {
+__device__ void phase_scan_c(const Dev& d, int b0, int b1, int before) {
     __shared__ int wsum[32];
     __shared__ int carry;
-    const int b0 = blockIdx.x * chunk, b1 = min(b0 + chunk, d.ncells);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (threadIdx.x == 0) carry = __ldcg(d.bsum + blockIdx.x);
+    if (threadIdx.x == 0) carry = before;
     __syncthreads();
     for (int base = b0; base < b1; base += blockDim.x) {
         const int c = base + threadIdx.x;
@@ -1814,6 +1877,53 @@ struct PhaseClock {
 
 __device__ __forceinline__ void k_pre_rebuild(const Dev& d, const StepParams& sp, PhaseClock& clk);
 
+// Nose-Hoover steps: the first kick alone, then Thermostat::update per type
+// (integrator.rs:35-39): each type's temperature before its scaling adds
+// psi_dot * dt/2 (thermostat.rs:59-65); the scaling itself uses the lambda
+// computed before the kick, in the drift phase.  Returns true when the launch
+// must stop.
+__device__ __forceinline__ bool nose_hoover_kick(const Dev& d, const StepParams& sp) {
+    if (d.mixed) phase_kick<true>(d, sp); else phase_kick<false>(d, sp);
+    // (in tree order a thread sums the atoms it kicked: no barrier in between)
+    if (d.refmode && grid_barrier(d)) return true;
+    for (int t = 0; t <= d.last_type; ++t)
+        if (nh_psi_of_type(d, sp, t)) return true;
+    return false;
+}
+
+// The coupling factors of a step, before its kick (integrator.rs:20-29), each
+// phase closed by a grid barrier.  Returns true when the launch must stop.
+__device__ __forceinline__ bool coupling_phases(const Dev& d, const StepParams& sp) {
+    const int sel = d.last_type;
+    // Nose-Hoover with several types: calculate_lambda runs once per type,
+    // each adding its psi_dot * dt/2 (thermostat.rs:35-39, called per type
+    // from integrator.rs:23-26); the last type's pass below adds its own
+    // and sets lambda from the sum
+    if (sp.thermo_nh)
+        for (int t = 0; t < sel; ++t)
+            if (nh_psi_of_type(d, sp, t)) return true;
+    if (d.refmode) {
+        if (phase_serial(d, sp, sel, true)) return true;
+        if (grid_barrier(d)) return true;
+    } else if (d.mixed && d.ntot >= FX_MIN_ATOMS) {
+        phase_partials_fx(d, sel);
+        if (grid_barrier(d)) return true;
+        phase_chunk_sums_fx(d);
+        if (grid_barrier(d)) return true;
+        phase_finalize_fx(d, sp, sel);
+        if (grid_barrier(d)) return true;
+    } else if (d.mixed) {
+        phase_partials1(d, sel);
+        if (sums_then<7>(d, [&](int b, int n) { phase_finalize_single(d, sp, sel, b, n); })) return true;
+    } else {
+        phase_partials1(d, sel);
+        if (sums_then<7>(d, [&](int b, int n) { phase_finalize1(d, sel, b, n); })) return true;
+        phase_partials2(d, sel);
+        if (sums_then<1>(d, [&](int b, int n) { phase_finalize2(d, sp, true, sel, b, n); })) return true;
+    }
+    return false;
+}
+
 // 6 blocks of 128 threads per SM (80 registers): at the default 64 registers
 // the phases spilled (measured: the rebuild's sort phases ran ~1.8x slower).
 __global__ void __launch_bounds__(TILE, 6) k_pre(Dev d, StepParams sp) {
@@ -1848,7 +1958,7 @@ __global__ void __launch_bounds__(TILE, 6) k_pre(Dev d, StepParams sp) {
             clk.mark(TR_DECIDE);
             return;
         }
-        phase_decide(d, sp);
+        phase_decide(d, sp, blockIdx.x, gridDim.x);
         if (grid_barrier(d)) return;
         clk.mark(TR_DECIDE);
         if (*(volatile unsigned int*)(d.bar + 2) == 0u) return;
@@ -1857,67 +1967,27 @@ __global__ void __launch_bounds__(TILE, 6) k_pre(Dev d, StepParams sp) {
         return;
     }
     if (sp.do_drift && sp.coupled) {
-        const int sel = d.last_type;
-        // Nose-Hoover with several types: calculate_lambda runs once per type,
-        // each adding its psi_dot * dt/2 (thermostat.rs:35-39, called per type
-        // from integrator.rs:23-26); the last type's pass below adds its own
-        // and sets lambda from the sum
-        if (sp.thermo_nh)
-            for (int t = 0; t < sel; ++t)
-                if (nh_psi_of_type(d, sp, t)) return;
-        if (d.refmode) {
-            if (phase_serial(d, sp, sel, true)) return;
-            if (grid_barrier(d)) return;
-        } else if (d.mixed && d.ntot >= FX_MIN_ATOMS) {
-            phase_partials_fx(d, sel);
-            if (grid_barrier(d)) return;
-            phase_chunk_sums_fx(d);
-            if (grid_barrier(d)) return;
-            phase_finalize_fx(d, sp, sel);
-            if (grid_barrier(d)) return;
-        } else if (d.mixed) {
-            phase_partials1(d, sel);
-            if (grid_barrier(d)) return;
-            phase_chunk_sums<7>(d);
-            if (grid_barrier(d)) return;
-            phase_finalize_single(d, sp, sel);
-            if (grid_barrier(d)) return;
-        } else {
-            phase_partials1(d, sel);
-            if (grid_barrier(d)) return;
-            phase_chunk_sums<7>(d);
-            if (grid_barrier(d)) return;
-            phase_finalize1(d, sel);
-            if (grid_barrier(d)) return;
-            phase_partials2(d, sel);
-            if (grid_barrier(d)) return;
-            phase_chunk_sums<1>(d);
-            if (grid_barrier(d)) return;
-            phase_finalize2(d, sp, true, sel);
-            if (grid_barrier(d)) return;
-        }
+        if (coupling_phases(d, sp)) return;
         clk.mark(TR_COUPLING);
     }
-    if (sp.do_drift && sp.thermo_nh) {
-        if (d.mixed) phase_kick<true>(d, sp); else phase_kick<false>(d, sp);
-        if (grid_barrier(d)) return;
-        // Thermostat::update per type after the kick (integrator.rs:35-39):
-        // each type's temperature before its scaling adds psi_dot * dt/2
-        // (thermostat.rs:59-65); the scaling itself uses the lambda computed
-        // before the kick, in the drift phase
-        for (int t = 0; t <= d.last_type; ++t)
-            if (nh_psi_of_type(d, sp, t)) return;
-        if (d.mixed) phase_drift<true>(d, sp, true); else phase_drift<false>(d, sp, true);
-        if (grid_barrier(d)) return;
-    } else if (sp.do_drift || !sp.force_rebuild) {
+    const bool moved = sp.do_drift || !sp.force_rebuild;
+    if (moved) {
         // (a forced rebuild without a step -- upload, refresh -- recomputes
         // every mirror in its gather: nothing here to do for it)
-        if (d.mixed) phase_drift<true>(d, sp, false); else phase_drift<false>(d, sp, false);
+        const bool nh = sp.do_drift && sp.thermo_nh;
+        if (nh && nose_hoover_kick(d, sp)) return;
+        if (d.mixed) phase_drift<true>(d, sp, nh); else phase_drift<false>(d, sp, nh);
+    }
+    if (moved && d.nrep <= TILE) {
+        // a thread per replica: the last block to arrive decides for all
+        if (grid_barrier_then(d, [&] { phase_decide(d, sp, 0, 1); })) return;
+        clk.mark(TR_DRIFT);
+    } else {
+        if (moved && grid_barrier(d)) return;
+        clk.mark(TR_DRIFT);
+        phase_decide(d, sp, blockIdx.x, gridDim.x);
         if (grid_barrier(d)) return;
     }
-    clk.mark(TR_DRIFT);
-    phase_decide(d, sp);
-    if (grid_barrier(d)) return;
     clk.mark(TR_DECIDE);
     if (*(volatile unsigned int*)(d.bar + 2) == 0u) return;
     if (clk.tr) atomicAdd(clk.tr + TR_REBUILD_LAUNCHES, 1ull);
@@ -1927,7 +1997,7 @@ __global__ void __launch_bounds__(TILE, 6) k_pre(Dev d, StepParams sp) {
 // The rebuild phases of k_pre (replicas with their rebuild flag set).
 __device__ __forceinline__ void k_pre_rebuild(const Dev& d, const StepParams& sp, PhaseClock& clk) {
     if (blockIdx.x == 0) phase_work_list(d);
-    phase_zero_cells(d);
+    phase_zero_cells(d, blockIdx.x, gridDim.x);
     if (grid_barrier(d)) return;
     clk.mark(TR_ZERO);
     phase_bin(d);
@@ -1940,7 +2010,7 @@ __device__ __forceinline__ void k_pre_rebuild(const Dev& d, const StepParams& sp
     phase_scan_b(d);
     if (grid_barrier(d)) return;
     clk.mark(TR_SCAN_B);
-    phase_scan_c(d, chunk);
+    phase_scan_c(d, blockIdx.x * chunk, min((int)(blockIdx.x + 1) * chunk, d.ncells), __ldcg(d.bsum + blockIdx.x));
     if (grid_barrier(d)) return;
     clk.mark(TR_SCAN_C);
     phase_scatter(d, !sp.do_drift);
@@ -1955,6 +2025,589 @@ __device__ __forceinline__ void k_pre_rebuild(const Dev& d, const StepParams& sp
     phase_build_list(d);
 }
 
+// ---------------------------------------------------------------------------
+// Whole chunks of small systems in one cooperative launch.
+//
+// A step of a few thousand atoms is five or six launches of a few microseconds
+// each, most of it launch latency and kernels that fill a tenth of the chip
+// with one thread per atom.  k_steps runs all n steps of a chunk: the phases
+// of k_pre, the direct list build and the force pass with `lanes` threads per
+// atom, separated by grid barriers; the reductions' last stages and the
+// rebuild decision run in the last block to arrive at a barrier.
+//
+// The force sums are exact (mixed path), so sharing an atom's list out over
+// more lanes changes no bit of them; the FP32 potential and virial and the
+// FP64 path's sums are added entry by entry in list order, as one thread per
+// atom adds them.
+//
+// Data written by this launch is read with plain or L2 loads, never with
+// non-coherent ones (the barrier's fences order them).
+
+// Dynamic shared memory of a block: during a rebuild the candidates of a cell
+// (16-byte mirrors and 4-byte entries), else the lists of its first atoms.
+constexpr int STEPS_WIN = 1800;
+constexpr int STEPS_SMEM = STEPS_WIN * 20;
+
+// What a block of k_steps keeps in shared memory besides Dev.
+struct StepsShared {
+    float4 tab[27];       // cell shifts and displacement constants of replica rep
+    float tcs[8];
+    int rep;
+    // the block's first unit of atoms (the only one of most launches): its
+    // tile and its lists, kept from one step to the next until a rebuild
+    int4 tile;
+    int unit, listed;
+    int n[TILE];          // list lengths
+    // force sums on their way from the lanes to one thread per atom
+    long long f[3][TILE];
+    float pe[TILE], vr[TILE];
+    int skip[TILE];       // no atom, or left to band_atom
+};
+
+// The tile of unit u and its replica's constants; lists that fit are copied
+// into `lists` ([atom][entry], row words apart) the first time a block sees
+// its first unit after a rebuild.
+__device__ __forceinline__ int4 steps_unit(const Dev& d, StepsShared& S, uint32_t* lists, int row, int u, int lanes) {
+    const bool first = u == (int)blockIdx.x;
+    int4 tl;
+    if (first && S.unit == u) tl = S.tile;
+    else tl = d.tiles[u / lanes];
+    const RepDev* R = d.rep + tl.x;
+    if (tl.x != S.rep || (first && !S.listed)) {   // block-uniform
+        __syncthreads();
+        shift_table(S.tab, R);
+        if (threadIdx.x == 0) { drift_consts(*R, S.tcs); S.rep = tl.x; }
+        if (first) {
+            const int per = TILE / lanes, a = threadIdx.x / lanes, lane = threadIdx.x % lanes;
+            const int at = (u % lanes) * per + a;
+            const int s = tl.y + at;
+            const int n = at < tl.z ? d.nn[s] : 0;
+            if (lane == 0) S.n[a] = n;
+            const uint32_t* list = d.nbr + list_index(at < tl.z ? s : tl.y, 0, 1, R->begin, R->n, d.cap);
+            for (int k = lane; k < min(n, row); k += lanes) lists[a * row + k] = list[(size_t)k * R->n];
+            if (threadIdx.x == 0) { S.tile = tl; S.unit = u; S.listed = 1; }
+        }
+        __syncthreads();
+    }
+    return tl;
+}
+
+// The force pass of a block's atoms (mixed path); lanes: a power of two <= 32.
+template <bool NAIVE, bool NOE>
+__device__ __noinline__ void steps_force_mixed(const Dev& d, const StepParams& sp, int lanes, StepsShared& S,
+                                               uint32_t* lists, int row) {
+    const unsigned FULL = 0xffffffffu;
+    const int N = d.ntot;
+    const int per = TILE / lanes, a = threadIdx.x / lanes, lane = threadIdx.x % lanes;
+    const float fscale = d.fscale;
+    const float fscale_t = NAIVE ? 1.0f : fscale * 1.1920928955078125e-07f;   // fscale / 2^23 (exact)
+    const float rl = (float)(d.rlist * 1.01);
+    const float split_limit = 2097152.0f / rl;       // as in k_force_mixed
+    const float range_limit = 4294967296.0f / rl;
+    for (int u = blockIdx.x; u < d.ntiles * lanes; u += gridDim.x) {
+        const int4 tl = steps_unit(d, S, lists, row, u, lanes);
+        const RepDev* R = d.rep + tl.x;
+        const float4* tab = S.tab;
+        const int at = (u % lanes) * per + a;
+        const bool act = at < tl.z;
+        const int s = tl.y + (act ? at : 0);
+        // the epilogue's atom (one thread per atom, from the block's first on)
+        // and its operands, on their way
+        const int es = tl.y + (u % lanes) * per + (int)threadIdx.x;
+        const bool eact = (int)threadIdx.x < per && (u % lanes) * per + (int)threadIdx.x < tl.z;
+        if (eact) {
+            prefetch_l1(d.vel + es);
+            prefetch_l1(d.vel + N + es);
+            prefetch_l1(d.vel + 2 * N + es);
+            if (sp.fused) {
+                prefetch_l1(d.pos + es);
+                prefetch_l1(d.mir0 + es);
+                prefetch_l1(d.cell + es);
+            }
+        }
+        const bool kept = u == (int)blockIdx.x && d.cap <= row;   // the lists are in shared memory
+        const int rn = R->n;
+        const float4 xi = d.mir[s];
+        const int ty = type_of(xi);
+        const bool brute = R->mode == MODE_BRUTE;
+        const int n = !act ? 0 : kept ? S.n[a] : d.nn[s];
+        const uint32_t* list = kept ? lists + a * row : d.nbr + list_index(s, 0, 1, R->begin, rn, d.cap);
+        const size_t step = kept ? 1 : (size_t)rn;
+        MixedAcc<NAIVE, NOE> acc;
+        acc.init();
+        bool band = false;
+        FixAcc bs[3];       // NOE: the sums as k_force_band rounds their terms
+        for (int c = 0; c < 3; ++c) bs[c].init();
+        float pe = 0.f, vr = 0.f, nx = 0.f, ny = 0.f, nz = 0.f;
+        const int rounds = __reduce_max_sync(FULL, (n + lanes - 1) / lanes);
+        uint32_t e = lane < n ? list[(size_t)lane * step] : 0u;
+        for (int i = 0; i < rounds; ++i) {
+            const int k = i * lanes + lane;
+            const bool have = k < n;
+            const float4 xj = d.mir[e & IDX_MASK];
+            const uint32_t ec = e;
+            if (k + lanes < n) e = list[(size_t)(k + lanes) * step];
+            bool in = false;
+            float fs = 0.f, uu = 0.f, r2 = 0.f, dz = 0.f;
+            f2_t dxy = 0ull;
+            if (have) {
+                const PairDev& PD = d.pair[ty * MAX_TYPES + type_of(xj)];
+                const PairF P = pairf(PD);
+                if (!brute) {
+                    const float4 sh = tab[ec >> IDX_BITS];
+                    dxy = add2(sub2(f2(xj.x, xj.y), f2(xi.x, xi.y)), f2(sh.x, sh.y));
+                    dz = __fadd_rn(__fsub_rn(xj.z, xi.z), sh.z);
+                    const float dx = f2_lo(dxy), dy = f2_hi(dxy);
+                    r2 = fmaf(dz, dz, fmaf(dy, dy, __fmul_rn(dx, dx)));
+                    in = r2 < P.rc2_lo;
+                    if (!in && r2 <= P.rc2_hi) {
+                        band = true;
+                        float bx, by;
+                        if (NOE && !NAIVE && exact_pair(d, R, s, (int)(ec & IDX_MASK), PD, bx, by, dz)) {
+                            in = true;
+                            dxy = f2(bx, by);
+                            r2 = fmaf(dz, dz, fmaf(by, by, __fmul_rn(bx, bx)));
+                        }
+                    }
+                } else {
+                    float dx, dy;
+                    in = exact_pair(d, R, s, (int)(ec & IDX_MASK), PD, dx, dy, dz);
+                    if (in) {
+                        dxy = f2(dx, dy);
+                        r2 = fmaf(dz, dz, fmaf(dy, dy, __fmul_rn(dx, dx)));
+                    }
+                }
+                if (in) {
+                    lj_f32(P, r2, fs, uu);
+                    if (!NAIVE) acc.add(dxy, dz, r2, fs, uu, fscale_t);
+                    if (NOE && !NAIVE) {
+                        // (there dx g is rounded before it is split; here
+                        // the paired instructions fuse the two)
+                        const float g = __fmul_rn(fs, fscale_t), dd[3] = {f2_lo(dxy), f2_hi(dxy), dz};
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            const float tt = __fmul_rn(dd[c], g);
+                            const float h = __fadd_rn(tt, FIX_MAGIC);
+                            bs[c].hi += __float_as_uint(h) - FIX_MAGIC_BITS;
+                            bs[c].lo += __float_as_uint(fmaf(__fsub_rn(tt, __fsub_rn(h, FIX_MAGIC)), 8388608.0f,
+                                                             FIX_MAGIC)) - FIX_MAGIC_BITS;
+                        }
+                    }
+                }
+            }
+            if (!NOE || NAIVE) {
+                // the sums whose order matters: entry by entry over the lanes
+                for (int q = 0; q < lanes; ++q) {
+                    const bool qi = __shfl_sync(FULL, in, q, lanes);
+                    const float qf = __shfl_sync(FULL, fs, q, lanes);
+                    if (NAIVE) {
+                        const float qx = __shfl_sync(FULL, f2_lo(dxy), q, lanes), qy = __shfl_sync(FULL, f2_hi(dxy), q, lanes),
+                                    qz = __shfl_sync(FULL, dz, q, lanes);
+                        if (qi) { nx = fmaf(qx, qf, nx); ny = fmaf(qy, qf, ny); nz = fmaf(qz, qf, nz); }
+                    }
+                    if (!NOE) {
+                        const float qu = __shfl_sync(FULL, uu, q, lanes), qr = __shfl_sync(FULL, r2, q, lanes);
+                        if (qi) { pe = __fadd_rn(pe, qu); vr = fmaf(qf, qr, vr); }
+                    }
+                }
+            }
+        }
+        long long sx = acc.ax.total(), sy = acc.ay.total(), sz = acc.az.total();
+        float gmax = acc.gmax;
+        for (int off = lanes / 2; off > 0; off >>= 1) {
+            gmax = fmaxf(gmax, __shfl_xor_sync(FULL, gmax, off));
+            band |= __shfl_xor_sync(FULL, (int)band, off) != 0;
+        }
+        constexpr bool IN_LANE = NOE && !NAIVE;   // band pairs were decided in the loop
+        if (IN_LANE && band) { sx = bs[0].total(); sy = bs[1].total(); sz = bs[2].total(); }
+        if (!NAIVE && act && (IN_LANE || !band) && (gmax > split_limit || n > FIX_FOLD)) {
+            // a term may exceed the exact range of the split, or the list is
+            // as long as k_force_mixed converts: exact conversions
+            if (gmax > range_limit) atomicOr(d.err, E_FIXED);
+            sx = sy = sz = 0;
+            for (int k = lane; k < n; k += lanes) {
+                const uint32_t ek = list[(size_t)k * step];
+                const int j = (int)(ek & IDX_MASK);
+                const float4 xj = d.mir[j];
+                const float4 sh = tab[ek >> IDX_BITS];
+                float dx = __fadd_rn(__fsub_rn(xj.x, xi.x), sh.x), dy = __fadd_rn(__fsub_rn(xj.y, xi.y), sh.y),
+                      dz = __fadd_rn(__fsub_rn(xj.z, xi.z), sh.z);
+                const PairDev& PD = d.pair[ty * MAX_TYPES + type_of(xj)];
+                const PairF P = pairf(PD);
+                if (brute) {
+                    if (!exact_pair(d, R, s, j, PD, dx, dy, dz)) continue;
+                } else {
+                    const float q2 = fmaf(dz, dz, fmaf(dy, dy, __fmul_rn(dx, dx)));
+                    if (q2 > P.rc2_hi) continue;
+                    if (q2 >= P.rc2_lo && !exact_pair(d, R, s, j, PD, dx, dy, dz)) continue;
+                }
+                float fs, uu;
+                lj_f32(P, fmaf(dz, dz, fmaf(dy, dy, __fmul_rn(dx, dx))), fs, uu);
+                const float g = __fmul_rn(fs, fscale);
+                sx += __float2ll_rn(__fmul_rn(dx, g));
+                sy += __float2ll_rn(__fmul_rn(dy, g));
+                sz += __float2ll_rn(__fmul_rn(dz, g));
+            }
+        }
+        for (int off = lanes / 2; off > 0; off >>= 1) {
+            sx += __shfl_xor_sync(FULL, sx, off);
+            sy += __shfl_xor_sync(FULL, sy, off);
+            sz += __shfl_xor_sync(FULL, sz, off);
+        }
+        // one thread per atom finishes: a warp of them costs the FP64 pipe no
+        // more than a single lane would
+        if (lane == 0) {
+            S.skip[a] = !act || (band && !IN_LANE);
+            if (NAIVE) {
+                S.f[0][a] = __float_as_int(nx); S.f[1][a] = __float_as_int(ny); S.f[2][a] = __float_as_int(nz);
+            } else {
+                S.f[0][a] = sx; S.f[1][a] = sy; S.f[2][a] = sz;
+            }
+            if (!NOE) { S.pe[a] = pe; S.vr[a] = vr; }
+        }
+        __syncthreads();
+        if ((int)threadIdx.x < ((per + 31) & ~31)) {   // whole warps
+            float disp = 0.f;
+            if (eact && !S.skip[threadIdx.x]) {
+                double F[3];
+                for (int c = 0; c < 3; ++c) {
+                    const long long v = S.f[c][threadIdx.x];
+                    F[c] = NAIVE ? flt_to_dbl(__int_as_float((int)v)) : fixed_to_double(v, d.fscale_log2);
+                }
+                if (!NOE) {
+                    d.frc[es] = F[0]; d.frc[N + es] = F[1]; d.frc[2 * N + es] = F[2];
+                    d.epot[es] = flt_to_dbl(S.pe[threadIdx.x]); d.evir[es] = flt_to_dbl(S.vr[threadIdx.x]);
+                }
+                disp = kick_and_drift<true>(d, sp, R, S.tcs, es, type_of(d.mir[es]), F[0], F[1], F[2]);
+            }
+            if (sp.fused) note_displacement(d, tl.x, disp);
+        }
+        // atoms with a pair in the band, the whole warp for each (as k_force_band:
+        // the order of its potential and virial sums)
+        unsigned left = IN_LANE ? 0u : __ballot_sync(FULL, act && band && lane == 0);
+        while (left) {
+            const int src = __ffs(left) - 1;
+            left &= left - 1u;
+            band_atom<NAIVE, true>(d, sp, __shfl_sync(FULL, s, src), tl.x, true);
+            __syncwarp();
+        }
+        __syncthreads();
+    }
+}
+
+// The same for the FP64 path (lanes of at least eight): each lane the terms of
+// its entry, added in list order.
+__device__ __noinline__ void steps_force_fp64(const Dev& d, const StepParams& sp, int lanes, StepsShared& S,
+                                              uint32_t* lists, int row) {
+    const unsigned FULL = 0xffffffffu;
+    const int N = d.ntot;
+    const int per = TILE / lanes, a = threadIdx.x / lanes, lane = threadIdx.x % lanes;
+    for (int u = blockIdx.x; u < d.ntiles * lanes; u += gridDim.x) {
+        const int4 tl = steps_unit(d, S, lists, row, u, lanes);
+        const RepDev* R = d.rep + tl.x;
+        const float4* tab = S.tab;
+        const int at = (u % lanes) * per + a;
+        const bool act = at < tl.z;
+        const int s = tl.y + (act ? at : 0);
+        const bool kept = u == (int)blockIdx.x && d.cap <= row;
+        const double box[3] = {R->box[0], R->box[1], R->box[2]};
+        const float Lf[3] = {(float)box[0], (float)box[1], (float)box[2]};
+        const bool brute = R->mode == MODE_BRUTE;
+        const double4_32a pi = d.pos[s];
+        const float4 mi = d.mir[s];
+        const int ty = type_of(pi);
+        const int n = !act ? 0 : kept ? S.n[a] : d.nn[s];
+        const uint32_t* list = kept ? lists + a * row : d.nbr + list_index(s, 0, 1, R->begin, R->n, d.cap);
+        const size_t step = kept ? 1 : (size_t)R->n;
+        double sum = 0.0;
+        const int rounds = __reduce_max_sync(FULL, (n + lanes - 1) / lanes);
+        for (int i = 0; i < rounds; ++i) {
+            const int k = i * lanes + lane;
+            PairTerms o{0.0, 0.0, 0.0, 0.0, 0.0};
+            bool in = false;
+            if (k < n) {
+                const uint32_t e = list[(size_t)k * step];
+                const int j = (int)(e & IDX_MASK);
+                const float4 mj = d.mir[j];
+                const PairDev& P = d.pair[ty * MAX_TYPES + type_of(mj)];
+                const float4 sh = tab[e >> IDX_BITS];
+                float ex = mj.x - mi.x + sh.x, ey = mj.y - mi.y + sh.y, ez = mj.z - mi.z + sh.z;
+                if (brute) {
+                    if (ex < -0.5f * Lf[0]) ex += Lf[0]; else if (ex > 0.5f * Lf[0]) ex -= Lf[0];
+                    if (ey < -0.5f * Lf[1]) ey += Lf[1]; else if (ey > 0.5f * Lf[1]) ey -= Lf[1];
+                    if (ez < -0.5f * Lf[2]) ez += Lf[2]; else if (ez > 0.5f * Lf[2]) ez -= Lf[2];
+                }
+                if (!(ex * ex + ey * ey + ez * ez > P.rc2f_hi * 1.0001f)) {
+                    const double4_32a pj = d.pos[j];
+                    const double rx = min_image_ref(__dsub_rn(pj.x, pi.x), box[0]);
+                    const double ry = min_image_ref(__dsub_rn(pj.y, pi.y), box[1]);
+                    const double rz = min_image_ref(__dsub_rn(pj.z, pi.z), box[2]);
+                    const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), __dmul_rn(rz, rz));
+                    in = d.refmode ? ref_terms<false>(rx, ry, rz, r2, P, o) : r2_terms<false>(rx, ry, rz, r2, P, o);
+                }
+            }
+            // the sums whose order matters, entry by entry over the lanes; lane
+            // c of an atom adds component c (an FP64 add costs the warp 64
+            // cycles however many lanes take part)
+            unsigned any = __ballot_sync(FULL, in);
+            for (int off = 16; off >= lanes; off >>= 1) any |= any >> off;   // entries some atom of the warp has
+            for (int q = 0; q < lanes; ++q) {
+                if (!(any >> q & 1u)) continue;
+                const bool qi = __shfl_sync(FULL, in, q, lanes);
+                const double gx = __shfl_sync(FULL, o.gx, q, lanes), gy = __shfl_sync(FULL, o.gy, q, lanes),
+                             gz = __shfl_sync(FULL, o.gz, q, lanes), uu = __shfl_sync(FULL, o.u, q, lanes),
+                             tt = __shfl_sync(FULL, o.t, q, lanes);
+                if (qi) sum = __dadd_rn(sum, lane == 0 ? gx : lane == 1 ? gy : lane == 2 ? gz : lane == 3 ? uu : tt);
+            }
+        }
+        const double fx = __shfl_sync(FULL, sum, 0, lanes), fy = __shfl_sync(FULL, sum, 1, lanes),
+                     fz = __shfl_sync(FULL, sum, 2, lanes), pe = __shfl_sync(FULL, sum, 3, lanes),
+                     vr = __shfl_sync(FULL, sum, 4, lanes);
+        float disp = 0.f;
+        if (act && lane == 0) {
+            d.frc[s] = fx; d.frc[N + s] = fy; d.frc[2 * N + s] = fz;
+            d.epot[s] = pe; d.evir[s] = vr;
+            disp = kick_and_drift<false>(d, sp, R, S.tcs, s, ty, fx, fy, fz);
+        }
+        if (sp.fused) note_displacement(d, tl.x, disp);
+    }
+}
+
+// The rebuild decision of every replica (one block): decide_replica without
+// reading whole records where none is needed.  A rebuild's work list is made
+// and its cells are cleared here as well.
+__device__ __noinline__ void steps_decide(const Dev& d, const StepParams& sp) {
+    bool any = false;
+    for (int r = threadIdx.x; r < d.nrep; r += blockDim.x) {
+        if (rebuild_needed_at(d, sp, d.rep + r)) {
+            any = true;
+            decide_replica(d, sp, r);
+        } else {
+            RepDev* W = d.rep + r;
+            W->pending = __ldcg(&W->baro_on) ? __ldcg(&W->myu) : 1.0;
+            W->steps_since = __ldcg(&W->steps_since) + 1;
+            W->rebuild = 0;
+        }
+    }
+    if (__syncthreads_or(any)) {
+        phase_work_list(d);
+        phase_zero_cells(d, 0, 1);
+    }
+}
+
+// Lists of the rebuilding cell-mode replicas, one block per cell: the shifted
+// mirrors of the 27 neighbour cells in shared memory, then a warp per own atom
+// tests 32 of them at a time and appends the hits -- the tests, entries and
+// order of list_direct.  (There a warp takes a whole cell; with the few cells
+// of a small system that left most of the chip idle and took 49 us for 2,016
+// atoms.)
+
+__device__ __noinline__ void steps_lists(const Dev& d, uint32_t* smem) {
+    __shared__ int nb_start[28], nb_off[28];
+    const unsigned FULL = 0xffffffffu;
+    float4* cx = reinterpret_cast<float4*>(smem);
+    uint32_t* ce = smem + 4 * STEPS_WIN;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int m = d.rb[0], nwork = rb_cell_off(d)[m];
+    for (int wi = blockIdx.x; wi < nwork; wi += gridDim.x) {
+        const int i = rb_locate(rb_cell_off(d), m, wi);
+        const int r = rb_rep(d)[i];
+        const RepDev* W = d.rep + r;
+        if (W->mode != MODE_CELLS) continue;
+        const int c = W->cell_base + wi - rb_cell_off(d)[i];
+        const float rl = (float)(W->rlist * (1.0 + 1e-5));
+        const int nc[3] = {W->nc[0], W->nc[1], W->nc[2]};
+        const long long rbeg = W->begin;
+        const int rn = W->n;
+        const float cs[3] = {dbl_to_flt_rn(W->cs[0]), dbl_to_flt_rn(W->cs[1]), dbl_to_flt_rn(W->cs[2])};
+        const int ib = d.cell_start[c], in = d.cell_count[c];
+        if (ib < rbeg || ib + in > rbeg + rn) {
+            if (threadIdx.x == 0) atomicOr(d.err, E_CELLS);
+            continue;
+        }
+        __syncthreads();
+        if (w == 0) {
+            int ox, oy, oz, start = 0, cnt = 0;
+            decode_cell(c - W->cell_base, nc, ox, oy, oz);
+            if (lane < 27) {
+                int x = ox + lane % 3 - 1, y = oy + (lane / 3) % 3 - 1, z = oz + lane / 9 - 1;
+                x = x < 0 ? x + nc[0] : (x >= nc[0] ? x - nc[0] : x);
+                y = y < 0 ? y + nc[1] : (y >= nc[1] ? y - nc[1] : y);
+                z = z < 0 ? z + nc[2] : (z >= nc[2] ? z - nc[2] : z);
+                const int cj = W->cell_base + (x * nc[1] + y) * nc[2] + z;
+                start = d.cell_start[cj];
+                cnt = d.cell_count[cj];
+                if (start < rbeg || start + cnt > rbeg + rn) { atomicOr(d.err, E_CELLS); cnt = 0; }
+            }
+            int incl = cnt;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int y = __shfl_up_sync(FULL, incl, off);
+                if (lane >= off) incl += y;
+            }
+            if (lane < 28) { nb_start[lane] = start; nb_off[lane] = incl - cnt; }
+        }
+        __syncthreads();
+        const int total = nb_off[27];
+        // candidate p of the stream: its entry word and shifted mirror
+        auto candidate = [&](int p, uint32_t& e, float4& x) {
+            int lo = 0, hi = 26;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (nb_off[mid] <= p) lo = mid; else hi = mid - 1;
+            }
+            const int j = nb_start[lo] + p - nb_off[lo];
+            e = (uint32_t)j | ((uint32_t)lo << IDX_BITS);
+            x = d.mir[j];
+            x.x = __fadd_rn(x.x, __fmul_rn((float)(lo % 3 - 1), cs[0]));
+            x.y = __fadd_rn(x.y, __fmul_rn((float)((lo / 3) % 3 - 1), cs[1]));
+            x.z = __fadd_rn(x.z, __fmul_rn((float)(lo / 9 - 1), cs[2]));
+        };
+        const bool held = total <= STEPS_WIN;
+        if (held)
+            for (int p = threadIdx.x; p < total; p += blockDim.x) candidate(p, ce[p], cx[p]);
+        __syncthreads();
+        int cmax = 0;
+        for (int a = w; a < in; a += TILE / 32) {
+            const int s = ib + a;
+            const float4 xi = d.mir[s];
+            const int ti = type_of(xi);
+            uint32_t* list = d.nbr + list_index(s, 0, 1, rbeg, rn, d.cap);
+            const int self = nb_off[CODE_ZERO] + a;
+            int cnt = 0;
+            for (int q = 0; q < total; q += 32) {
+                const int p = q + lane;
+                bool hit = false;
+                uint32_t e = 0u;
+                if (p < total) {
+                    float4 x;
+                    if (held) { e = ce[p]; x = cx[p]; } else candidate(p, e, x);
+                    const float ex = __fsub_rn(x.x, xi.x), ey = __fsub_rn(x.y, xi.y), ez = __fsub_rn(x.z, xi.z);
+                    hit = fmaf(ez, ez, fmaf(ey, ey, fmaf(ex, ex, -__fmul_rn(rl, rl)))) < 0.f && type_of(x) >= ti &&
+                          p != self;
+                }
+                const unsigned got = __ballot_sync(FULL, hit);
+                const int k = cnt + __popc(got & ((1u << lane) - 1u));
+                if (hit && k < d.cap) list[(size_t)k * rn] = e;
+                cnt += __popc(got);
+            }
+            const int nfill = min(cnt, d.cap);
+            if (d.refmode) sort_lists_by_rank(d, s, lane == 0 ? nfill : 0, rbeg, rn);
+            if (lane == 0) {
+                d.nn[s] = nfill;
+                if (cnt > d.cap) {
+                    atomicOr(d.err, E_NLIST);
+                    atomicMax(d.max_needed, cnt);
+                }
+            }
+            cmax = max(cmax, cnt);
+        }
+        if (lane == 0 && cmax > 0) atomicMax(&d.rep[r].max_nn, cmax);
+    }
+}
+
+// The rebuild of k_pre with the scans in the last block to arrive, then the
+// lists and the end of the rebuild.
+__device__ __noinline__ bool steps_rebuild(const Dev& d, uint32_t* st_smem) {
+    phase_bin(d);
+    if (grid_barrier_then(d, [&] { phase_scan_c(d, 0, d.ncells, 0); })) return true;
+    phase_scatter(d, false);
+    if (grid_barrier(d)) return true;
+    if (d.mixed) phase_sort_gather<true>(d, false); else phase_sort_gather<false>(d, false);
+    if (grid_barrier(d)) return true;
+    phase_build_list(d);
+    steps_lists(d, st_smem);
+    return grid_barrier_then(d, [&] { close_rebuild(d, d.direct_list != 0); });
+}
+
+// Coupling and motion of a step that the previous force pass did not drift.
+__device__ __noinline__ bool steps_motion(const Dev& d, const StepParams& sp) {
+    if (sp.coupled && coupling_phases(d, sp)) return true;
+    if (sp.thermo_nh && nose_hoover_kick(d, sp)) return true;
+    if (d.mixed) phase_drift<true>(d, sp, sp.thermo_nh != 0); else phase_drift<false>(d, sp, sp.thermo_nh != 0);
+    return false;
+}
+
+// One step's motion up to its positions, its list and its forces; the last
+// barrier of a step is the next one's rebuild decision.
+__global__ void __launch_bounds__(TILE, 4) k_steps(Dev d_in, StepParams sp_in, int n, int naive, int lanes) {
+    if (chunk_failed(d_in)) return;
+    extern __shared__ __align__(16) uint32_t st_smem[];
+    __shared__ __align__(16) unsigned char dev_mem[sizeof(Dev)];
+    __shared__ StepsShared S;
+    Dev& d = *reinterpret_cast<Dev*>(dev_mem);   // the buffer pair is swapped after every fused step
+    if (threadIdx.x == 0) { d = d_in; S.rep = -1; S.unit = -1; S.listed = 0; }
+    StepParams sp = sp_in;
+    barrier_setup(sp, true);
+    tile_rep_reset();
+    if (sp.hold_block == (int)blockIdx.x && threadIdx.x == 0) {   // failure test, as in k_pre
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2 * g_bar_limit) __nanosleep(1000);
+    }
+    __syncthreads();
+    const int row = STEPS_SMEM / 4 / (TILE / lanes);   // list words shared memory holds per atom
+    const bool fusable = !sp.coupled && !sp.thermo_nh;
+    const int nf = fusable ? ((n - 1) & ~1) : 0;
+    for (int i = 0; i < n; ++i) {
+        const bool predrifted = i >= 1 && i <= nf;
+        if (!predrifted && steps_motion(d, sp)) return;
+        if (grid_barrier_then(d, [&] { steps_decide(d, sp); })) return;
+        const bool rebuild = *(volatile unsigned int*)(d.bar + 2) != 0u;
+        if (rebuild && steps_rebuild(d, st_smem)) return;
+        // the force pass's per-replica constants stay in shared memory while
+        // neither box nor cells change
+        if (rebuild || sp.coupled) {
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                S.rep = -1;
+                if (rebuild) S.listed = 0;
+            }
+            __syncthreads();
+        }
+        sp.fused = i < nf ? 1 : 0;
+        if (!d.mixed) steps_force_fp64(d, sp, lanes, S, st_smem, row);
+        else if (naive) steps_force_mixed<true, false>(d, sp, lanes, S, st_smem, row);
+        else if (sp.fused) steps_force_mixed<false, true>(d, sp, lanes, S, st_smem, row);
+        else steps_force_mixed<false, false>(d, sp, lanes, S, st_smem, row);
+        __syncthreads();
+        if (sp.fused && threadIdx.x == 0) {
+            double4_32a* const p = d.pos; d.pos = d.pos_next; d.pos_next = p;
+            float4* const m = d.mir; d.mir = d.mir_next; d.mir_next = m;
+        }
+        sp.fused = 0;
+        // an unfused step's forces are read by the next step's kick or sums
+        if (i >= nf && i + 1 < n && grid_barrier(d)) return;
+    }
+}
+
+// Host side of k_steps: resident blocks per SM.
+
+cudaError_t steps_init(int* blocks_per_sm) {
+    const cudaError_t err = cudaFuncSetAttribute(k_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, STEPS_SMEM);
+    if (err != cudaSuccess) return err;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_steps, TILE, STEPS_SMEM);
+}
+
+cudaError_t launch_steps(const Dev& d, const StepParams& sp, int n, bool naive, int max_blocks, cudaStream_t st) {
+    // as many lanes per atom as the resident threads allow; the FP64 path adds
+    // an entry at a time over a warp, so two atoms a warp at least, and its
+    // sums need eight lanes
+    int lanes = d.mixed ? 32 : 16;
+    while (lanes > (d.mixed ? 1 : 8) && d.ntiles * lanes > max_blocks) lanes /= 2;
+    const int folds = d.refmode ? 6 * d.nrep : 1;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(std::min(max_blocks, std::max(d.ntiles * lanes, folds)));
+    lc.blockDim = dim3(TILE);
+    lc.dynamicSmemBytes = STEPS_SMEM;
+    lc.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, k_steps, d, sp, n, naive ? 1 : 0, lanes);
+}
+
 // Macro parameters of type `sel` (solver/src/macro_parameters): results land
 // in the replica records (vcm, mom, ke, pe, thermal, T, P, count).
 // 6 blocks per SM, as k_pre: the engine launches both on one grid size.
@@ -1966,16 +2619,9 @@ __global__ void __launch_bounds__(TILE, 6) k_macro(Dev d, StepParams sp, int sel
         return;
     }
     phase_partials1(d, sel);
-    if (grid_barrier(d)) return;
-    phase_chunk_sums<7>(d);
-    if (grid_barrier(d)) return;
-    phase_finalize1(d, sel);
-    if (grid_barrier(d)) return;
+    if (sums_then<7>(d, [&](int b, int n) { phase_finalize1(d, sel, b, n); })) return;
     phase_partials2(d, sel);
-    if (grid_barrier(d)) return;
-    phase_chunk_sums<1>(d);
-    if (grid_barrier(d)) return;
-    phase_finalize2(d, sp, false, sel);
+    sums_then<1>(d, [&](int b, int n) { phase_finalize2(d, sp, false, sel, b, n); });
 }
 
 // End of an mdgb_step call: finish the barostat update of the last step

@@ -260,6 +260,10 @@ __host__ __device__ __forceinline__ size_t pair_room(size_t n, int cap, int sing
 cudaError_t launch_pair_build(const Dev& d, cudaStream_t st);
 cudaError_t launch_pair_forces(const Dev& d, const StepParams& sp, bool kick, int num_sms, cudaStream_t st);
 
+// Whole chunks of small systems in one launch (kernels_step.cu).
+cudaError_t steps_init(int* blocks_per_sm);
+cudaError_t launch_steps(const Dev& d, const StepParams& sp, int n, bool naive, int max_blocks, cudaStream_t st);
+
 // Closes the rebuild k_pre started (one block, every thread).
 __device__ __forceinline__ void close_rebuild(const Dev& d, bool direct) {
     for (int r = threadIdx.x; r < d.nrep; r += blockDim.x) {
@@ -476,12 +480,15 @@ __device__ __forceinline__ float mirror_disp(float4 m, float4 m0, const float* t
 }
 
 // A replica record read through L2 (other blocks may have written it in
-// this launch).
+// this launch).  Unrolled whole: only the fields a caller uses are loaded, all
+// at once (as a loop every word went through local memory, four loads at a
+// time, several microseconds a call).  Index no array of the copy with a
+// variable -- that would keep the whole of it in memory.
 __device__ __forceinline__ RepDev load_rep(const RepDev* p) {
     RepDev r;
     const long long* src = reinterpret_cast<const long long*>(p);
     long long* dst = reinterpret_cast<long long*>(&r);
-#pragma unroll 4
+#pragma unroll
     for (int i = 0; i < (int)(sizeof(RepDev) / 8); ++i) dst[i] = __ldcg(src + i);
     return r;
 }
@@ -495,7 +502,7 @@ __device__ __forceinline__ bool rebuild_needed(const Dev& d, const StepParams& s
                                                double box0, double box_build0, unsigned max_disp_bits,
                                                double rlist) {
     const int steps_since = steps_since0 + (sp.do_drift ? 1 : 0);
-    const double sc = __ddiv_rn(box0, box_build0);
+    const double sc = box0 == box_build0 ? 1.0 : __ddiv_rn(box0, box_build0);
     const double maxd = (double)__uint_as_float(max_disp_bits);
     const double limit = __dsub_rn(__dsub_rn(__dmul_rn(sc, rlist), d.rcmax), __dmul_rn(1e-5, rlist));
     return sp.force_rebuild || rebuild || (__dmul_rn(2.0, maxd) > limit) ||
