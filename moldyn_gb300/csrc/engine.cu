@@ -22,7 +22,12 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
+#include <utility>
 #include <vector>
+
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include "../../include/mdgb.h"
 #include "host_math.h"
@@ -1422,6 +1427,62 @@ int get_coupling_impl(mdgb_engine* e, mdgb_thermostat* th, mdgb_barostat* ba) {
     return MDGB_OK;
 }
 
+// The caller's output pages that are mapped, marked accessed by host threads
+// before the device writes them.  The GPU reaches pageable memory through the
+// host's page tables and takes a page whose access flag the host has cleared
+// since its last use as a fault of about 10 us, one after the other: an
+// 8M-atom state (704 MB) took 4.2 ms to copy where no flag was cleared and 30
+// to 100 ms where many were.  A host thread sets a flag in about 0.1 us.  Pages
+// not mapped yet (a buffer's first use) are left to the device, which gets
+// them in 26 to 58 ms for that state where host threads took 250 ms.  The
+// contents stay; the copies are issued after the threads are done.  Below
+// MIN_BYTES the time this takes shows (0.1 ms of 8 at 88 MB) and what it saves
+// does not.
+void settle_pages(const std::vector<std::pair<char*, size_t>>& out) {
+    constexpr size_t MIN_BYTES = size_t(128) << 20;
+    constexpr size_t PAGES_PER_THREAD = 2048;
+    size_t total = 0;
+    for (auto& o : out) total += o.second;
+    const long ps = sysconf(_SC_PAGESIZE);
+    if (total < MIN_BYTES || ps <= 0) return;
+    const size_t page = (size_t)ps;
+    std::vector<std::thread> pool;
+    try {
+        struct Run { char* base; std::vector<unsigned char> mapped; };
+        std::vector<Run> runs;
+        size_t pages = 0;
+        for (auto& o : out) {
+            // whole pages inside the buffer (its ragged ends stay as they are)
+            char* b = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(o.first) + page - 1) / page * page);
+            char* e = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(o.first) + o.second) / page * page);
+            if (e <= b) continue;
+            Run r{b, std::vector<unsigned char>((size_t)(e - b) / page)};
+            if (mincore(b, (size_t)(e - b), r.mapped.data()) != 0) continue;
+            pages += r.mapped.size();
+            runs.push_back(std::move(r));
+        }
+        const size_t nt = std::max<size_t>(1, std::min({(size_t)8, (size_t)std::thread::hardware_concurrency(),
+                                                         pages / PAGES_PER_THREAD}));
+        auto work = [&runs, page, nt](size_t t) {
+            for (const Run& r : runs) {
+                const size_t n = r.mapped.size();
+                for (size_t k = n * t / nt; k < n * (t + 1) / nt; ++k)
+                    if (r.mapped[k] & 1) {
+                        volatile char* p = r.base + k * page;
+                        *p = *p;
+                    }
+            }
+        };
+        try {
+            for (size_t t = 1; t < nt; ++t) pool.emplace_back(work, t);
+        } catch (...) {   // no thread to be had: its pages stay as they are
+        }
+        work(0);
+        for (auto& th : pool) th.join();
+    } catch (...) {       // out of memory: the copies work all the same
+    }
+}
+
 // The requested arrays gathered into the caller's order on the device, then
 // copied straight into the caller's buffers (pageable memory is fine).
 int download_impl(mdgb_engine* e, double* pos, double* vel, double* force, double* pot, double* temp,
@@ -1438,6 +1499,14 @@ int download_impl(mdgb_engine* e, double* pos, double* vel, double* force, doubl
         void* args[] = {(void*)&e->dev, (void*)&op, (void*)&ov, (void*)&of, (void*)&oe, (void*)&ot};
         CU(cudaLaunchKernel((const void*)k_gather_out, dim3((unsigned)((N + 255) / 256)), dim3(256), args, 0,
                             e->stream));
+    }
+    if (e->host_direct) {
+        std::vector<std::pair<char*, size_t>> out;
+        auto add = [&](double* p, size_t doubles) {
+            if (p) out.emplace_back(reinterpret_cast<char*>(p), doubles * sizeof(double));
+        };
+        add(pos, 3 * N); add(vel, 3 * N); add(force, 3 * N); add(pot, N); add(temp, N);
+        settle_pages(out);
     }
     if (pos) CU(cudaMemcpyAsync(pos, op, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
     if (vel) CU(cudaMemcpyAsync(vel, ov, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
