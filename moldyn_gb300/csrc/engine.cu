@@ -39,6 +39,8 @@ __global__ void k_macro(Dev d, StepParams sp, int sel);
 __global__ void k_apply_pending(Dev d);
 __global__ void k_apply_pending_box(Dev d);
 __global__ void k_gather_out(Dev d, double*, double*, double*, double*, double*);
+__global__ void k_type_count(const int4* tiles, const uint16_t* type, int ntypes, int* count, int* bad);
+__global__ void k_type_scan(const int2* reps, int ntypes, int* count, int* total);
 __global__ void k_scatter_in(Dev d, const double*, const double*, const uint16_t*, const int*, int);
 __global__ void k_scatter_forces(Dev d, const double*, const double*, const double*);
 __global__ void k_pairs(Dev d, long long capacity, int* out_i, int* out_j, unsigned long long* count);
@@ -127,8 +129,12 @@ struct mdgb_engine {
     // from it directly (no pinned host copy: on this platform the copy engine
     // reads and writes pageable memory at full link speed)
     double* d_out = nullptr;     // [11][N] caller-order staging (pos, vel, force, potential, temp)
-    int* d_in_i = nullptr;       // [N] reference ranks (several types)
     uint16_t* d_in_t = nullptr;  // [N] caller type ids
+    // uploads of several types: tiles, counts per tile and type, totals (grown
+    // to the largest such upload; not part of the state's allocations, since
+    // they are needed before a state may be given up)
+    void* type_buf = nullptr;
+    size_t type_bytes = 0;
     int* h_err = nullptr;        // pinned
     unsigned long long* trace_buf = nullptr;  // per-phase ns of k_pre (MDGB_FLAG_TRACE)
     int lb_grid = 1, lm_grid = 1, lb_cap = -1, lb_ncells = -1;  // list-build launch shapes for (cap, cells)
@@ -1086,6 +1092,63 @@ int autotune_tpa(mdgb_engine* e) {
     return rebuild_lists(e);  // lists in the chosen layouts
 }
 
+// Counts of every type per tile (exclusive over the tiles of a replica when
+// done, [tile][MAX_TYPES] in *count_out) and each replica's type offsets.
+// Refuses a type id >= ntypes and a type without atoms in some replica.
+int count_types(mdgb_engine* e, int N, const uint16_t* type, int ntypes, const std::vector<int4>& tiles,
+                std::vector<RepDev>& reps, int** count_out) {
+    const size_t nt = tiles.size(), nr = reps.size();
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t s_cnt = up(nt * MAX_TYPES * sizeof(int)), s_tot = up((nr * MAX_TYPES + 1) * sizeof(int)),
+                 s_tiles = up(nt * sizeof(int4)), s_reps = up(nr * sizeof(int2)),
+                 s_type = e->host_direct ? 0 : up((size_t)N * sizeof(uint16_t));
+    const size_t bytes = s_cnt + s_tot + s_tiles + s_reps + s_type;
+    if (bytes > e->type_bytes) {
+        if (e->type_buf) cudaFree(e->type_buf);
+        e->type_buf = nullptr;
+        e->type_bytes = 0;
+        CU(cudaMalloc(&e->type_buf, bytes));
+        e->type_bytes = bytes;
+    }
+    char* q = static_cast<char*>(e->type_buf);
+    int* count = reinterpret_cast<int*>(q); q += s_cnt;
+    int* total = reinterpret_cast<int*>(q); q += s_tot;
+    int4* d_tiles = reinterpret_cast<int4*>(q); q += s_tiles;
+    int2* d_reps = reinterpret_cast<int2*>(q); q += s_reps;
+    std::vector<int2> spans(nr);
+    for (size_t r = 0; r < nr; ++r) spans[r] = make_int2(reps[r].tile_begin, reps[r].ntiles);
+    CU(cudaMemcpyAsync(d_tiles, tiles.data(), nt * sizeof(int4), cudaMemcpyHostToDevice, e->stream));
+    CU(cudaMemcpyAsync(d_reps, spans.data(), nr * sizeof(int2), cudaMemcpyHostToDevice, e->stream));
+    int* bad = total + nr * MAX_TYPES;
+    CU(cudaMemsetAsync(bad, 0, sizeof(int), e->stream));
+    const uint16_t* d_type = type;   // read where it lies, as the scatter kernel does
+    if (!e->host_direct) {
+        CU(cudaMemcpyAsync(q, type, (size_t)N * sizeof(uint16_t), cudaMemcpyHostToDevice, e->stream));
+        d_type = reinterpret_cast<const uint16_t*>(q);
+    }
+    k_type_count<<<(unsigned)nt, TILE, 0, e->stream>>>(d_tiles, d_type, ntypes, count, bad);
+    k_type_scan<<<(unsigned)nr, 256, 0, e->stream>>>(d_reps, ntypes, count, total);
+    CU(cudaGetLastError());
+    std::vector<int> tot(nr * MAX_TYPES + 1);
+    CU(cudaMemcpyAsync(tot.data(), total, tot.size() * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+    CU(cudaStreamSynchronize(e->stream));
+    if (tot.back()) return fail(e, MDGB_ERR_INVALID_ARGUMENT, "type id >= ntypes");
+    for (size_t r = 0; r < nr; ++r) {
+        RepDev& R = reps[r];
+        for (int t = 0; t < ntypes; ++t) {
+            const int c = tot[r * MAX_TYPES + t];
+            if (c == 0)
+                return fail(e, MDGB_ERR_INVALID_ARGUMENT,
+                            "every type 0..ntypes-1 needs at least one atom in every replica "
+                            "(the reference indexes particles[type][0])");
+            R.type_off[t + 1] = R.type_off[t] + c;
+            R.last_type_count = c;
+        }
+    }
+    *count_out = count;
+    return MDGB_OK;
+}
+
 // Upload of a state (one replica or an ensemble).  An upload whose shape
 // (atoms, replicas, tiles, cells, reduction chunks) equals the previous one
 // keeps the device allocations, the neighbour list (if large enough), the
@@ -1111,40 +1174,30 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
         if (!(mass_per_type[t] > 0.0)) return fail(e, MDGB_ERR_INVALID_ARGUMENT, "mass must be positive");
     const int N = (int)n;
 
-    // reference ranks (type-major within each replica) and per-replica type
-    // offsets; with one type the rank is the index itself and the type ids are
-    // checked on the device
-    std::vector<int> rank;
+    // tiles of each replica, and its type offsets (the reference's order is
+    // type-major).  With one type the rank is the index itself and the type ids
+    // are checked by the scatter kernel; with several the device counts the
+    // types per tile and scans the counts, which gives the scatter kernel every
+    // atom's rank (a loop over the atoms here took 1.3 ms of a 500,000-atom
+    // frame's 2.8).
     std::vector<RepDev> reps(nrep, RepDev{});
+    std::vector<int4> tiles;
+    for (int r = 0; r < nrep; ++r) {
+        RepDev& R = reps[r];
+        const int nr = (int)(offsets[r + 1] - offsets[r]);
+        R.begin = offsets[r];
+        R.n = nr;
+        R.tile_begin = (int)tiles.size();
+        for (int b = 0; b < nr; b += TILE) tiles.push_back(make_int4(r, (int)(offsets[r] + b), std::min(TILE, nr - b), 0));
+        R.ntiles = (int)tiles.size() - R.tile_begin;
+        R.type_off[0] = 0;
+        for (int t = 1; t <= MAX_TYPES; ++t) R.type_off[t] = nr;
+        R.last_type_count = nr;
+    }
+    int* d_type_count = nullptr;
     if (ntypes > 1) {
-        rank.resize(N);
-        for (int r = 0; r < nrep; ++r) {
-            std::vector<int64_t> cnt(ntypes + 1, 0);
-            for (int64_t i = offsets[r]; i < offsets[r + 1]; ++i) {
-                if (type[i] >= ntypes) return fail(e, MDGB_ERR_INVALID_ARGUMENT, "type id >= ntypes");
-                cnt[type[i] + 1]++;
-            }
-            for (int t = 0; t < ntypes; ++t)
-                if (cnt[t + 1] == 0)
-                    return fail(e, MDGB_ERR_INVALID_ARGUMENT,
-                                "every type 0..ntypes-1 needs at least one atom in every replica "
-                                "(the reference indexes particles[type][0])");
-            for (int t = 0; t < ntypes; ++t) cnt[t + 1] += cnt[t];
-            RepDev& R = reps[r];
-            for (int t = 0; t <= ntypes; ++t) R.type_off[t] = (int)cnt[t];
-            for (int t = ntypes + 1; t <= MAX_TYPES; ++t) R.type_off[t] = (int)cnt[ntypes];
-            std::vector<int64_t> fill(cnt.begin(), cnt.end() - 1);
-            for (int64_t i = offsets[r]; i < offsets[r + 1]; ++i) rank[i] = (int)(offsets[r] + fill[type[i]]++);
-            R.last_type_count = (int)(cnt[ntypes] - cnt[ntypes - 1]);
-        }
-    } else {
-        for (int r = 0; r < nrep; ++r) {
-            RepDev& R = reps[r];
-            const int nr = (int)(offsets[r + 1] - offsets[r]);
-            R.type_off[0] = 0;
-            for (int t = 1; t <= MAX_TYPES; ++t) R.type_off[t] = nr;
-            R.last_type_count = nr;
-        }
+        const int rc = count_types(e, N, type, ntypes, tiles, reps, &d_type_count);
+        if (rc) return rc;
     }
 
     // potentials and list radius (host side: the cell capacity depends on it)
@@ -1156,7 +1209,6 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
     // tuning may choose)
     const bool auto_skin = skin_auto(e);
     const double rl_cells = e->rcmax + (auto_skin ? std::min(e->skin, SKIN_FRACTIONS[0] * e->rcmax) : e->skin);
-    std::vector<int4> tiles;
     std::vector<int> cell_rep;
     int max_rep_n = 0;
     double max_density = 0.0;
@@ -1164,11 +1216,6 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
         RepDev& R = reps[r];
         const int nr = (int)(offsets[r + 1] - offsets[r]);
         max_rep_n = std::max(max_rep_n, nr);
-        R.begin = offsets[r];
-        R.n = nr;
-        R.tile_begin = (int)tiles.size();
-        for (int b = 0; b < nr; b += TILE) tiles.push_back(make_int4(r, (int)(offsets[r] + b), std::min(TILE, nr - b), 0));
-        R.ntiles = (int)tiles.size() - R.tile_begin;
         double prod = 1.0;
         for (int a = 0; a < 3; ++a) {
             const double L = boxes[3 * r + a];
@@ -1294,7 +1341,7 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
             (rc = dalloc(e, &e->snap_pos, N)) || (rc = dalloc(e, &e->snap_d, 8 * (size_t)N)) ||
             (rc = dalloc(e, &e->snap_i, 4 * (size_t)N)) || (rc = dalloc(e, &e->snap_mir0, N)) ||
             (rc = dalloc(e, &e->snap_rep, nrep)) || (rc = dalloc(e, &e->d_out, 11 * (size_t)N)) ||
-            (rc = dalloc(e, &e->d_in_i, N)) || (rc = dalloc(e, &e->d_in_t, N)))
+            (rc = dalloc(e, &e->d_in_t, N)))
             return rc;
     }
     if (!e->h_err) CU(cudaMallocHost((void**)&e->h_err, 4 * sizeof(int)));
@@ -1355,25 +1402,21 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
     const double* dpos = pos;
     const double* vptr = vel;
     const uint16_t* tptr = type;
-    const int* rptr = ntypes > 1 ? rank.data() : nullptr;
     if (!e->host_direct) {
         double* spos = e->d_out;
         double* svel = e->d_out + 3 * (size_t)N;
         CU(cudaMemcpyAsync(spos, pos, 3 * (size_t)N * sizeof(double), cudaMemcpyHostToDevice, e->stream));
         if (vel) CU(cudaMemcpyAsync(svel, vel, 3 * (size_t)N * sizeof(double), cudaMemcpyHostToDevice, e->stream));
         CU(cudaMemcpyAsync(e->d_in_t, type, (size_t)N * sizeof(uint16_t), cudaMemcpyHostToDevice, e->stream));
-        if (ntypes > 1)
-            CU(cudaMemcpyAsync(e->d_in_i, rank.data(), (size_t)N * sizeof(int), cudaMemcpyHostToDevice, e->stream));
         dpos = spos;
         vptr = vel ? svel : nullptr;
         tptr = e->d_in_t;
-        rptr = ntypes > 1 ? e->d_in_i : nullptr;
     }
     int nt = ntypes;
-    void* args[] = {(void*)&e->dev, (void*)&dpos, (void*)&vptr, (void*)&tptr, (void*)&rptr, (void*)&nt};
-    CU(cudaLaunchKernel((const void*)k_scatter_in, dim3((N + 255) / 256), dim3(256), args, 0, e->stream));
-    // the kernel may read the caller's arrays and the local rank table: done
-    // before anything below can return
+    void* args[] = {(void*)&e->dev, (void*)&dpos, (void*)&vptr, (void*)&tptr, (void*)&d_type_count, (void*)&nt};
+    CU(cudaLaunchKernel((const void*)k_scatter_in, dim3(ntiles), dim3(TILE), args, 0, e->stream));
+    // the kernel may read the caller's arrays: done before anything below can
+    // return
     if (e->host_direct && ntypes > 1) CU(cudaStreamSynchronize(e->stream));
     e->thermo_on = e->baro_on = e->thermo_nh = false;
     if (ntypes == 1) {   // the type ids were checked on the device
@@ -1569,6 +1612,7 @@ mdgb_engine::~mdgb_engine() {
     for (auto& p : prof) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
     for (auto& p : prof_free) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
     if (h_err) cudaFreeHost(h_err);
+    if (type_buf) cudaFree(type_buf);
     for (int c = 0; c < 3; ++c) {
         if (aux[c]) cudaStreamDestroy(aux[c]);
         if (join_ev[c]) cudaEventDestroy(join_ev[c]);

@@ -2673,17 +2673,90 @@ __global__ void k_gather_out(Dev d, double* out_pos, double* out_vel, double* ou
     if (out_tmp) out_tmp[o] = d.evir[s];
 }
 
-// Caller order -> device (upload): the device order starts as the caller's;
-// the first rebuild sorts it by cell.  in_rank null: one type, the rank is the
-// index.  A type id >= ntypes is flagged (E_INPUT) and replaced by 0, so no
-// later kernel indexes the pair table with it.
-__global__ void k_scatter_in(Dev d, const double* in_pos, const double* in_vel, const uint16_t* in_type,
-                             const int* in_rank, int ntypes) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+// Atoms of each type in every tile (one block each); bad: a type id >= ntypes.
+__global__ void __launch_bounds__(TILE) k_type_count(const int4* tiles, const uint16_t* type, int ntypes, int* count,
+                                                     int* bad) {
+    __shared__ int c[MAX_TYPES];
+    const int4 tl = tiles[blockIdx.x];
+    const bool act = (int)threadIdx.x < tl.z;
+    const int ty = act ? (int)type[tl.y + threadIdx.x] : -1;
+    if (ty >= ntypes) atomicOr(bad, 1);
+    if (threadIdx.x < MAX_TYPES) c[threadIdx.x] = 0;
+    __syncthreads();
+    for (int t = 0; t < ntypes; ++t) {
+        const unsigned m = __ballot_sync(0xffffffffu, ty == t);
+        if ((threadIdx.x & 31) == 0 && m) atomicAdd(c + t, __popc(m));
+    }
+    __syncthreads();
+    if (threadIdx.x < MAX_TYPES) count[(size_t)blockIdx.x * MAX_TYPES + threadIdx.x] = c[threadIdx.x];
+}
+
+// The counts of a replica's tiles (reps: first tile, tiles), type by type,
+// replaced by their exclusive prefix sums; total: the replica's counts.  One
+// block per replica.
+__global__ void __launch_bounds__(256) k_type_scan(const int2* reps, int ntypes, int* count, int* total) {
+    __shared__ int wsum[8];
+    const int2 R = reps[blockIdx.x];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int t = 0; t < ntypes; ++t) {
+        int carry = 0;
+        for (int b = 0; b < R.y; b += 256) {
+            const int i = b + (int)threadIdx.x;
+            int* p = count + (size_t)(R.x + i) * MAX_TYPES + t;
+            const int v = i < R.y ? *p : 0;
+            int incl = v;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, off);
+                if (lane >= off) incl += y;
+            }
+            __syncthreads();
+            if (lane == 31) wsum[w] = incl;
+            __syncthreads();
+            int before = carry, all = 0;
+            for (int k = 0; k < 8; ++k) {
+                if (k < w) before += wsum[k];
+                all += wsum[k];
+            }
+            if (i < R.y) *p = before + incl - v;
+            carry += all;
+        }
+        if (threadIdx.x == 0) total[blockIdx.x * MAX_TYPES + t] = carry;
+    }
+}
+
+// Caller order -> device (upload), one block per tile: the device order starts
+// as the caller's; the first rebuild sorts it by cell.  type_count: with
+// several types, the atoms of each type in the replica's earlier tiles
+// (k_type_scan), from which the atom's rank follows; null: one type, the rank
+// is the index, and a type id >= ntypes is flagged (E_INPUT) and replaced by
+// 0, so no later kernel indexes the pair table with it.
+__global__ void __launch_bounds__(TILE) k_scatter_in(Dev d, const double* in_pos, const double* in_vel,
+                                                     const uint16_t* in_type, const int* type_count, int ntypes) {
+    __shared__ int wcount[TILE / 32][MAX_TYPES];
+    const int4 tl = d.tiles[blockIdx.x];
+    const bool act = (int)threadIdx.x < tl.z;
+    const int s = tl.y + threadIdx.x;
     const int N = d.ntot;
-    if (s >= N) return;
-    int ty = (int)in_type[s];
+    int ty = act ? (int)in_type[s] : -1;
     if (ty >= ntypes) { atomicOr(d.err, E_INPUT); ty = 0; }
+    int rk = s;
+    if (type_count) {
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        int within = 0;
+        for (int t = 0; t < ntypes; ++t) {
+            const unsigned m = __ballot_sync(0xffffffffu, ty == t);
+            if (lane == 0) wcount[w][t] = __popc(m);
+            if (ty == t) within = __popc(m & ((1u << lane) - 1u));
+        }
+        __syncthreads();
+        if (act) {
+            for (int k = 0; k < w; ++k) within += wcount[k][ty];
+            const RepDev* R = d.rep + tl.x;
+            rk = (int)R->begin + R->type_off[ty] + type_count[(size_t)blockIdx.x * MAX_TYPES + ty] + within;
+        }
+    }
+    if (!act) return;
     double4_32a p;
     p.x = in_pos[3 * (size_t)s]; p.y = in_pos[3 * (size_t)s + 1]; p.z = in_pos[3 * (size_t)s + 2];
     p.w = __longlong_as_double((long long)ty);
@@ -2695,7 +2768,6 @@ __global__ void k_scatter_in(Dev d, const double* in_pos, const double* in_vel, 
     d.epot[s] = 0.0;
     d.evir[s] = 0.0;
     d.orig[s] = s;
-    int rk = in_rank ? in_rank[s] : s;
     if (rk < 0 || rk >= N) { atomicOr(d.err, E_BOUNDS); rk = s; }
     d.rank[s] = rk;
     d.slot_of_rank[rk] = s;
