@@ -44,6 +44,12 @@ __device__ __forceinline__ double min_image_ref(double r, double L) {
     return r;
 }
 
+// |r| > L/2, as min_image_ref decides it.
+__device__ __forceinline__ bool beyond_half(double r, double L) {
+    return ((unsigned long long)__double_as_longlong(r) & 0x7FFFFFFFFFFFFFFFull) >
+           (unsigned long long)__double_as_longlong(L) - (1ull << 52);
+}
+
 // The terms of one pair, from the side of the atom the displacement starts at.
 struct PairTerms {
     double gx, gy, gz, u, t;

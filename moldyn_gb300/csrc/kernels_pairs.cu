@@ -10,7 +10,7 @@
 //                 virial terms once, from the side of its owner.  Candidates
 //                 outside r_cut (FP32 prefilter) are dropped before the FP64
 //                 work: a warp queues what passes and computes 32 at a time.
-//   k_pair_sums   one thread per atom: walks its list in list order and adds
+//   k_pair_sums   four lanes per atom: walk its list in list order and add
 //                 the records (the partner's with the force negated), then the
 //                 second half kick and, on NVE chunks, the next step's kick
 //                 and drift.
@@ -26,13 +26,15 @@
 // by binary search in its (ascending) list.  A pair listed by the later atom
 // only (within rounding of the list radius, far outside r_cut) has none.
 //
-// 256,000 atoms, one NVE pass: 3.66 ms with k_force_fp64; 0.42 + 0.23 ms in
+// 256,000 atoms, one NVE pass: 3.66 ms with k_force_fp64; 0.39 + 0.21 ms in
 // tree order here, and 0.41 ms more at a rebuild (every ninth step).  23,256
-// atoms in reference order: 0.53 -> 0.18 ms.  k_pair_terms keeps the FP64 pipe
-// busy 82 % of the time; k_pair_sums waits for its record gathers (FP64 43 %).
+// atoms in reference order: 0.53 -> 0.14 ms.  k_pair_terms keeps the FP64 pipe
+// busy over 80 % of the time; k_pair_sums waits for its record gathers.
+// (Summing runs of tiles on a second stream beside the next run's terms was
+// slower: 15.5 to 17.7 ms for 20 steps of 256,000 atoms against 14.9.)
 #include <algorithm>
 
-#include "force_common.cuh"
+#include "force_mixed.cuh"
 
 namespace mdgb {
 
@@ -175,9 +177,15 @@ __global__ void __launch_bounds__(TILE) k_pair_terms(Dev d, int parts) {
         const int j = (int)(ij.y & IDX_MASK);
         const double4_32a pi = d.pos[ij.x], pj = d.pos[j];
         const PairDev& P = d.pair[type_of(pi) * MAX_TYPES + type_of(pj)];
-        const double rx = min_image_ref(__dsub_rn(pj.x, pi.x), box[0]);   // potential.rs:181-200
-        const double ry = min_image_ref(__dsub_rn(pj.y, pi.y), box[1]);
-        const double rz = min_image_ref(__dsub_rn(pj.z, pi.z), box[2]);
+        double rx = __dsub_rn(pj.x, pi.x), ry = __dsub_rn(pj.y, pi.y), rz = __dsub_rn(pj.z, pi.z);
+        // potential.rs:181-200, by a vote: most warps hold no pair across the
+        // boundary (as predicated adds the three would be issued for every warp)
+        const bool across = beyond_half(rx, box[0]) || beyond_half(ry, box[1]) || beyond_half(rz, box[2]);
+        if (__any_sync(__activemask(), across)) {
+            rx = min_image_ref(rx, box[0]);
+            ry = min_image_ref(ry, box[1]);
+            rz = min_image_ref(rz, box[2]);
+        }
         const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), __dmul_rn(rz, rz));
         PairTerms o;
         o.u = 0.0;
@@ -222,40 +230,62 @@ __global__ void __launch_bounds__(TILE) k_pair_terms(Dev d, int parts) {
 }
 
 // ---------------------------------------------------------------------------
-// Per-atom sums in list order.  FORCE: a fused NVE pass, whose potential and
-// virial nobody reads (the chunk's last pass writes them) -- no record is then
-// read but its one sector, and neither forces nor sums are stored.
+// Per-atom sums in list order, four lanes per atom: lane c adds component c of
+// the records (the fourth potential and virial), so an atom's lanes read a
+// record's sector together and a warp adds for eight atoms at a time -- the
+// same FP64 work as a thread per atom (three or five adds for 32 atoms against
+// one or two for eight) with four times the loads in flight, which is what
+// bounds it: 71 -> 36 us at 23,256 atoms, 235 -> 209 us at 256,000.  The block's first warp then finishes its 32 atoms, a thread
+// each.  FORCE: a fused NVE pass, whose potential and virial nobody reads (the
+// chunk's last pass writes them).
+constexpr int SUM_LANES = 4;
+
 template <bool KICK, bool FORCE>
 __global__ void __launch_bounds__(TILE) k_pair_sums(Dev d, StepParams sp) {
     if (chunk_failed(d)) return;
+    constexpr int PER = TILE / SUM_LANES;
     __shared__ float tcs[8];
+    __shared__ double S[5][PER];
     const int N = d.ntot;
-    const int4 tl = d.tiles[blockIdx.x];
+    const int4 tl = d.tiles[blockIdx.x / SUM_LANES];
+    const int first = (blockIdx.x % SUM_LANES) * PER;
+    if (first >= tl.z) return;
     const RepDev* R = d.rep + tl.x;
     const long long rbeg = R->begin;
     const int rn = R->n;
     if (KICK && sp.fused && threadIdx.x == 0) drift_consts(*R, tcs);
-    __syncthreads();
-    const int s = tl.y + threadIdx.x;
-    const bool act = (int)threadIdx.x < tl.z;
-    double fx = 0.0, fy = 0.0, fz = 0.0, pe = 0.0, vr = 0.0;
-    const int n = act ? d.nn[s] : 0;
-    const uint32_t* row = d.pair_of + list_index(s, 0, 1, rbeg, rn, d.cap);
-    // 32 entries at a time: which of them lie inside r_cut, then their records
-    // in order, four loaded before any is added
+    const int a = threadIdx.x / SUM_LANES, c = threadIdx.x % SUM_LANES;
+    const unsigned group = ((1u << SUM_LANES) - 1u) << (threadIdx.x & 31 & ~(SUM_LANES - 1));
+    const int s = tl.y + first + a;
+    const int n = first + a < tl.z ? d.nn[s] : 0;
+    if (KICK && threadIdx.x < PER && first + (int)threadIdx.x < tl.z) {   // the epilogue's operands, on their way
+        const int es = tl.y + first + threadIdx.x;
+        for (int k = 0; k < 3; ++k) prefetch_l2(d.vel + (size_t)k * N + es);
+        if (sp.fused) {
+            prefetch_l2(d.pos + es);
+            prefetch_l2(d.mir0 + es);
+            prefetch_l2(d.cell + es);
+        }
+    }
+    double sum = 0.0, vir = 0.0;
+    const uint32_t* row = d.pair_of + list_index(first + a < tl.z ? s : tl.y, 0, 1, rbeg, rn, d.cap);
+    const double* rec = reinterpret_cast<const double*>(d.pair_rec) + c;
+    // 32 entries at a time: which of them lie inside r_cut (a lane looks at
+    // eight), then their records in order, four loaded before any is added
     constexpr int NB = 4;
     for (int k0 = 0; k0 < n; k0 += 32) {
-        const int m = min(32, n - k0);
         uint32_t in = 0u;
-#pragma unroll 8
-        for (int q = 0; q < m; ++q) {
-            const uint32_t r = __ldg(row + (size_t)(k0 + q) * rn);
-            if (r != PAIR_NONE && __ldg(d.pair_in + (r & ~PAIR_NEG))) in |= 1u << q;
+#pragma unroll
+        for (int q = 0; q < 32 / SUM_LANES; ++q) {
+            const int k = k0 + q * SUM_LANES + c;
+            const uint32_t r = k < n ? __ldg(row + (size_t)k * rn) : PAIR_NONE;
+            if (r != PAIR_NONE && __ldg(d.pair_in + (r & ~PAIR_NEG))) in |= 1u << (q * SUM_LANES + c);
         }
+#pragma unroll
+        for (int off = SUM_LANES / 2; off > 0; off >>= 1) in |= __shfl_xor_sync(group, in, off);
         while (in) {
             uint32_t r[NB];
-            double2 a[NB], b[NB];
-            double v[NB];
+            double x[NB], v[NB];
 #pragma unroll
             for (int u = 0; u < NB; ++u) {
                 r[u] = PAIR_NONE;
@@ -265,38 +295,38 @@ __global__ void __launch_bounds__(TILE) k_pair_sums(Dev d, StepParams sp) {
 #pragma unroll
             for (int u = 0; u < NB; ++u)
                 if (r[u] != PAIR_NONE) {
-                    const double2* p = reinterpret_cast<const double2*>(d.pair_rec + (r[u] & ~PAIR_NEG));
-                    a[u] = __ldg(p);
-                    b[u] = __ldg(p + 1);
-                    if (!FORCE) v[u] = __ldg(d.pair_vir + (r[u] & ~PAIR_NEG));
+                    x[u] = __ldg(rec + 4 * (size_t)(r[u] & ~PAIR_NEG));
+                    if (!FORCE && c == 3) v[u] = __ldg(d.pair_vir + (r[u] & ~PAIR_NEG));
                 }
 #pragma unroll
             for (int u = 0; u < NB; ++u)
                 if (r[u] != PAIR_NONE) {
-                    const unsigned long long neg = (unsigned long long)(r[u] & PAIR_NEG) << 32;
-                    auto sgn = [&](double x) {
-                        return __longlong_as_double((long long)((unsigned long long)__double_as_longlong(x) ^ neg));
-                    };
-                    fx = __dadd_rn(fx, sgn(a[u].x));
-                    fy = __dadd_rn(fy, sgn(a[u].y));
-                    fz = __dadd_rn(fz, sgn(b[u].x));
-                    if (!FORCE) {
-                        pe = __dadd_rn(pe, b[u].y);
-                        vr = __dadd_rn(vr, v[u]);
-                    }
+                    // the partner's record: the force negated
+                    const unsigned long long neg = c < 3 ? (unsigned long long)(r[u] & PAIR_NEG) << 32 : 0ull;
+                    const double y =
+                        __longlong_as_double((long long)((unsigned long long)__double_as_longlong(x[u]) ^ neg));
+                    if (!FORCE || c < 3) sum = __dadd_rn(sum, y);
+                    if (!FORCE && c == 3) vir = __dadd_rn(vir, v[u]);
                 }
         }
     }
+    S[c][a] = sum;
+    if (!FORCE && c == 3) S[4][a] = vir;
+    __syncthreads();
+    if (threadIdx.x >= PER) return;
     float disp = 0.f;
-    if (act) {
+    if (first + (int)threadIdx.x < tl.z) {
+        const int es = tl.y + first + threadIdx.x;
+        const double fx = S[0][threadIdx.x], fy = S[1][threadIdx.x], fz = S[2][threadIdx.x];
         if (!FORCE) {
-            d.frc[s] = fx; d.frc[N + s] = fy; d.frc[2 * N + s] = fz;
-            d.epot[s] = pe; d.evir[s] = vr;
+            d.frc[es] = fx; d.frc[N + es] = fy; d.frc[2 * N + es] = fz;
+            d.epot[es] = S[3][threadIdx.x]; d.evir[es] = S[4][threadIdx.x];
         }
-        if (KICK) disp = kick_and_drift<false>(d, sp, R, tcs, s, type_of(d.pos[s]), fx, fy, fz);
+        if (KICK) disp = kick_and_drift<false>(d, sp, R, tcs, es, type_of(d.pos[es]), fx, fy, fz);
     }
     if (KICK && sp.fused) note_displacement(d, tl.x, disp);
 }
+static_assert(TILE / SUM_LANES == 32, "one warp finishes a block's atoms");
 
 // ---------------------------------------------------------------------------
 // Host side.
@@ -320,9 +350,9 @@ cudaError_t launch_pair_forces(const Dev& d, const StepParams& sp, bool kick, in
         if (force) k_pair_terms<false, true><<<grid, TILE, 0, st>>>(d, parts);
         else k_pair_terms<false, false><<<grid, TILE, 0, st>>>(d, parts);
     }
-    if (force) k_pair_sums<true, true><<<d.ntiles, TILE, 0, st>>>(d, sp);
-    else if (kick) k_pair_sums<true, false><<<d.ntiles, TILE, 0, st>>>(d, sp);
-    else k_pair_sums<false, false><<<d.ntiles, TILE, 0, st>>>(d, sp);
+    if (force) k_pair_sums<true, true><<<d.ntiles * SUM_LANES, TILE, 0, st>>>(d, sp);
+    else if (kick) k_pair_sums<true, false><<<d.ntiles * SUM_LANES, TILE, 0, st>>>(d, sp);
+    else k_pair_sums<false, false><<<d.ntiles * SUM_LANES, TILE, 0, st>>>(d, sp);
     return cudaGetLastError();
 }
 
