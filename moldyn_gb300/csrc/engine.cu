@@ -37,7 +37,8 @@ namespace mdgb {
 __global__ void k_pre(Dev d, StepParams sp);
 __global__ void k_macro(Dev d, StepParams sp, int sel);
 __global__ void k_apply_pending(Dev d);
-__global__ void k_apply_pending_box(Dev d);
+__global__ void k_snapshot(Dev d, SnapArrays a);
+__global__ void k_set_coupling(Dev d, RepCoupling c);
 __global__ void k_gather_out(Dev d, double*, double*, double*, double*, double*);
 __global__ void k_type_count(const int4* tiles, const uint16_t* type, int ntypes, int* count, int* bad);
 __global__ void k_type_scan(const int2* reps, int ntypes, int* count, int* total);
@@ -135,7 +136,13 @@ struct mdgb_engine {
     // they are needed before a state may be given up)
     void* type_buf = nullptr;
     size_t type_bytes = 0;
-    int* h_err = nullptr;        // pinned
+    // pinned: error words, replica 0's record after a step, and room for the
+    // outputs of a small download (one copy, then the host's own)
+    char* h_pin = nullptr;
+    int* h_err = nullptr;        // in h_pin
+    RepDev* h_rep = nullptr;     // in h_pin
+    bool rep_fresh = false;      // h_rep is the record the last step call left
+    bool coupling_set = false;   // some replica's coupling flags may be on
     unsigned long long* trace_buf = nullptr;  // per-phase ns of k_pre (MDGB_FLAG_TRACE)
     int lb_grid = 1, lm_grid = 1, lb_cap = -1, lb_ncells = -1;  // list-build launch shapes for (cap, cells)
     // the other position / mirror buffer of each pair (fused NVE drift)
@@ -181,6 +188,10 @@ struct mdgb_engine {
 };
 
 namespace {
+
+// Pinned memory of an engine: head (error words, one replica record), outputs.
+constexpr size_t PIN_HEAD = 1024, PIN_OUT = size_t(256) << 10;
+static_assert(64 + sizeof(RepDev) <= PIN_HEAD, "the record fits");
 
 int fail(mdgb_engine* e, int code, const std::string& msg) {
     if (e) e->err = msg;
@@ -574,6 +585,13 @@ int clear_err(mdgb_engine* e) {
     return MDGB_OK;
 }
 
+// What a chunk needs to be run again, copied aside, and the error words and the
+// barrier cleared, in one launch: for small states the eleven copies and two
+// clears were most of a step call's launches.  (From 262,144 atoms on the
+// copies themselves are what counts.)
+constexpr int SNAP_KERNEL_MAX = 262144;
+int begin_chunk(mdgb_engine* e);
+
 int snapshot(mdgb_engine* e, bool restore) {
     const size_t N = e->ntot;
     auto cp = [&](void* dst, const void* src, size_t bytes) {
@@ -605,6 +623,25 @@ int snapshot(mdgb_engine* e, bool restore) {
         CU(cp(d.mir0, e->snap_mir0, N * sizeof(float4)));
         CU(cp(d.rep, e->snap_rep, e->nrep * sizeof(RepDev)));
     }
+    return MDGB_OK;
+}
+
+int begin_chunk(mdgb_engine* e) {
+    if (e->ntot >= SNAP_KERNEL_MAX) {
+        const int rc = clear_err(e);
+        return rc ? rc : snapshot(e, false);
+    }
+    const size_t N = e->ntot;
+    Dev& d = e->dev;
+    const SnapArrays a{{e->snap_pos, e->snap_d, e->snap_d + 3 * N, e->snap_d + 6 * N, e->snap_d + 7 * N, e->snap_i,
+                        e->snap_i + N, e->snap_i + 2 * N, e->snap_i + 3 * N, e->snap_mir0, e->snap_rep},
+                       {d.pos, d.vel, d.frc, d.epot, d.evir, d.orig, d.rank, d.cell, d.slot_of_rank, d.mir0, d.rep},
+                       {N * sizeof(double4_32a), 3 * N * sizeof(double), 3 * N * sizeof(double), N * sizeof(double),
+                        N * sizeof(double), N * sizeof(int), N * sizeof(int), N * sizeof(int), N * sizeof(int),
+                        N * sizeof(float4), e->nrep * sizeof(RepDev)}};
+    void* args[] = {(void*)&e->dev, (void*)&a};
+    const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((N + 255) / 256, 4 * (size_t)e->num_sms));
+    CU(cudaLaunchKernel((const void*)k_snapshot, dim3(grid), dim3(256), args, 0, e->stream));
     return MDGB_OK;
 }
 
@@ -849,9 +886,7 @@ int step_impl(mdgb_engine* e, int64_t nsteps, double dt) {
     int retries = 0;
     while (done < nsteps) {
         const int n = (int)std::min<int64_t>(chunk, nsteps - done);
-        int rc = clear_err(e);
-        if (rc) return rc;
-        rc = snapshot(e, false);
+        int rc = begin_chunk(e);
         if (rc) return rc;
         if (e->test_hold_block >= 0) {
             // the armed failure test: this chunk eager, its first step kernel
@@ -866,8 +901,12 @@ int step_impl(mdgb_engine* e, int64_t nsteps, double dt) {
         }
         if (rc) return rc;
         int flags = 0;
+        // a single system's coupling state comes back with the error words
+        const bool with_rep = e->nrep == 1 && (e->thermo_on || e->baro_on);
+        if (with_rep) CU(cudaMemcpyAsync(e->h_rep, e->dev.rep, sizeof(RepDev), cudaMemcpyDeviceToHost, e->stream));
         rc = read_err(e, &flags);
         if (rc) return rc;
+        e->rep_fresh = with_rep;
         if (flags & E_TIMEOUT) {
             // a grid barrier gave up: the rest of the chunk did nothing; put
             // the state back as the chunk found it, so the engine stays usable
@@ -900,9 +939,7 @@ int step_impl(mdgb_engine* e, int64_t nsteps, double dt) {
     if (e->baro_on) {
         void* args[] = {(void*)&e->dev};
         CU(cudaLaunchKernel((const void*)k_apply_pending, dim3(e->ntiles), dim3(TILE), args, 0, e->stream));
-        CU(cudaLaunchKernel((const void*)k_apply_pending_box, dim3((e->nrep + 127) / 128), dim3(128), args, 0,
-                            e->stream));
-        e->st.kernel_launches += 2;
+        e->st.kernel_launches++;
     }
     e->forces_valid = true;
     return MDGB_OK;
@@ -1344,7 +1381,13 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
             (rc = dalloc(e, &e->d_in_t, N)))
             return rc;
     }
-    if (!e->h_err) CU(cudaMallocHost((void**)&e->h_err, 4 * sizeof(int)));
+    if (!e->h_pin) {
+        CU(cudaMallocHost((void**)&e->h_pin, PIN_HEAD + PIN_OUT));
+        e->h_err = reinterpret_cast<int*>(e->h_pin);
+        e->h_rep = reinterpret_cast<RepDev*>(e->h_pin + 64);
+    }
+    e->coupling_set = false;
+    e->rep_fresh = false;
     CU(cudaMemcpyAsync((void*)d.pair, pair_tab.data(), pair_tab.size() * sizeof(PairDev), cudaMemcpyHostToDevice,
                        e->stream));
 
@@ -1432,6 +1475,28 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
 
 int set_coupling_impl(mdgb_engine* e, const mdgb_thermostat* th, const mdgb_barostat* ba) {
     if (!e->has_state) return fail(e, MDGB_ERR_NO_STATE, "no state uploaded");
+    e->rep_fresh = false;
+    if (!th && !ba && !e->coupling_set) return MDGB_OK;   // off already
+    if (e->nrep == 1) {
+        RepCoupling c{};
+        c.thermo_on = th ? 1 : 0;
+        if (th) {
+            if (th->kind != MDGB_THERMOSTAT_BERENDSEN && th->kind != MDGB_THERMOSTAT_NOSE_HOOVER)
+                return fail(e, MDGB_ERR_INVALID_ARGUMENT, "unknown thermostat kind");
+            c.thermo_kind = th->kind;
+            c.th_tau = th->tau; c.th_T0 = th->target_temperature; c.lambda = th->lambda; c.psi = th->psi;
+        }
+        c.baro_on = ba ? 1 : 0;
+        if (ba) { c.ba_beta = ba->beta; c.ba_tau = ba->tau; c.ba_P0 = ba->target_pressure; c.myu = ba->myu; }
+        e->thermo_nh = th && th->kind == MDGB_THERMOSTAT_NOSE_HOOVER;
+        e->thermo_on = th != nullptr;
+        e->baro_on = ba != nullptr;
+        e->coupling_set = th || ba;
+        void* args[] = {(void*)&e->dev, (void*)&c};
+        CU(cudaLaunchKernel((const void*)k_set_coupling, dim3(1), dim3(32), args, 0, e->stream));
+        return MDGB_OK;
+    }
+    e->coupling_set = th || ba;
     CU(cudaMemcpyAsync(e->rep_host.data(), e->dev.rep, e->nrep * sizeof(RepDev), cudaMemcpyDeviceToHost, e->stream));
     CU(cudaStreamSynchronize(e->stream));
     bool any_nh = false;
@@ -1460,6 +1525,12 @@ int set_coupling_impl(mdgb_engine* e, const mdgb_thermostat* th, const mdgb_baro
 }
 
 int get_coupling_impl(mdgb_engine* e, mdgb_thermostat* th, mdgb_barostat* ba) {
+    if (!th && !ba) return MDGB_OK;
+    if (e->nrep == 1 && e->rep_fresh) {
+        if (th) { th->lambda = e->h_rep->lambda; th->psi = e->h_rep->psi; }
+        if (ba) ba->myu = e->h_rep->myu;
+        return MDGB_OK;
+    }
     CU(cudaMemcpyAsync(e->rep_host.data(), e->dev.rep, e->nrep * sizeof(RepDev), cudaMemcpyDeviceToHost, e->stream));
     CU(cudaStreamSynchronize(e->stream));
     for (int r = 0; r < e->nrep; ++r) {
@@ -1543,6 +1614,23 @@ int download_impl(mdgb_engine* e, double* pos, double* vel, double* force, doubl
         CU(cudaLaunchKernel((const void*)k_gather_out, dim3((unsigned)((N + 255) / 256)), dim3(256), args, 0,
                             e->stream));
     }
+    const size_t span = 11 * N * sizeof(double);
+    if (span <= PIN_OUT && e->nrep == 1) {
+        // small: everything gathered in one copy (and the record with it), then
+        // the host's own
+        double* hp = reinterpret_cast<double*>(e->h_pin + PIN_HEAD);
+        if (op || ov || of || oe || ot) CU(cudaMemcpyAsync(hp, o, span, cudaMemcpyDeviceToHost, e->stream));
+        if (boxes) CU(cudaMemcpyAsync(e->h_rep, e->dev.rep, sizeof(RepDev), cudaMemcpyDeviceToHost, e->stream));
+        CU(cudaStreamSynchronize(e->stream));
+        if (pos) std::memcpy(pos, hp, 3 * N * sizeof(double));
+        if (vel) std::memcpy(vel, hp + 3 * N, 3 * N * sizeof(double));
+        if (force) std::memcpy(force, hp + 6 * N, 3 * N * sizeof(double));
+        if (pot) std::memcpy(pot, hp + 9 * N, N * sizeof(double));
+        if (temp) std::memcpy(temp, hp + 10 * N, N * sizeof(double));
+        if (boxes)
+            for (int a = 0; a < 3; ++a) boxes[a] = e->h_rep->box[a];
+        return MDGB_OK;
+    }
     if (e->host_direct) {
         std::vector<std::pair<char*, size_t>> out;
         auto add = [&](double* p, size_t doubles) {
@@ -1611,7 +1699,7 @@ mdgb_engine::~mdgb_engine() {
     free_state(this);
     for (auto& p : prof) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
     for (auto& p : prof_free) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
-    if (h_err) cudaFreeHost(h_err);
+    if (h_pin) cudaFreeHost(h_pin);
     if (type_buf) cudaFree(type_buf);
     for (int c = 0; c < 3; ++c) {
         if (aux[c]) cudaStreamDestroy(aux[c]);

@@ -36,6 +36,7 @@
 // wrap, reductions, coupling factors) keeps the reference's unfused
 // multiply-then-add rounding unless a fused operation is written out.
 #include <algorithm>
+#include <atomic>
 
 #include "force_mixed.cuh"
 #include "list_direct.cuh"
@@ -2583,9 +2584,20 @@ __global__ void __launch_bounds__(TILE, 4) k_steps(Dev d_in, StepParams sp_in, i
 // Host side of k_steps: resident blocks per SM.
 
 cudaError_t steps_init(int* blocks_per_sm) {
-    const cudaError_t err = cudaFuncSetAttribute(k_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, STEPS_SMEM);
+    // a property of the device: asked once for each (not on every new engine)
+    static std::atomic<int> known[64];
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) return err;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_steps, TILE, STEPS_SMEM);
+    const bool slot = dev >= 0 && dev < 64;
+    if (slot && known[dev].load() > 0) {
+        *blocks_per_sm = known[dev].load();
+        return cudaSuccess;
+    }
+    err = cudaFuncSetAttribute(k_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, STEPS_SMEM);
+    if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_steps, TILE, STEPS_SMEM);
+    if (err == cudaSuccess && slot) known[dev].store(*blocks_per_sm);
+    return err;
 }
 
 cudaError_t launch_steps(const Dev& d, const StepParams& sp, int n, bool naive, int max_blocks, cudaStream_t st) {
@@ -2624,32 +2636,78 @@ __global__ void __launch_bounds__(TILE, 6) k_macro(Dev d, StepParams sp, int sel
     sums_then<1>(d, [&](int b, int n) { phase_finalize2(d, sp, false, sel, b, n); });
 }
 
-// End of an mdgb_step call: finish the barostat update of the last step
-// (x *= mu; the box part was applied... here as well, once per type).
+// End of an mdgb_step call: finish the barostat update of the last step: x *=
+// mu, then (the last block, when every block has read the factor) the box,
+// once per type.
 __global__ void __launch_bounds__(TILE) k_apply_pending(Dev d) {
-    const int t = blockIdx.x;
-    if (t >= d.ntiles) return;
-    const int4 tl = d.tiles[t];
+    __shared__ int last;
+    const int4 tl = d.tiles[blockIdx.x];
     const double f = d.rep[tl.x].pending;
-    if (f == 1.0) return;
-    const int s = tl.y + threadIdx.x;
-    if ((int)threadIdx.x < tl.z) {
-        double4_32a p = d.pos[s];
-        p.x = __dmul_rn(p.x, f); p.y = __dmul_rn(p.y, f); p.z = __dmul_rn(p.z, f);
-        d.pos[s] = p;
+    if (f != 1.0) {
+        const int s = tl.y + threadIdx.x;
+        if ((int)threadIdx.x < tl.z) {
+            double4_32a p = d.pos[s];
+            p.x = __dmul_rn(p.x, f); p.y = __dmul_rn(p.y, f); p.z = __dmul_rn(p.z, f);
+            d.pos[s] = p;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(d.bar + 6, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    for (int r = threadIdx.x; r < d.nrep; r += blockDim.x) {
+        RepDev* W = d.rep + r;
+        const double g = W->pending;
+        if (g == 1.0) continue;
+        for (int k = 0; k < d.ntypes; ++k)
+            for (int a = 0; a < 3; ++a) W->box[a] *= g;
+        for (int a = 0; a < 3; ++a) W->cs[a] = W->box[a] / (double)W->nc[a];
+        W->pending = 1.0;
+    }
+    if (threadIdx.x == 0) d.bar[6] = 0u;
+}
+
+// The arrays a chunk may have to be run again from, copied aside (each with the
+// widest words its addresses and length allow), and the error words and the
+// barrier cleared (bar[5] on are kept).
+template <class T>
+__device__ __forceinline__ void copy_words(void* dst, const void* src, size_t bytes) {
+    const size_t n = bytes / sizeof(T), step = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step)
+        static_cast<T*>(dst)[i] = static_cast<const T*>(src)[i];
+}
+__global__ void __launch_bounds__(256) k_snapshot(Dev d, SnapArrays a) {
+#pragma unroll 1
+    for (int k = 0; k < 11; ++k) {
+        const uintptr_t bits = (uintptr_t)a.dst[k] | (uintptr_t)a.src[k] | (uintptr_t)a.bytes[k];
+        if (!(bits & 15)) copy_words<uint4>(a.dst[k], a.src[k], a.bytes[k]);
+        else if (!(bits & 7)) copy_words<uint2>(a.dst[k], a.src[k], a.bytes[k]);
+        else copy_words<uint32_t>(a.dst[k], a.src[k], a.bytes[k]);
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 8) {
+        if (threadIdx.x < 2) d.err[threadIdx.x] = 0;
+        if (threadIdx.x < 5) d.bar[threadIdx.x] = 0u;
     }
 }
 
-__global__ void k_apply_pending_box(Dev d) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= d.nrep) return;
-    RepDev* W = d.rep + r;
-    const double f = W->pending;
-    if (f == 1.0) return;
-    for (int k = 0; k < d.ntypes; ++k)
-        for (int a = 0; a < 3; ++a) W->box[a] *= f;
-    for (int a = 0; a < 3; ++a) W->cs[a] = W->box[a] / (double)W->nc[a];
-    W->pending = 1.0;
+// A single system's coupling settings.
+__global__ void k_set_coupling(Dev d, RepCoupling c) {
+    if (threadIdx.x != 0) return;
+    RepDev* W = d.rep;
+    W->thermo_on = c.thermo_on;
+    if (c.thermo_on) {
+        W->thermo_kind = c.thermo_kind;
+        W->th_tau = c.th_tau; W->th_T0 = c.th_T0;
+        W->lambda = c.lambda; W->psi = c.psi;
+    }
+    W->baro_on = c.baro_on;
+    if (c.baro_on) {
+        W->ba_beta = c.ba_beta; W->ba_tau = c.ba_tau; W->ba_P0 = c.ba_P0;
+        W->myu = c.myu;
+    }
 }
 
 // Device -> caller order (for download): out[orig[s]] = value[s]; a null

@@ -110,6 +110,20 @@ struct __align__(16) FxRow {
 };
 static_assert(sizeof(FxRow) == 128, "FxRow is 128 bytes");
 
+// A replica's coupling settings (k_set_coupling).
+struct RepCoupling {
+    int thermo_on, thermo_kind, baro_on, pad;
+    double th_tau, th_T0, lambda, psi;
+    double ba_beta, ba_tau, ba_P0, myu;
+};
+
+// Arrays k_snapshot copies: destination, source, bytes.
+struct SnapArrays {
+    void* dst[11];
+    const void* src[11];
+    size_t bytes[11];
+};
+
 struct StepParams {
     double dt;
     double kick_c[MAX_TYPES];  // dt / (2 m_t), computed on the host as the reference does
@@ -175,7 +189,8 @@ struct Dev {
     int* slot_of_rank;
     int* bsum;         // [grid] scan block sums
     unsigned int* bar; // [8] grid barrier count, generation; any rebuild; list-build blocks done;
-                       //   a cell too crowded for the paired list build; direct builds so far
+                       //   a cell too crowded for the paired list build; direct builds so far;
+                       //   k_apply_pending blocks done
     int* rb;           // rebuild work list, built by the step kernel when it rebuilds:
                        //   [0] count m of rebuilding replicas, [1] how many of them come
                        //   first because the paired list build does not take them (brute
