@@ -130,7 +130,7 @@ def splat_params(camera: Camera, mode: int = MODE_TYPE, gradient=DEFAULT_GRADIEN
 def splat(particles: np.ndarray, params: _lib.CSplatParams, width: int, height: int) -> np.ndarray:
     """mdgb_splat: (height, width, 4) float32 RGBA."""
     parts = np.ascontiguousarray(particles, dtype=F32).reshape(-1, 12)
-    out = np.zeros((height, width, 4), dtype=F32)
+    out = np.empty((height, width, 4), dtype=F32)   # every pixel is written
     L = _lib.load()
     rc = L.mdgb_splat(parts, parts.shape[0], C.byref(params), int(width), int(height), out)
     if rc != _lib.MDGB_OK:
