@@ -1363,7 +1363,7 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
             (rc = dalloc(e, &d.nn, N)) || (rc = dalloc(e, &d.tiles, ntiles)) ||
             (rc = dalloc(e, &d.rep, nrep)) || (rc = dalloc(e, &d.part, 8 * (size_t)ntiles)) ||
             (rc = dalloc(e, &d.cpart, 8 * chunks.size())) || (rc = dalloc(e, &d.chunks, chunks.size())) ||
-            (rc = dalloc(e, &d.fx_part, ntiles)) || (rc = dalloc(e, &d.fx_cpart, chunks.size())) ||
+            (rc = dalloc(e, &d.fx_part, ntiles)) ||
             (rc = dalloc(e, &d.err, 2)) || (rc = dalloc(e, &d.max_needed, 1)) ||
             (rc = dalloc(e, &d.cell_count, ncells)) ||
             (rc = dalloc(e, &d.cell_start, ncells + 1)) || (rc = dalloc(e, &d.cell_rep, ncells)) ||

@@ -395,23 +395,27 @@ __device__ __forceinline__ double temperature_of(double thermal, long long n) {
 }
 
 // Coupling factors from the reduced T and P (thermostat.rs:31-39, barostat.rs:29-30).
+__device__ __forceinline__ void thermostat_factor(RepDev* W, const RepDev& R, double T, double dt) {
+    if (!R.thermo_on) return;
+    if (R.thermo_kind == 0) {
+        const double l2 = 1.0 + dt / R.th_tau * (R.th_T0 / T - 1.0);
+        W->lambda = sqrt(l2);
+    } else {
+        const double psi_dot = -((R.th_T0 / T) - 1.0) / R.th_tau;
+        const double psi = R.psi + psi_dot * (dt / 2.0);
+        W->psi = psi;
+        W->lambda = exp(-psi * dt / 2.0);
+    }
+}
+__device__ __forceinline__ void barostat_factor(RepDev* W, const RepDev& R, double P, double dt) {
+    if (!R.baro_on) return;
+    const double m3 = 1.0 + dt * R.ba_beta / R.ba_tau * (P - R.ba_P0);
+    W->myu = cbrt(m3);
+}
 __device__ __forceinline__ void coupling_factors(RepDev* W, const RepDev& R, double T, double P,
                                                  double dt) {
-    if (R.thermo_on) {
-        if (R.thermo_kind == 0) {
-            const double l2 = 1.0 + dt / R.th_tau * (R.th_T0 / T - 1.0);
-            W->lambda = sqrt(l2);
-        } else {
-            const double psi_dot = -((R.th_T0 / T) - 1.0) / R.th_tau;
-            const double psi = R.psi + psi_dot * (dt / 2.0);
-            W->psi = psi;
-            W->lambda = exp(-psi * dt / 2.0);
-        }
-    }
-    if (R.baro_on) {
-        const double m3 = 1.0 + dt * R.ba_beta / R.ba_tau * (P - R.ba_P0);
-        W->myu = cbrt(m3);
-    }
+    thermostat_factor(W, R, T, dt);
+    barostat_factor(W, R, P, dt);
 }
 
 // Finalize pass 2.  coupling: first apply the box part of the pending
@@ -483,14 +487,13 @@ __device__ void phase_finalize_single(const Dev& d, const StepParams& sp, int se
 // ---------------------------------------------------------------------------
 // Exact sums for the mixed path's coupled steps (replaces the FP64 tree of
 // passes partials1 / chunk sums there).  A double x = m 2^(e - 1075)
-// (m < 2^53) goes onto the binary grid of its tile, unit 2^(T - 1075 - FX_K)
-// with T the largest exponent of that quantity in the tile, as a 128-bit
-// integer; tiles, then chunks, then replicas are added exactly after
-// aligning to the larger grid (bits below 2^-96 of the largest value drop,
-// toward zero).  Integer work only -- GB300's FP64 pipe is narrow -- and the
-// sums do not depend on the order of the additions.  Headroom: a tile sum is
-// below 2^104, a chunk sum below 2^112, a replica of up to 2^27 atoms below
-// 2^124.
+// (m < 2^53) goes onto a binary grid, unit 2^(T - 1075 - FX_K) with T from the
+// largest exponent of that quantity met so far by the warp (fx_grid), as a
+// 128-bit integer; lanes, warps, then blocks are added exactly after aligning
+// to the larger grid (bits below 2^-96 of the largest value drop, toward zero).
+// Integer work only -- GB300's FP64 pipe is narrow -- and the sums do not
+// depend on the order of the additions.  Headroom: below 2^100 a value, so a
+// replica of up to 2^27 atoms stays below 2^127.
 // Below this many atoms the coupled reductions are latency-bound and the
 // FP64 tree (fewer dependent steps) is faster; from here on the exact sums
 // (no FP64 pipe work) are.
@@ -501,15 +504,24 @@ __device__ __forceinline__ int fx_exp(double x) {
     return e ? e : 1;   // subnormals and zero: exponent 1 without the hidden bit
 }
 
+// The grid for values up to exponent e: rounded up to the end of a group of
+// four, so that warps and blocks nearly always share one and their sums add
+// without shifts.  (Exponents near the top stay: 0x7FF marks non-finite values.)
+constexpr int FX_T0 = 3;
+__device__ __forceinline__ int fx_grid(int e) { return e < 0x7FC ? (e | 3) : e; }
+
 __device__ __forceinline__ __int128 fx_place(double x, int T) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
     const int e = (int)((b >> 52) & 0x7FFull);
     unsigned long long m = b & 0x000FFFFFFFFFFFFFull;
     if (e) m |= 1ull << 52;
     const int s = (e ? e : 1) - T + FX_K;
-    __int128 v = 0;
-    if (s >= 0) v = (__int128)m << s;          // s <= FX_K: below 2^97
-    else if (s > -64) v = (__int128)(m >> (-s));
+    if (s >= 0) {   // s <= FX_K: below 2^100 (two 64-bit shifts of the signed mantissa)
+        const long long v = (b >> 63) ? -(long long)m : (long long)m;
+        const long long hi = (v >> 1) >> (63 - s);
+        return (__int128)(((unsigned __int128)(unsigned long long)hi << 64) | ((unsigned long long)v << s));
+    }
+    const __int128 v = s > -64 ? (__int128)(m >> (-s)) : (__int128)0;
     return (b >> 63) ? -v : v;
 }
 
@@ -550,194 +562,267 @@ __device__ __forceinline__ double fx_to_double(__int128 v, int T) {
     return neg ? -r : r;
 }
 
-// Pass 1 of a coupled step on the mixed path: one exact row per tile, one
-// warp per tile (four atoms per lane, all their loads issued before any
-// arithmetic; no block-wide synchronisation), warps striding over the tiles.
-__device__ void phase_partials_fx(const Dev& d, int sel) {
-    const int lane = threadIdx.x & 31;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    const int N = d.ntot;
-    for (int t = gw; t < d.ntiles; t += nw) {
-        const int4 tl = d.tiles[t];
-        double vx[4], vy[4], vz[4], vir[4], pot[4];
-        bool in[4];
+// Pass 1 of a coupled step on the mixed path.  Every warp walks one run of
+// consecutive tiles and keeps its lanes' exact sums in registers: nothing is
+// exchanged between lanes until the run (or its replica) ends, where a vote
+// per pair of atoms is all that a tile needs of the other lanes -- whether a
+// quantity's grid has to be widened.  (Before, each tile's sums were reduced
+// over the warp and stored as a row -- 120 shuffles and 128 bytes a tile --
+// and rows were summed by chunk, then by replica, a grid barrier after each.)
+//
+// The row of a run stands at the index of its first tile in fx_part; a block
+// whose tiles are all of one replica leaves one row for its warps together.
+// fx_row_at() below finds a replica's rows again.
+//
+// Bound by integer issue (about 25 instructions a value): 8M atoms 92 us, 1M 22.
+// The whole coupling stage, both Berendsen couplings: 70,304 atoms 36 -> 21 us,
+// 1M 94 -> 56, 8M 214 -> 147, 512 replicas of 4.46M atoms 136 -> 97.
+struct FxRun {
+    __int128 s[FX_NQ];
+    int T[FX_NQ];      // grid of every quantity, the same in all lanes
+    unsigned cnt;
+    __device__ __forceinline__ void init() {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int a = lane + 32 * k;
-            in[k] = a < tl.z;
-            const int s = tl.y + (in[k] ? a : 0);
-            vx[k] = __ldcg(d.vel + s); vy[k] = __ldcg(d.vel + N + s); vz[k] = __ldcg(d.vel + 2 * N + s);
-            vir[k] = __ldcg(d.evir + s); pot[k] = __ldcg(d.epot + s);
-            if (!d.single_type && in[k])
-                in[k] = (int)__ldcg(reinterpret_cast<const long long*>(d.pos + s) + 3) == sel;
-        }
-        double v2[4];
-        int ex[FX_NQ];
+        for (int q = 0; q < FX_NQ; ++q) { s[q] = 0; T[q] = FX_T0; }
+        cnt = 0;
+    }
+};
+
+// Tiles per warp; a block's run is its warps' runs one after another.
+__device__ __forceinline__ int fx_tiles_per_warp(const Dev& d) {
+    const int warps = (int)gridDim.x * (TILE / 32);
+    return (d.ntiles + warps - 1) / warps;
+}
+
+// One value per lane and quantity onto the lanes' sums (whole warps only).
+__device__ __forceinline__ void fx_run_add(FxRun& a, const double (&x)[FX_NQ]) {
+    bool wider = false;
 #pragma unroll
-        for (int q = 0; q < FX_NQ; ++q) ex[q] = 1;
-        int nonfinite = 0;
-        unsigned cnt = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (!in[k]) { vx[k] = vy[k] = vz[k] = vir[k] = pot[k] = 0.0; }
-            v2[k] = __fma_rn(vz[k], vz[k], __fma_rn(vy[k], vy[k], __dmul_rn(vx[k], vx[k])));
-            cnt += __popc(__ballot_sync(0xffffffffu, in[k]));
-            const int e[FX_NQ] = {fx_exp(vx[k]), fx_exp(vy[k]), fx_exp(vz[k]), fx_exp(vir[k]), fx_exp(v2[k]),
-                                  fx_exp(pot[k])};
-#pragma unroll
-            for (int q = 0; q < FX_NQ; ++q) {
-                nonfinite |= e[q] == 0x7FF;
-                ex[q] = max(ex[q], e[q]);
-            }
-        }
-        nonfinite = __reduce_or_sync(0xffffffffu, nonfinite);
-        FxRow* row = d.fx_part + t;
+    for (int q = 0; q < FX_NQ; ++q) wider |= fx_exp(x[q]) > a.T[q];
+    if (__any_sync(0xffffffffu, wider)) {
 #pragma unroll
         for (int q = 0; q < FX_NQ; ++q) {
-            const int T = __reduce_max_sync(0xffffffffu, ex[q]);
-            __int128 v = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const double xk = q == 0 ? vx[k] : q == 1 ? vy[k] : q == 2 ? vz[k] : q == 3 ? vir[k]
-                                : q == 4 ? v2[k] : pot[k];
-                v += fx_place(xk, T);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += fx_shfl_xor(v, o);
-            if (lane == 0) { row->s[q] = v; row->ex[q] = (unsigned short)T; }
+            const int T = max(a.T[q], fx_grid(__reduce_max_sync(0xffffffffu, fx_exp(x[q]))));
+            a.s[q] = fx_align(a.s[q], a.T[q], T);
+            a.T[q] = T;
         }
-        if (lane == 0) { row->count = cnt; row->nonfinite = nonfinite; }
+    }
+#pragma unroll
+    for (int q = 0; q < FX_NQ; ++q) a.s[q] += fx_place(x[q], a.T[q]);
+}
+
+__device__ __forceinline__ void fx_run_tile(const Dev& d, const int4 tl, int sel, FxRun& a) {
+    const int lane = threadIdx.x & 31;
+    const int N = d.ntot;
+#pragma unroll 1
+    for (int k = 0; k < TILE; k += 64) {
+        if (k >= tl.z) break;
+        double x[2][FX_NQ];
+        bool in[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = lane + k + 32 * h;
+            in[h] = i < tl.z;
+            const int s = tl.y + (in[h] ? i : 0);
+            x[h][0] = __ldcg(d.vel + s); x[h][1] = __ldcg(d.vel + N + s); x[h][2] = __ldcg(d.vel + 2 * N + s);
+            x[h][3] = __ldcg(d.evir + s); x[h][5] = __ldcg(d.epot + s);
+            if (!d.single_type && in[h])
+                in[h] = (int)__ldcg(reinterpret_cast<const long long*>(d.pos + s) + 3) == sel;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (!in[h]) x[h][0] = x[h][1] = x[h][2] = x[h][3] = x[h][5] = 0.0;
+            x[h][4] = __fma_rn(x[h][2], x[h][2], __fma_rn(x[h][1], x[h][1], __dmul_rn(x[h][0], x[h][0])));
+            a.cnt += __popc(__ballot_sync(0xffffffffu, in[h]));
+            fx_run_add(a, x[h]);
+        }
     }
 }
 
-// Rows [0, n) added exactly by one warp: lane l takes rows l, l + 32, ...
-// (each row read whole, 128 bytes, eight 16-byte loads) onto its own running
-// grid, widened when a row needs it; then the lanes' sums onto the warp's
-// grid.  The result, valid in every lane, is on the grid of the largest
-// exponent.  Deterministic: the same rows always go to the same lanes in the
-// same order.
-__device__ __forceinline__ FxRow fx_warp_sum(const FxRow* rows, int n, int first = -1, int stride = 32) {
+// Lane q (below FX_NQ) of a row's readers and writers keeps quantity q, lane
+// FX_NQ the count.  An infinity or NaN leaves its exponent, 0x7FF, as the grid.
+struct FxTerm {
+    __int128 s;
+    int T;
+};
+__device__ __forceinline__ FxTerm fx_add(FxTerm a, FxTerm b) {
+    const int T = max(a.T, b.T);
+    return FxTerm{fx_align(a.s, a.T, T) + fx_align(b.s, b.T, T), T};
+}
+__device__ __forceinline__ void fx_set_term(FxRow* row, int q, FxTerm v) {
+    if (q < FX_NQ) { row->s[q] = v.s; row->ex[q] = (unsigned short)v.T; }
+    else if (q == FX_NQ) row->count = (long long)v.s;
+}
+
+// The warp's sums: the term of lane q in that lane.
+__device__ __forceinline__ FxTerm fx_run_term(const FxRun& a) {
     const int lane = threadIdx.x & 31;
-    if (first < 0) first = lane;
-    int T[FX_NQ];
-    __int128 s[FX_NQ];
-#pragma unroll
-    for (int q = 0; q < FX_NQ; ++q) { T[q] = 1; s[q] = 0; }
-    long long cnt = 0;
-    int nf = 0;
-    for (int t = first; t < n; t += stride) {
-        const longlong2* p = reinterpret_cast<const longlong2*>(rows + t);
-        longlong2 w[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) w[k] = __ldcg(p + k);
-        // w[0..5]: s[0..5] (low, high 64 bits); w[6]: ex[0..5] and nonfinite; w[7].x: count
-        const unsigned long long e03 = (unsigned long long)w[6].x;
-        const unsigned long long e45 = (unsigned long long)w[6].y;
-        int re[FX_NQ];
-        re[0] = (int)(e03 & 0xFFFF); re[1] = (int)((e03 >> 16) & 0xFFFF);
-        re[2] = (int)((e03 >> 32) & 0xFFFF); re[3] = (int)(e03 >> 48);
-        re[4] = (int)(e45 & 0xFFFF); re[5] = (int)((e45 >> 16) & 0xFFFF);
-        nf |= (int)(e45 >> 32);
-        cnt += w[7].x;
-#pragma unroll
-        for (int q = 0; q < FX_NQ; ++q) {
-            const longlong2 h = w[q];   // s[q] occupies 16 bytes: lo, hi
-            const __int128 v = (__int128)(((unsigned __int128)(unsigned long long)h.y << 64) |
-                                          (unsigned long long)h.x);
-            if (re[q] > T[q]) { s[q] = fx_align(s[q], T[q], re[q]); T[q] = re[q]; }
-            s[q] += fx_align(v, re[q], T[q]);
-        }
-    }
-    FxRow out;
+    FxTerm mine{(__int128)a.cnt, FX_T0};
 #pragma unroll
     for (int q = 0; q < FX_NQ; ++q) {
-        const int Tw = __reduce_max_sync(0xffffffffu, T[q]);
-        __int128 v = fx_align(s[q], T[q], Tw);
+        __int128 v = a.s[q];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += fx_shfl_xor(v, o);
-        out.s[q] = v;
-        out.ex[q] = (unsigned short)Tw;
+        if (lane == q) mine = FxTerm{v, a.T[q]};
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        nf |= __shfl_xor_sync(0xffffffffu, nf, o);
-    }
-    out.count = cnt;
-    out.nonfinite = nf;
-    return out;
+    return mine;
 }
 
-// The same with a whole block (threads take rows tid, tid + blockDim, ...),
-// then the warps' sums combined in a fixed order.  Result valid in thread 0.
-__device__ __forceinline__ FxRow fx_block_sum(const FxRow* rows, int n) {
-    __shared__ FxRow sm_w[TILE / 32];   // k_pre and k_macro blocks have TILE threads
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    FxRow r = fx_warp_sum(rows, n, (int)threadIdx.x, (int)blockDim.x);
-    __syncthreads();   // a previous call's rows are read
-    if (lane == 0) sm_w[w] = r;
+// The block's terms from its warps', in warp order; valid in lanes 0 .. FX_NQ
+// of the first warp.
+__device__ __forceinline__ FxTerm fx_block_term(FxTerm v) {
+    __shared__ __int128 sm_s[TILE / 32][FX_NQ + 1];
+    __shared__ int sm_T[TILE / 32][FX_NQ + 1];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncthreads();   // a previous call's terms are read
+    if (lane <= FX_NQ) { sm_s[w][lane] = v.s; sm_T[w][lane] = v.T; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 1; i < nw; ++i) {
-            const FxRow& o = sm_w[i];
+    if (threadIdx.x <= FX_NQ)
+        for (int i = 1; i < TILE / 32; ++i) v = fx_add(v, FxTerm{sm_s[i][lane], sm_T[i][lane]});
+    return v;
+}
+
+__device__ void phase_partials_fx(const Dev& d, int sel) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int perw = fx_tiles_per_warp(d), per = perw * (TILE / 32);
+    const int b0 = blockIdx.x * per, b1 = min(d.ntiles, b0 + per);
+    if (b0 >= b1) return;
+    const bool whole = d.tiles[b0].x == d.tiles[b1 - 1].x;
+    int first = b0 + w * perw, rep = -1;
+    const int end = min(b1, first + perw);
+    FxRun run;
+    run.init();
+    for (int t = first; t < end; ++t) {
+        const int4 tl = d.tiles[t];
+        if (tl.x != rep && t > first) {
+            fx_set_term(d.fx_part + first, lane, fx_run_term(run));
+            run.init();
+            first = t;
+        }
+        rep = tl.x;
+        fx_run_tile(d, tl, sel, run);
+    }
+    FxTerm r = fx_run_term(run);
+    if (whole) {
+        r = fx_block_term(r);
+        if (threadIdx.x <= FX_NQ) fx_set_term(d.fx_part + b0, lane, r);
+    } else if (first < end) {
+        fx_set_term(d.fx_part + first, lane, r);
+    }
+}
+
+// Where candidate i of a replica with tiles [a, e) has its row, or -1: the
+// blocks that hold tiles of it (nb of them) by their first warp, then the other
+// warps of the first and the last block, which it may share with neighbours.
+__device__ __forceinline__ int fx_row_at(const Dev& d, int a, int e, int perw, int i) {
+    const int per = perw * (TILE / 32);
+    const int f = a / per, l = (e - 1) / per, nb = l - f + 1;
+    int b = f + i, w = 0;
+    if (i >= nb) {
+        const int k = i - nb;
+        w = 1 + (k >> 1);
+        b = (k & 1) ? l : f;
+        if ((k & 1) && l == f) return -1;
+    }
+    const int s = b * per;
+    if (a <= s && min(s + per, d.ntiles) <= e) return w == 0 ? s : -1;
+    const int ws = max(a, s + w * perw);
+    return ws < min(e, s + (w + 1) * perw) ? ws : -1;
+}
+
+// The rows of the replica with tiles [a, e) added exactly by the block: eight
+// lanes a row, one quantity each, sixteen rows at a time, eight loads of each
+// lane in flight; then the lanes of a quantity in a fixed order.  (1M atoms, 652
+// rows, with the factors: 29 us; a thread a row, all quantities one after
+// another, took 45.)  Deterministic: the same rows always go to the same threads
+// in the same order.  Valid in lanes 0 .. FX_NQ of the first warp.
+__device__ __forceinline__ FxTerm fx_replica_sum(const Dev& d, int a, int e) {
+    constexpr int GROUPS = TILE / 8, BATCH = 8;
+    const int perw = fx_tiles_per_warp(d), per = perw * (TILE / 32);
+    const int n = (e - 1) / per - a / per + 1 + 2 * (TILE / 32 - 1);
+    const int q = threadIdx.x & 7;
+    FxTerm sum{0, FX_T0};
+    for (int i0 = threadIdx.x >> 3; i0 < n; i0 += GROUPS * BATCH) {
+        longlong2 h[BATCH];
+        unsigned short T[BATCH];
+        bool ok[BATCH];
 #pragma unroll
-            for (int q = 0; q < FX_NQ; ++q) {
-                const int T = max((int)r.ex[q], (int)o.ex[q]);
-                r.s[q] = fx_align(r.s[q], r.ex[q], T) + fx_align(o.s[q], o.ex[q], T);
-                r.ex[q] = (unsigned short)T;
-            }
-            r.count += o.count;
-            r.nonfinite |= o.nonfinite;
+        for (int k = 0; k < BATCH; ++k) {   // (nothing here depends on a load)
+            const int i = i0 + GROUPS * k;
+            const int at = i < n && q <= FX_NQ ? fx_row_at(d, a, e, perw, i) : -1;
+            ok[k] = at >= 0;
+            const FxRow* row = d.fx_part + (ok[k] ? at : 0);
+            h[k] = __ldcg(reinterpret_cast<const longlong2*>(row) + (q < FX_NQ ? q : FX_NQ + 1));
+            T[k] = __ldcg(row->ex + (q < FX_NQ ? q : 0));
+        }
+#pragma unroll
+        for (int k = 0; k < BATCH; ++k) {
+            const long long hi = ok[k] && q < FX_NQ ? h[k].y : 0, lo = ok[k] ? h[k].x : 0;
+            const __int128 v = (__int128)(((unsigned __int128)(unsigned long long)hi << 64) | (unsigned long long)lo);
+            sum = fx_add(sum, FxTerm{v, ok[k] && q < FX_NQ ? (int)T[k] : FX_T0});
         }
     }
-    return r;
-}
-
-// One block per chunk of tile rows.
-__device__ void phase_chunk_sums_fx(const Dev& d) {
-    for (int c = blockIdx.x; c < d.nchunks; c += gridDim.x) {
-        const int4 ch = d.chunks[c];
-        const FxRow r = fx_block_sum(d.fx_part + ch.y, ch.z);
-        if (threadIdx.x == 0) d.fx_cpart[c] = r;
-    }
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1)
+        sum = fx_add(sum, FxTerm{fx_shfl_xor(sum.s, o), __shfl_xor_sync(0xffffffffu, sum.T, o)});
+    return fx_block_term(sum);
 }
 
 // Mixed path, coupled steps: the replica's exact sums as doubles, then what
 // phase_finalize2 does (box, T, P, coupling).  sum_i |v_i - vcm|^2 = sum
 // |v_i|^2 - n |vcm|^2 (as sum v_i = n vcm): one pass over the atoms.
-__device__ void phase_finalize_fx(const Dev& d, const StepParams& sp, int sel) {
+// The FP64 operations are one dependent chain of about 64 cycles each, so what
+// can go beside it does: the quantities' conversions and divisions in lanes of
+// one warp, the box in another's, the barostat's factor in a third.
+__device__ void phase_finalize_fx(const Dev& d, const StepParams& sp, int sel, int block, int blocks) {
+    __shared__ double sm_x[FX_NQ + 1], sm_vcm[3], sm_box[3];
     const double m = d.mass[sel];
-    for (int r = blockIdx.x; r < d.nrep; r += gridDim.x) {   // one block per replica
+    const int tid = threadIdx.x;
+    for (int r = block; r < d.nrep; r += blocks) {   // one block per replica
         const RepDev R = load_rep(d.rep + r);
-        const FxRow F = fx_block_sum(d.fx_cpart + R.chunk_begin, R.nchunks);
-        if (threadIdx.x == 0) {
-            double S[7];
+        RepDev* W = d.rep + r;
+        // (every thread has read the record when this returns: it may be written)
+        const FxTerm F = fx_replica_sum(d, R.tile_begin, R.tile_begin + R.ntiles);
+        if (tid < 32) {
             const double nan = __longlong_as_double(0x7FF8000000000000ll);
-            S[0] = fx_to_double(F.s[0], F.ex[0]); S[1] = fx_to_double(F.s[1], F.ex[1]);
-            S[2] = fx_to_double(F.s[2], F.ex[2]); S[3] = (double)F.count;
-            S[4] = fx_to_double(F.s[3], F.ex[3]); S[5] = fx_to_double(F.s[4], F.ex[4]);
-            S[6] = fx_to_double(F.s[5], F.ex[5]);
-            if (F.nonfinite)
-                for (int k = 0; k < 7; ++k) if (k != 3) S[k] = nan;
-            RepDev* W = d.rep + r;
-            const double vc[3] = {S[0] / S[3], S[1] / S[3], S[2] / S[3]};
-            W->vcm[0] = vc[0]; W->vcm[1] = vc[1]; W->vcm[2] = vc[2];
-            W->mom[0] = S[0] * m; W->mom[1] = S[1] * m; W->mom[2] = S[2] * m;
-            W->msum = S[3] * m; W->virsum = S[4]; W->ke = 0.5 * (m * S[5]); W->pe = S[6] * 0.5;
-            W->count = F.count;
-            const double p1 = m * (S[5] - S[3] * (vc[0] * vc[0] + vc[1] * vc[1] + vc[2] * vc[2]));
-            const double th = 0.5 * p1;
-            double box[3] = {R.box[0], R.box[1], R.box[2]};
-            if (R.pending != 1.0) {
-                for (int k = 0; k < d.ntypes; ++k)
-                    for (int a = 0; a < 3; ++a) box[a] *= R.pending;
-                for (int a = 0; a < 3; ++a) { W->box[a] = box[a]; W->cs[a] = box[a] / (double)R.nc[a]; }
+            const bool nonfinite = __any_sync(0xffffffffu, tid < FX_NQ && F.T == 0x7FF);
+            const double x = tid >= FX_NQ ? (double)(long long)F.s : nonfinite ? nan : fx_to_double(F.s, F.T);
+            const double vc = x / __shfl_sync(0xffffffffu, x, FX_NQ);
+            if (tid <= FX_NQ) sm_x[tid] = x;
+            if (tid < 3) {
+                sm_vcm[tid] = vc;
+                W->vcm[tid] = vc;
+                W->mom[tid] = x * m;
             }
-            const double volume = box[0] * box[1] * box[2];
-            const double T = temperature_of(th, F.count);
-            const double P = (p1 + (-S[4]) * 0.5) / volume / 3.0;
-            W->thermal = th; W->T = T; W->P = P;
-            coupling_factors(W, R, T, P, sp.dt);
+            if (tid == FX_NQ) W->count = (long long)F.s;
+        } else if (tid >= 64 && tid < 67) {
+            const int a = tid - 64;
+            double L = a == 0 ? R.box[0] : a == 1 ? R.box[1] : R.box[2];
+            const int nc = a == 0 ? R.nc[0] : a == 1 ? R.nc[1] : R.nc[2];
+            if (R.pending != 1.0) {
+                for (int k = 0; k < d.ntypes; ++k) L *= R.pending;
+                W->box[a] = L;
+                W->cs[a] = L / (double)nc;
+            }
+            sm_box[a] = L;
+        }
+        __syncthreads();
+        if (tid == 0 || tid == 32) {
+            const double n = sm_x[FX_NQ], vv = sm_x[4], vir = sm_x[3];
+            const double p1 =
+                m * (vv - n * (sm_vcm[0] * sm_vcm[0] + sm_vcm[1] * sm_vcm[1] + sm_vcm[2] * sm_vcm[2]));
+            if (tid == 0) {
+                const double th = 0.5 * p1;
+                const double T = temperature_of(th, (long long)n);
+                W->msum = n * m; W->virsum = vir; W->ke = 0.5 * (m * vv); W->pe = sm_x[5] * 0.5;
+                W->thermal = th; W->T = T;
+                thermostat_factor(W, R, T, sp.dt);
+            } else {
+                const double volume = sm_box[0] * sm_box[1] * sm_box[2];
+                const double P = (p1 + (-vir) * 0.5) / volume / 3.0;
+                W->P = P;
+                barostat_factor(W, R, P, sp.dt);
+            }
         }
     }
 }
@@ -1798,50 +1883,19 @@ __device__ void phase_build_list(const Dev& d) {
         if ((int)threadIdx.x < tl.z) {
             const float4 xi = __ldcg(d.mir + s);
             const int ti = type_of(xi);
-            if (R.mode == MODE_CELLS) {
-                int cx, cy, cz;
-                decode_cell(d.cell[s] - R.cell_base, R.nc, cx, cy, cz);
-                const float cs[3] = {(float)R.cs[0], (float)R.cs[1], (float)R.cs[2]};
-                for (int dz = -1; dz <= 1; ++dz) {
-                    int z = cz + dz; z = z < 0 ? z + R.nc[2] : (z >= R.nc[2] ? z - R.nc[2] : z);
-                    for (int dy = -1; dy <= 1; ++dy) {
-                        int y = cy + dy; y = y < 0 ? y + R.nc[1] : (y >= R.nc[1] ? y - R.nc[1] : y);
-                        for (int dx = -1; dx <= 1; ++dx) {
-                            int x = cx + dx; x = x < 0 ? x + R.nc[0] : (x >= R.nc[0] ? x - R.nc[0] : x);
-                            const int cj = R.cell_base + (x * R.nc[1] + y) * R.nc[2] + z;
-                            const uint32_t code = (uint32_t)((dx + 1) + 3 * (dy + 1) + 9 * (dz + 1));
-                            const float sx = (float)dx * cs[0], sy = (float)dy * cs[1], sz = (float)dz * cs[2];
-                            int jb = __ldcg(d.cell_start + cj), je = jb + __ldcg(d.cell_count + cj);
-                            if (jb < R.begin || je > R.begin + R.n) { atomicOr(d.err, E_CELLS); continue; }
-                            for (int j = jb; j < je; ++j) {
-                                if (j == s) continue;
-                                const float4 xj = __ldcg(d.mir + j);
-                                if (type_of(xj) < ti) continue;
-                                const float ex = xj.x - xi.x + sx, ey = xj.y - xi.y + sy,
-                                            ez = xj.z - xi.z + sz;
-                                if (ex * ex + ey * ey + ez * ez < rl2) {
-                                    if (cnt < cap) d.nbr[list_index(s, cnt, tpa, R.begin, R.n, cap)] = (uint32_t)j | (code << IDX_BITS);
-                                    ++cnt;
-                                }
-                            }
-                        }
-                    }
+            const float L[3] = {(float)R.box[0], (float)R.box[1], (float)R.box[2]};
+            for (int j = (int)R.begin; j < (int)R.begin + R.n; ++j) {
+                if (j == s) continue;
+                const float4 xj = __ldcg(d.mir + j);
+                if (type_of(xj) < ti) continue;
+                float e[3] = {xj.x - xi.x, xj.y - xi.y, xj.z - xi.z};
+                for (int a = 0; a < 3; ++a) {
+                    if (e[a] < -0.5f * L[a]) e[a] += L[a];
+                    else if (e[a] > 0.5f * L[a]) e[a] -= L[a];
                 }
-            } else {
-                const float L[3] = {(float)R.box[0], (float)R.box[1], (float)R.box[2]};
-                for (int j = (int)R.begin; j < (int)R.begin + R.n; ++j) {
-                    if (j == s) continue;
-                    const float4 xj = __ldcg(d.mir + j);
-                    if (type_of(xj) < ti) continue;
-                    float e[3] = {xj.x - xi.x, xj.y - xi.y, xj.z - xi.z};
-                    for (int a = 0; a < 3; ++a) {
-                        if (e[a] < -0.5f * L[a]) e[a] += L[a];
-                        else if (e[a] > 0.5f * L[a]) e[a] -= L[a];
-                    }
-                    if (e[0] * e[0] + e[1] * e[1] + e[2] * e[2] < rl2) {
-                        if (cnt < cap) d.nbr[list_index(s, cnt, tpa, R.begin, R.n, cap)] = (uint32_t)j | ((uint32_t)CODE_ZERO << IDX_BITS);
-                        ++cnt;
-                    }
+                if (e[0] * e[0] + e[1] * e[1] + e[2] * e[2] < rl2) {
+                    if (cnt < cap) d.nbr[list_index(s, cnt, tpa, R.begin, R.n, cap)] = (uint32_t)j | ((uint32_t)CODE_ZERO << IDX_BITS);
+                    ++cnt;
                 }
             }
             const int n = min(cnt, cap);
@@ -1894,6 +1948,8 @@ __device__ __forceinline__ bool nose_hoover_kick(const Dev& d, const StepParams&
 
 // The coupling factors of a step, before its kick (integrator.rs:20-29), each
 // phase closed by a grid barrier.  Returns true when the launch must stop.
+// LARGE: the system may have FX_MIN_ATOMS atoms.
+template <bool LARGE>
 __device__ __forceinline__ bool coupling_phases(const Dev& d, const StepParams& sp) {
     const int sel = d.last_type;
     // Nose-Hoover with several types: calculate_lambda runs once per type,
@@ -1906,13 +1962,16 @@ __device__ __forceinline__ bool coupling_phases(const Dev& d, const StepParams& 
     if (d.refmode) {
         if (phase_serial(d, sp, sel, true)) return true;
         if (grid_barrier(d)) return true;
-    } else if (d.mixed && d.ntot >= FX_MIN_ATOMS) {
+    } else if (LARGE && d.mixed && d.ntot >= FX_MIN_ATOMS) {
         phase_partials_fx(d, sel);
-        if (grid_barrier(d)) return true;
-        phase_chunk_sums_fx(d);
-        if (grid_barrier(d)) return true;
-        phase_finalize_fx(d, sp, sel);
-        if (grid_barrier(d)) return true;
+        // (several replicas: a block each, finalized side by side)
+        if (d.nrep == 1) {
+            if (grid_barrier_then(d, [&] { phase_finalize_fx(d, sp, sel, 0, 1); })) return true;
+        } else {
+            if (grid_barrier(d)) return true;
+            phase_finalize_fx(d, sp, sel, blockIdx.x, gridDim.x);
+            if (grid_barrier(d)) return true;
+        }
     } else if (d.mixed) {
         phase_partials1(d, sel);
         if (sums_then<7>(d, [&](int b, int n) { phase_finalize_single(d, sp, sel, b, n); })) return true;
@@ -1925,9 +1984,11 @@ __device__ __forceinline__ bool coupling_phases(const Dev& d, const StepParams& 
     return false;
 }
 
-// 6 blocks of 128 threads per SM (80 registers): at the default 64 registers
-// the phases spilled (measured: the rebuild's sort phases ran ~1.8x slower).
-__global__ void __launch_bounds__(TILE, 6) k_pre(Dev d, StepParams sp) {
+// 5 blocks of 128 threads per SM (96 registers): at the default 64 registers
+// the phases spilled (the rebuild's sort phases ran ~1.8x slower), at 80 less so
+// (8M atoms, a coupled step: 2871 us, 2854 at 96, the same at 128; 512 replicas
+// 1760, 1744 and, with the sort phases short of warps, 1793 at 128).
+__global__ void __launch_bounds__(TILE, 5) k_pre(Dev d, StepParams sp) {
     if (chunk_failed(d)) return;
     barrier_setup(sp);
     tile_rep_reset();
@@ -1968,7 +2029,7 @@ __global__ void __launch_bounds__(TILE, 6) k_pre(Dev d, StepParams sp) {
         return;
     }
     if (sp.do_drift && sp.coupled) {
-        if (coupling_phases(d, sp)) return;
+        if (coupling_phases<true>(d, sp)) return;
         clk.mark(TR_COUPLING);
     }
     const bool moved = sp.do_drift || !sp.force_rebuild;
@@ -2523,7 +2584,7 @@ __device__ __noinline__ bool steps_rebuild(const Dev& d, uint32_t* st_smem) {
 
 // Coupling and motion of a step that the previous force pass did not drift.
 __device__ __noinline__ bool steps_motion(const Dev& d, const StepParams& sp) {
-    if (sp.coupled && coupling_phases(d, sp)) return true;
+    if (sp.coupled && coupling_phases<false>(d, sp)) return true;
     if (sp.thermo_nh && nose_hoover_kick(d, sp)) return true;
     if (d.mixed) phase_drift<true>(d, sp, sp.thermo_nh != 0); else phase_drift<false>(d, sp, sp.thermo_nh != 0);
     return false;

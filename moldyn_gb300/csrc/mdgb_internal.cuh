@@ -98,14 +98,14 @@ struct RepDev {
 
 // One row of the exact (128-bit fixed-point) sums of the mixed path's coupled
 // steps: per quantity (v_x, v_y, v_z, temp, v.v, potential) an integer sum on
-// the binary grid of its exponent ex (unit 2^(ex - 1075 - FX_K)), the atom
-// count and a flag for non-finite inputs.  128 bytes.
+// the binary grid of its exponent ex (unit 2^(ex - 1075 - FX_K); 0x7FF when an
+// input was not finite), and the atom count.  128 bytes.
 constexpr int FX_NQ = 6;
-constexpr int FX_K = 44;
+constexpr int FX_K = 47;
 struct __align__(16) FxRow {
     __int128 s[FX_NQ];
     unsigned short ex[FX_NQ];
-    int nonfinite;
+    int pad;
     long long count;
 };
 static_assert(sizeof(FxRow) == 128, "FxRow is 128 bytes");
@@ -217,8 +217,7 @@ struct Dev {
     unsigned char* pair_in;     // per record: 1 if within r_cut at the last force pass
     int2* pair_tile;            // [ntiles] first record, record count
     int* pair_count;            // [nrep] records handed out since the rebuild
-    FxRow* fx_part;             // [ntiles] exact tile sums (mixed path, coupled steps)
-    FxRow* fx_cpart;            // [nchunks] exact chunk sums
+    FxRow* fx_part;             // [ntiles] exact sums, at the first tile of each run (mixed path, coupled steps)
 };
 
 // k_pre phases recorded with MDGB_FLAG_TRACE (slot indices; TR_SORT stays 0,
