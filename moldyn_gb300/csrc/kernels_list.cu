@@ -10,9 +10,8 @@
 // pairs inside rlist, which the force kernels decide exactly.  Two builds
 // produce it:
 //
-// Paired (replicas of at least LIST_PAIRED_MIN_ATOMS atoms whose cells hold
-// at most 32 atoms, the usual case).  k_list_masks: one
-// warp per cell A tests A's atoms against the atoms of A and of its 13
+// Paired (replicas that list_paired takes, with cells of at most 32 atoms, the
+// usual case).  k_list_masks: one warp per cell A tests A's atoms against the atoms of A and of its 13
 // forward neighbour cells (codes 14..26), so each pair of neighbouring cells
 // is tested once, from one side.  A candidate stream of those cells is
 // walked 32 candidates at a time, one per lane, each tested against every
@@ -26,7 +25,7 @@
 // pass, so in the [k / tpa][atom][k % tpa] layout the stores of a pass are
 // contiguous.
 //
-// Direct (smaller replicas, where the second pass costs more than the
+// Direct (the other replicas, where the second pass costs more than the
 // halved tests save; every replica when a cell of more than 32 atoms is
 // anywhere in the rebuild, or with MDGB_FLAG_DIRECT_LIST).  One warp per
 // cell, 32 of the cell's atoms at a

@@ -1405,10 +1405,11 @@ __device__ void phase_work_list(const Dev& d) {
             int v[3] = {0, 0, 0};
             if (r < d.nrep) {
                 const RepDev* W = d.rep + r;
-                const bool paired = W->n >= LIST_PAIRED_MIN_ATOMS && __ldcg(&W->mode) == MODE_CELLS;
+                const int cells = __ldcg(&W->nc[0]) * __ldcg(&W->nc[1]) * __ldcg(&W->nc[2]);
+                const bool paired = list_paired(W->n, cells) && __ldcg(&W->mode) == MODE_CELLS;
                 if (__ldcg(&W->rebuild) && paired == (pass == 1)) {
                     v[0] = 1;
-                    v[1] = __ldcg(&W->nc[0]) * __ldcg(&W->nc[1]) * __ldcg(&W->nc[2]);
+                    v[1] = cells;
                     v[2] = W->ntiles;
                 }
             }

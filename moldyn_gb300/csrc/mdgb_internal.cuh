@@ -194,7 +194,7 @@ struct Dev {
     int* rb;           // rebuild work list, built by the step kernel when it rebuilds:
                        //   [0] count m of rebuilding replicas, [1] how many of them come
                        //   first because the paired list build does not take them (brute
-                       //   mode, or fewer than LIST_PAIRED_MIN_ATOMS atoms), then nrep ids,
+                       //   mode, or list_paired says no), then nrep ids,
                        //   m + 1 prefix offsets of their cells and m + 1 of their tiles
     uint32_t* lmask;   // [27][N] paired list build: hit word of (shift code, atom)
     uint32_t* nbs;     // [ncells][27] start of each neighbour cell, tagged with its shift code
@@ -245,7 +245,19 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // The rebuild work list (Dev::rb): replica ids and prefix offsets of their
 // cells and tiles.  Work item w (a cell or a tile of a rebuilding replica,
 // counted over the list) -> the list position i with off[i] <= w < off[i+1].
-constexpr int LIST_PAIRED_MIN_ATOMS = 32768;  // smaller replicas: the direct list build
+// Which replicas take the paired list build.  The list phase of a step by the
+// lower limit (512 replicas of 64 to 64,000 atoms, 74 of them rebuilt a step):
+// 4,096 568 us, 6,144 525, 8,192 521, 16,384 536, 32,768 561; one system of
+// 17,408 atoms 4.0 us paired, 5.8 direct.  A cell of more than 32 atoms sends the
+// whole rebuild to the direct build, after the tests were done: a grid of few
+// cells an axis rounds its cells up most, so a small replica has to have room
+// (22 atoms a cell 523 us, 24 521, no limit 521 here; dense replicas of 2,048
+// to 8,192 atoms, 14 and more a cell, let in: 669).
+constexpr int LIST_PAIRED_MIN_ATOMS = 8192, LIST_PAIRED_ANY_ATOMS = 32768, LIST_PAIRED_CELL_ATOMS = 24;
+__host__ __device__ __forceinline__ bool list_paired(int atoms, int cells) {
+    return atoms >= LIST_PAIRED_ANY_ATOMS ||
+           (atoms >= LIST_PAIRED_MIN_ATOMS && atoms <= LIST_PAIRED_CELL_ATOMS * cells);
+}
 __device__ __forceinline__ const int* rb_rep(const Dev& d) { return d.rb + 2; }
 __device__ __forceinline__ const int* rb_cell_off(const Dev& d) { return d.rb + 2 + d.nrep; }
 __device__ __forceinline__ const int* rb_tile_off(const Dev& d) { return d.rb + 3 + 2 * d.nrep; }

@@ -158,3 +158,28 @@ def test_reference_order_lists_of_every_length(Engine, oracle, rho, skin, direct
     e.close()
     assert np.array_equal(out["force"], st.force)
     assert np.array_equal(out["potential"], st.potential) and np.array_equal(out["temp"], st.temp)
+
+
+@pytest.mark.parametrize("sizes", [[(13, 13, 13, 0.8442), (12, 12, 12, 0.8442), (14, 13, 15, 0.05)],
+                                   [(16, 16, 17, 0.5), (9, 10, 9, 0.3), (13, 12, 13, 0.8442), (20, 19, 20, 0.02)]])
+def test_paired_build_of_mid_size_replicas(Engine, sizes):
+    """Replicas on both sides of the paired build's limit (6,912 to 30,400
+    atoms), dense and dilute, rebuilt together and apart: the direct build gives
+    the same trajectories."""
+    systems = [gs.fcc(s[:3], rho=s[3], jitter=0.05, seed=i + 51, t_star=1.0 + 0.3 * i) for i, s in enumerate(sizes)]
+    offs = np.cumsum([0] + [len(s[0]) for s in systems])
+    pos = np.concatenate([s[0] for s in systems])
+    vel = np.concatenate([s[1] for s in systems])
+    outs, stats = [], []
+    for direct in (False, True):
+        e = Engine(precision="mixed", persistent=True, graph_steps=10, threads_per_atom=1, direct_list=direct)
+        e.set_potential(0, 0, 1.0, 1.0)
+        e.upload_ensemble(offs, np.zeros(len(pos), dtype=np.uint16), pos, vel, [1.0], np.array([s[2] for s in systems]))
+        e.compute_forces()
+        e.ensemble_step(40, 0.005)
+        outs.append(e.download())
+        stats.append(e.stats())
+        e.close()
+    for k in FIELDS:
+        assert np.array_equal(outs[0][k], outs[1][k]), k
+    assert stats[0].direct_list_builds == 0 and stats[1].direct_list_builds > 0
