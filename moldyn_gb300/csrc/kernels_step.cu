@@ -355,9 +355,10 @@ __device__ void phase_finalize1(const Dev& d, int sel, int block, int blocks) {
         const RepDev R = load_rep(d.rep + r);
         double S[7];
         warp_sum_tiles<7>(d, R, S);
-        if ((threadIdx.x & 31) == 0) {
-            RepDev* W = d.rep + r;
-            W->vcm[0] = S[0] / S[3]; W->vcm[1] = S[1] / S[3]; W->vcm[2] = S[2] / S[3];
+        RepDev* W = d.rep + r;
+        const int lane = threadIdx.x & 31;
+        if (lane < 3) W->vcm[lane] = (lane == 0 ? S[0] : lane == 1 ? S[1] : S[2]) / S[3];
+        if (lane == 0) {
             W->mom[0] = S[0] * m; W->mom[1] = S[1] * m; W->mom[2] = S[2] * m;
             W->msum = S[3] * m; W->virsum = S[4]; W->ke = 0.5 * (m * S[5]); W->pe = S[6] * 0.5;
             W->count = (long long)S[3];
@@ -412,10 +413,57 @@ __device__ __forceinline__ void barostat_factor(RepDev* W, const RepDev& R, doub
     const double m3 = 1.0 + dt * R.ba_beta / R.ba_tau * (P - R.ba_P0);
     W->myu = cbrt(m3);
 }
-__device__ __forceinline__ void coupling_factors(RepDev* W, const RepDev& R, double T, double P,
-                                                 double dt) {
-    thermostat_factor(W, R, T, dt);
-    barostat_factor(W, R, P, dt);
+// A replica's last stage by one warp.  Its dozen FP64 divisions are chains of
+// dependent operations at about 64 cycles each: those that do not need one
+// another are lanes of the same instructions (argon, 1,000 atoms, a coupled step
+// in the reference's order: 85.8 -> 82.8 us).  All lanes call; every lane has
+// read its copy of the record before the first store.
+//
+// The centre-of-mass velocity sum_a / den (lanes 0-2) beside the box part of the
+// pending barostat update (lanes 3-5: box *= mu once per type, barostat.rs:45).
+__device__ __forceinline__ void finalize_frame(const Dev& d, RepDev* W, const RepDev& R, bool coupling, double s0,
+                                               double s1, double s2, double den, double (&vc)[3], double (&box)[3]) {
+    const int lane = threadIdx.x & 31, a = lane < 3 ? lane : lane - 3;
+    double L = a == 0 ? R.box[0] : a == 1 ? R.box[1] : R.box[2];
+    const int nc = a == 0 ? R.nc[0] : a == 1 ? R.nc[1] : R.nc[2];
+    const bool scale = coupling && R.pending != 1.0;
+    if (scale)
+        for (int k = 0; k < d.ntypes; ++k) L *= R.pending;
+    const double q = (lane < 3 ? (a == 0 ? s0 : a == 1 ? s1 : s2) : L) / (lane < 3 ? den : (double)nc);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        vc[k] = __shfl_sync(0xffffffffu, q, k);
+        box[k] = __shfl_sync(0xffffffffu, L, 3 + k);
+    }
+    if (lane < 3) W->vcm[a] = q;
+    else if (lane < 6 && scale) { W->box[a] = L; W->cs[a] = q; }
+}
+
+// Temperature and thermostat factor (lane 0) beside pressure and barostat factor
+// (lane 1).  th: thermal energy of n atoms; pv: three times P V.
+__device__ __forceinline__ void finalize_coupling(RepDev* W, const RepDev& R, const StepParams& sp, bool coupling,
+                                                  bool pressure, double th, long long n, double pv, double volume) {
+    const int lane = threadIdx.x & 31;
+    const bool t = lane == 0;
+    const double dt = sp.dt;
+    double q = (t ? 2.0 * th : pv) / (t ? 3.0 * (double)n * K_B : volume);
+    if (t) q *= 100.0;                                              // T (temperature_of)
+    const double x = (t ? R.th_T0 : q) / (t ? q : 3.0);             // T0 / T; P
+    if (t) { W->thermal = th; W->T = q; }
+    if (lane == 1 && pressure) W->P = x;
+    if (!coupling) return;
+    const bool nh = R.thermo_kind != 0;
+    const double y = (t ? (nh ? -(x - 1.0) : dt) : dt * R.ba_beta) / (t ? R.th_tau : R.ba_tau);
+    if (t && R.thermo_on) {
+        if (nh) {
+            const double psi = R.psi + y * (dt / 2.0);
+            W->psi = psi;
+            W->lambda = exp(-psi * dt / 2.0);
+        } else {
+            W->lambda = sqrt(1.0 + y * (x - 1.0));
+        }
+    }
+    if (lane == 1 && R.baro_on) W->myu = cbrt(1.0 + y * (x - R.ba_P0));
 }
 
 // Finalize pass 2.  coupling: first apply the box part of the pending
@@ -431,20 +479,11 @@ __device__ void phase_finalize2(const Dev& d, const StepParams& sp, bool couplin
         const double sdv = S1[0];
         const double p1 = d.mass[sel] * sdv;              // sum m |v - vcm|^2 (pressure.rs:13-17)
         const double th = 0.5 * p1;                        // energy.rs:25-37
-        if ((threadIdx.x & 31) == 0) {
-            RepDev* W = d.rep + r;
-            double box[3] = {R.box[0], R.box[1], R.box[2]};
-            if (coupling && R.pending != 1.0) {
-                for (int k = 0; k < d.ntypes; ++k)
-                    for (int a = 0; a < 3; ++a) box[a] *= R.pending;
-                for (int a = 0; a < 3; ++a) { W->box[a] = box[a]; W->cs[a] = box[a] / (double)R.nc[a]; }
-            }
-            const double volume = box[0] * box[1] * box[2];
-            const double T = temperature_of(th, R.count);
-            const double P = (p1 + (-R.virsum) * 0.5) / volume / 3.0;
-            W->thermal = th; W->T = T; W->P = P;
-            if (coupling) coupling_factors(W, R, T, P, sp.dt);
-        }
+        RepDev* W = d.rep + r;
+        double vc[3], box[3];
+        // (pass 1 has left the centre-of-mass velocity: divided by one, it stays)
+        finalize_frame(d, W, R, coupling, R.vcm[0], R.vcm[1], R.vcm[2], 1.0, vc, box);
+        finalize_coupling(W, R, sp, coupling, true, th, R.count, p1 + (-R.virsum) * 0.5, box[0] * box[1] * box[2]);
     }
 }
 
@@ -460,27 +499,17 @@ __device__ void phase_finalize_single(const Dev& d, const StepParams& sp, int se
         const RepDev R = load_rep(d.rep + r);
         double S[7];
         warp_sum_tiles<7>(d, R, S);
+        RepDev* W = d.rep + r;
+        double vc[3], box[3];
+        finalize_frame(d, W, R, true, S[0], S[1], S[2], S[3], vc, box);
         if ((threadIdx.x & 31) == 0) {
-            RepDev* W = d.rep + r;
-            const double vc[3] = {S[0] / S[3], S[1] / S[3], S[2] / S[3]};
-            W->vcm[0] = vc[0]; W->vcm[1] = vc[1]; W->vcm[2] = vc[2];
             W->mom[0] = S[0] * m; W->mom[1] = S[1] * m; W->mom[2] = S[2] * m;
             W->msum = S[3] * m; W->virsum = S[4]; W->ke = 0.5 * (m * S[5]); W->pe = S[6] * 0.5;
             W->count = (long long)S[3];
-            const double p1 = m * (S[5] - S[3] * (vc[0] * vc[0] + vc[1] * vc[1] + vc[2] * vc[2]));
-            const double th = 0.5 * p1;
-            double box[3] = {R.box[0], R.box[1], R.box[2]};
-            if (R.pending != 1.0) {
-                for (int k = 0; k < d.ntypes; ++k)
-                    for (int a = 0; a < 3; ++a) box[a] *= R.pending;
-                for (int a = 0; a < 3; ++a) { W->box[a] = box[a]; W->cs[a] = box[a] / (double)R.nc[a]; }
-            }
-            const double volume = box[0] * box[1] * box[2];
-            const double T = temperature_of(th, (long long)S[3]);
-            const double P = (p1 + (-S[4]) * 0.5) / volume / 3.0;
-            W->thermal = th; W->T = T; W->P = P;
-            coupling_factors(W, R, T, P, sp.dt);
         }
+        const double p1 = m * (S[5] - S[3] * (vc[0] * vc[0] + vc[1] * vc[1] + vc[2] * vc[2]));
+        finalize_coupling(W, R, sp, true, true, 0.5 * p1, (long long)S[3], p1 + (-S[4]) * 0.5,
+                          box[0] * box[1] * box[2]);
     }
 }
 
@@ -1104,12 +1133,6 @@ __device__ void phase_serial_terms1(const Dev& d, int sel, bool coupling) {
 }
 
 // Centre-of-mass velocity of replica r from the pass-1 folds.
-__device__ __forceinline__ void serial_vcm(const Dev& d, const RepDev& R, double vc[3]) {
-    const double* S = d.part + (size_t)R.tile_begin * 8;
-    const double sw = __ldcg(S + 3);
-    for (int a = 0; a < 3; ++a) vc[a] = __ldcg(S + a) / sw;
-}
-
 // Pass 2: row 0 thermal energy, rows 1-3 (as one) the pressure's three terms
 // of every atom, row 4 the negated virial.
 __device__ void phase_serial_terms2(const Dev& d, int sel) {
@@ -1122,7 +1145,8 @@ __device__ void phase_serial_terms2(const Dev& d, int sel) {
         const RepDev& R = tile_rep(d, tl.x);
         if (tl.x != vc_rep) {
             __syncthreads();
-            if (threadIdx.x == 0) serial_vcm(d, R, vc);
+            const double* S = d.part + (size_t)R.tile_begin * 8;
+            if (threadIdx.x < 3) vc[threadIdx.x] = __ldcg(S + threadIdx.x) / __ldcg(S + 3);
             __syncthreads();
             vc_rep = tl.x;
         }
@@ -1170,39 +1194,31 @@ __device__ void phase_serial_folds(const Dev& d, int sel, int pass, bool couplin
 // What the folds give, per replica: the macro parameters (k_macro), or T, P
 // and the coupling factors, or (nh_after_kick) the second psi update.
 __device__ void phase_serial_finalize(const Dev& d, const StepParams& sp, int sel, bool coupling, bool nh_after_kick) {
-    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nt = gridDim.x * blockDim.x;
-    for (int r = gt; r < d.nrep; r += nt) {
+    const int lane = threadIdx.x & 31;
+    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    for (int r = gw; r < d.nrep; r += nw) {   // one warp per replica
         const RepDev R = load_rep(d.rep + r);
         RepDev* W = d.rep + r;
         const double* A = d.part + (size_t)R.tile_begin * 8;
         const double* B = d.cpart + (size_t)R.chunk_begin * 8;
         const long long n = __ldcg(&W->type_off[sel + 1]) - __ldcg(&W->type_off[sel]);
         const double th = __ldcg(B);
-        const double T = temperature_of(th, n);
         if (nh_after_kick) {
-            nh_update_psi(W, R, T, sp.dt);
+            if (lane == 0) nh_update_psi(W, R, temperature_of(th, n), sp.dt);
             continue;
         }
-        double box[3] = {R.box[0], R.box[1], R.box[2]};
-        if (coupling && R.pending != 1.0) {
-            for (int k = 0; k < d.ntypes; ++k)
-                for (int a = 0; a < 3; ++a) box[a] *= R.pending;
-            for (int a = 0; a < 3; ++a) { W->box[a] = box[a]; W->cs[a] = box[a] / (double)R.nc[a]; }
+        const bool pressure = !coupling || R.baro_on;
+        const double kin = pressure ? __ldcg(B + 1) : 0.0, vir = pressure ? __ldcg(B + 2) : 0.0;
+        const double m0 = __ldcg(A), m1 = __ldcg(A + 1), m2 = __ldcg(A + 2), msum = __ldcg(A + 3);
+        double vc[3], box[3];
+        finalize_frame(d, W, R, coupling, m0, m1, m2, msum, vc, box);
+        if (lane == 0) {
+            W->mom[0] = m0; W->mom[1] = m1; W->mom[2] = m2;
+            W->msum = msum; W->count = n;
+            if (pressure) W->virsum = -vir;
+            if (!coupling) { W->ke = __ldcg(A + 4); W->pe = __ldcg(A + 5) / 2.0; }
         }
-        double P = 0.0;
-        if (!coupling || R.baro_on) {
-            const double volume = box[0] * box[1] * box[2];
-            P = (__ldcg(B + 1) + __ldcg(B + 2) * 0.5) / volume / 3.0;
-            W->virsum = -__ldcg(B + 2);
-            W->P = P;
-        }
-        serial_vcm(d, R, W->vcm);
-        for (int a = 0; a < 3; ++a) W->mom[a] = __ldcg(A + a);
-        W->msum = __ldcg(A + 3);
-        if (!coupling) { W->ke = __ldcg(A + 4); W->pe = __ldcg(A + 5) / 2.0; }
-        W->thermal = th; W->count = n; W->T = T;
-        if (coupling) coupling_factors(W, R, T, P, sp.dt);
+        finalize_coupling(W, R, sp, coupling, pressure, th, n, kin + vir * 0.5, box[0] * box[1] * box[2]);
     }
 }
 
