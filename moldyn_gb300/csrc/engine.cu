@@ -1,15 +1,18 @@
 // engine.cu -- host side of libmdgb: the C ABI declared in include/mdgb.h.
 //
 // Drives the kernels of kernels_step.cu / kernels_list.cu / kernels_force.cu
-// on one CUDA stream per handle.  One integrator step (integrator.rs:14-59)
-// is three or four launches:
+// on one CUDA stream per handle.  A small system's whole chunk of steps is one
+// launch (k_steps).  Otherwise one integrator step (integrator.rs:14-59) is:
 //   k_pre        (cooperative)  coupling reductions -> kick/drift/wrap -> rebuild
 //                               check -> [cell sort, only if needed]
-//   k_build_list                Verlet list of the rebuilt replicas (else returns)
-//   k_force_*                   LJ forces + second half kick (+ on NVE chunks the
+//   k_list_masks, k_build_list  Verlet list of the rebuilt replicas (else return)
+//   k_force_mixed               LJ forces + second half kick (+ on NVE chunks the
 //                               next step's kick and drift, double-buffered)
-//   k_force_band (mixed path)   the atoms with a pair in the FP32-undecidable
-//                               band around r_cut, with FP64 decisions
+//   k_force_band                mixed path: the atoms with a pair in the
+//                               FP32-undecidable band around r_cut, with FP64
+//                               decisions
+//   k_pair_terms, k_pair_sums   FP64 path with pair records (each pair's terms
+//                               once, then each atom's sums); k_force_fp64 else
 // Steps run in chunks; before each chunk the engine snapshots the mutable
 // device state, and if the chunk reports a neighbour-list overflow it grows
 // the list, restores the snapshot and re-runs the chunk -- so capacity

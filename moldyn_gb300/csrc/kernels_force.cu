@@ -6,12 +6,13 @@
 // |r_ij| <= r_cut, r_ij = x_j - x_i taken to the image picked by the
 // reference's single-shift rule (potential.rs:186-200).
 //
-// k_force_fp64  -- the plain path.  Every pair is evaluated with the
-//   reference's FP64 operation sequence through explicit round-to-nearest
-//   intrinsics (no contraction), so each pair term carries the reference's
-//   bits; with MDGB_FLAG_REFERENCE_ORDER the list is in the reference's j
-//   order and the per-atom sums are bit-identical too.  An FP32 prefilter on
-//   the mirror skips candidates that are certainly outside r_cut.
+// k_force_fp64  -- the plain path of systems without pair records
+//   (kernels_pairs.cu).  Every pair is evaluated with the reference's FP64
+//   operation sequence through explicit round-to-nearest intrinsics (no
+//   contraction), so each pair term carries the reference's bits; with
+//   MDGB_FLAG_REFERENCE_ORDER the list is in the reference's j order and the
+//   per-atom sums are bit-identical too.  An FP32 prefilter on the mirror
+//   skips candidates that are certainly outside r_cut.
 // k_force_mixed -- the chosen path.  FP32 pair maths from the float4 mirror
 //   (cell-relative coordinates, periodic cell shift from the list entry),
 //   force sums in deterministic 64-bit fixed point, potential/virial in FP32

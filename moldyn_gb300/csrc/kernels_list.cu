@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(LB_WARPS * 32, 11) k_build_list(Dev d) {
     __shared__ int s_last;
     // the paired build's masks are complete unless a cell was too crowded for them
     const bool direct = d.direct_list || *(volatile const unsigned int*)(d.bar + 4) != 0u;
-    list_direct<SINGLE, LB_WARPS, false>(d, lb_smem, direct);
+    list_direct<SINGLE, LB_WARPS>(d, lb_smem, direct);
     if (!direct) list_expand(d, lb_smem);
     if (d.pairs) return;   // k_pair_link closes the rebuild
     // The last block to finish closes the rebuild of every replica.

@@ -1,6 +1,7 @@
 // list_direct.cuh -- the direct Verlet-list build (every cell against its 27
-// neighbour cells), shared by k_build_list (kernels_list.cu) and the
-// whole-chunk kernel of small systems (kernels_step.cu).
+// neighbour cells; k_build_list, kernels_list.cu) and the reference-order sort
+// of a list, which the whole-chunk kernel of small systems (kernels_step.cu)
+// uses too.
 #pragma once
 #include <type_traits>
 
@@ -142,8 +143,8 @@ static __device__ __noinline__ void sort_lists_by_rank(const Dev& d, int s0, int
 
 // The direct build: every cell against the stream of its 27 neighbour cells.
 // all: every rebuilding replica (else those the paired build does not take).
-// WARPS: warps per block; COH: data of this launch (no non-coherent loads).
-template <bool SINGLE, int WARPS, bool COH>
+// WARPS: warps per block.
+template <bool SINGLE, int WARPS>
 __device__ __forceinline__ void list_direct(const Dev& d, uint32_t* lb_smem, bool all) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -247,7 +248,7 @@ __device__ __forceinline__ void list_direct(const Dev& d, uint32_t* lb_smem, boo
                 float4 x_n = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (lane < wn) {
                     e_n = cand[lane];
-                    x_n = COH ? d.mir[e_n & IDX_MASK] : __ldg(d.mir + (e_n & IDX_MASK));
+                    x_n = __ldg(d.mir + (e_n & IDX_MASK));
                 }
                 for (int q = 0; q < nq; ++q) {
                     const bool valid = (q << 5) + lane < wn;
@@ -257,7 +258,7 @@ __device__ __forceinline__ void list_direct(const Dev& d, uint32_t* lb_smem, boo
                     const int tj = type_of(x_n);
                     if (((q + 1) << 5) + lane < wn) {   // next chunk in flight
                         e_n = cand[((q + 1) << 5) + lane];
-                        x_n = COH ? d.mir[e_n & IDX_MASK] : __ldg(d.mir + (e_n & IDX_MASK));
+                        x_n = __ldg(d.mir + (e_n & IDX_MASK));
                     }
                     // bit i of `mine`: own atom i lists this lane's candidate
                     uint32_t mine, unused;
