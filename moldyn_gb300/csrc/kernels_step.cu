@@ -1364,7 +1364,7 @@ __device__ void phase_drift(const Dev& d, const StepParams& sp, bool kicked) {
                 }
                 d.vel[s] = vx; d.vel[N + s] = vy; d.vel[2 * N + s] = vz;
                 double x = p.x, y = p.y, z = p.z;
-                if (R.pending != 1.0) {                                  // barostat.rs:46-48
+                if (__double_as_longlong(R.pending) != 0x3FF0000000000000ll) {   // != 1.0; barostat.rs:46-48
                     x = dmul_nospec(x, R.pending); y = dmul_nospec(y, R.pending);
                     z = dmul_nospec(z, R.pending);
                 }
