@@ -103,6 +103,11 @@ extern "C" {
  * are the same.  The engine does this by itself for a rebuild in which a cell
  * holds more than 32 atoms. */
 #define MDGB_FLAG_DIRECT_LIST 16u
+/* FP64 only: keep no pair records (about 4 KB of device memory an atom in a
+ * liquid, taken from 4,096 atoms on with one thread per atom while half of
+ * the device's memory stays free; each pair is then computed once).  Without
+ * them a force pass takes longer and both atoms compute the pair. */
+#define MDGB_FLAG_NO_PAIR_RECORDS 32u
 
 typedef struct mdgb_engine mdgb_engine;
 

@@ -31,6 +31,7 @@ FLAG_PROFILE = 2
 FLAG_PERSISTENT = 4
 FLAG_TRACE = 8
 FLAG_DIRECT_LIST = 16
+FLAG_NO_PAIR_RECORDS = 32
 TRACE_PHASES = ["coupling", "drift", "decide", "zero_cells", "bin", "scan_a", "scan_b", "scan_c", "scatter",
                 "sort_cells", "gather", "verlet_list", "launches", "rebuild_launches"]
 THERMOSTAT_BERENDSEN = 0

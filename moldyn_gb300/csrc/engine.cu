@@ -223,14 +223,19 @@ void drop_graphs(mdgb_engine* e) {
     e->graphs.clear();
 }
 
+void free_pairs(mdgb_engine* e) {
+    if (e->pair_alloc) cudaFree(e->pair_alloc);
+    e->pair_alloc = nullptr;
+    e->dev.pairs = 0;
+}
+
 // Device allocations of a state (kept by an upload of the same shape).
 void free_state(mdgb_engine* e) {
     drop_graphs(e);
     for (void* p : e->allocs) cudaFree(p);
     e->allocs.clear();
     if (e->nbr_alloc) { cudaFree(e->nbr_alloc); e->nbr_alloc = nullptr; }
-    if (e->pair_alloc) { cudaFree(e->pair_alloc); e->pair_alloc = nullptr; }
-    e->dev.pairs = 0;
+    free_pairs(e);
     e->dev.nn = nullptr;
     e->has_state = false;
     e->forces_valid = false;
@@ -321,16 +326,18 @@ int upload_pairs(mdgb_engine* e) {
 // PAIR_MIN_ATOMS atoms on the pairs are computed once (kernels_pairs.cu);
 // below, where a step is a few launches of latency, and with several threads
 // per atom, k_force_fp64 evaluates both sides.  About 4 KB an atom in a
-// liquid: where the device has no room for that (a tenth of its memory is
-// left to others), the records are left out as well.
+// liquid, which only saves time: half of the device's memory is left to what
+// has to be there (other engines' states and lists), and a caller who wants
+// all of it sets MDGB_FLAG_NO_PAIR_RECORDS.
 constexpr int PAIR_MIN_ATOMS = 4096;
 
 void alloc_pairs(mdgb_engine* e) {
     Dev& d = e->dev;
-    d.pairs = 0;
+    free_pairs(e);
     e->pair_single = d.single_type;
-    if (e->pair_alloc) { cudaFree(e->pair_alloc); e->pair_alloc = nullptr; }
-    if (e->cfg.precision != MDGB_PRECISION_FP64 || e->ntot < PAIR_MIN_ATOMS || e->cfg.threads_per_atom > 1) return;
+    if (e->cfg.precision != MDGB_PRECISION_FP64 || e->ntot < PAIR_MIN_ATOMS || e->cfg.threads_per_atom > 1 ||
+        (e->cfg.flags & MDGB_FLAG_NO_PAIR_RECORDS))
+        return;
     const size_t N = e->ntot, room = pair_room(N, d.cap, d.single_type);
     if (room >= (size_t)PAIR_NEG) return;
     // sizes in whole 256 bytes, so that every array starts aligned
@@ -340,7 +347,7 @@ void alloc_pairs(mdgb_engine* e) {
                  s_tile = up(e->ntiles * sizeof(int2)), s_cnt = up(e->nrep * sizeof(int));
     const size_t total = s_rec + s_ij + s_vir + s_of + s_in + s_tile + s_cnt;
     size_t free_b = 0, all_b = 0;
-    if (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess || total + all_b / 10 > free_b ||
+    if (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess || total + all_b / 2 > free_b ||
         cudaMalloc(&e->pair_alloc, total) != cudaSuccess) {
         cudaGetLastError();
         e->pair_alloc = nullptr;
@@ -363,6 +370,7 @@ int alloc_nbr(mdgb_engine* e, int cap) {
     // the tpa-interleaved layout (nbr_index) needs cap to be a multiple of every tpa
     cap = std::max(8, (cap + 7) & ~7);
     if (e->nbr_alloc) { cudaFree(e->nbr_alloc); e->nbr_alloc = nullptr; }
+    free_pairs(e);   // they index the old list, and the new one may need their memory
     const size_t words = (size_t)cap * (size_t)e->ntot;
     void* q = nullptr;
     CU(cudaMalloc(&q, std::max<size_t>(words, 1) * sizeof(uint32_t)));

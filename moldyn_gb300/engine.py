@@ -64,12 +64,16 @@ class Engine:
     direct_list: build every neighbour list directly (each cell against all
     27 neighbour cells) rather than testing each pair of cells once; the same
     lists, for comparison.
+    pair_records: FP64 from 4,096 atoms -- keep a record per pair (about 4 KB of
+    device memory an atom, while half of the device stays free), so that each
+    pair is computed once; False leaves that memory alone.
     """
 
     def __init__(self, precision: str = "mixed", skin: float = 0.0, rebuild_every: int = 0,
                  threads_per_atom: int = 0, graph_steps: int = 0, neighbor_capacity: int = 0,
                  device: int = 0, reference_order: bool = False, profile: bool = False,
-                 persistent: bool = False, trace: bool = False, direct_list: bool = False):
+                 persistent: bool = False, trace: bool = False, direct_list: bool = False,
+                 pair_records: bool = True):
         L = load()
         cfg = _lib.Config()
         check(L.mdgb_config_default(C.byref(cfg)))
@@ -85,7 +89,8 @@ class Engine:
                      | (_lib.FLAG_PROFILE if profile else 0)
                      | (_lib.FLAG_PERSISTENT if persistent else 0)
                      | (_lib.FLAG_TRACE if trace else 0)
-                     | (_lib.FLAG_DIRECT_LIST if direct_list else 0))
+                     | (_lib.FLAG_DIRECT_LIST if direct_list else 0)
+                     | (0 if pair_records else _lib.FLAG_NO_PAIR_RECORDS))
         h = C.c_void_p()
         st = L.mdgb_create(C.byref(cfg), C.byref(h))
         if st != _lib.MDGB_OK:

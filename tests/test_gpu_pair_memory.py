@@ -1,0 +1,91 @@
+"""The FP64 path's pair records and the device's memory: they only save time, so
+they leave at least half of the device to others and can be left out.  Which
+pass runs shows in the kernels launched: a rebuild and a force pass are seven
+with records (step kernel, two of the list, two of the records, terms, sums)
+and four without.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from tests import gpu_systems as gs
+
+pytestmark = pytest.mark.gpu
+
+WITH, WITHOUT = 7, 4
+
+
+def hold_memory(share):
+    """Device memory held until less than `share` of the device is free."""
+    torch = pytest.importorskip("torch")
+    free, total = torch.cuda.mem_get_info()
+    return torch.empty(max(1, free - int(share * total)), dtype=torch.uint8, device="cuda")
+
+
+def give_back():
+    import torch
+    torch.cuda.empty_cache()
+
+
+def launches(e):
+    n = e.stats().kernel_launches
+    e.set_potential(0, 0, 1.0, 1.0)   # the next pass builds the lists
+    e.compute_forces()
+    return e.stats().kernel_launches - n
+
+
+def liquid(cells=(11, 11, 11), seed=3):
+    pos, vel, box = gs.fcc(cells, jitter=0.04, seed=seed)
+    return np.zeros(len(pos), dtype=np.uint16), pos, vel, [1.0], box
+
+
+def engine(**kw):
+    from moldyn_gb300.engine import Engine
+    e = Engine(precision="fp64", threads_per_atom=1, **kw)
+    e.set_potential(0, 0, 1.0, 1.0)
+    return e
+
+
+def test_records_leave_half_of_the_device():
+    e = engine()
+    e.upload(*liquid())
+    assert launches(e) == WITH
+    e.close()
+    held = hold_memory(0.45)
+    try:
+        e = engine()
+        e.upload(*liquid())
+        assert launches(e) == WITHOUT
+        e.close()
+    finally:
+        del held
+        give_back()
+
+
+def test_records_can_be_left_out(oracle):
+    state = liquid()
+    e = engine(pair_records=False, reference_order=True)
+    e.upload(*state)
+    assert launches(e) == WITHOUT
+    st = oracle.OracleState([len(state[0])], state[1], state[2], [1.0], state[4], oracle.pot_table(1, default=(1.0, 1.0)))
+    st.update_force()
+    assert np.array_equal(e.download()["force"], st.force)
+    e.close()
+
+
+def test_a_longer_list_is_given_the_records_memory():
+    """A list that grows frees the records first; they come back for the new one."""
+    types, pos, vel, mass, box = liquid()
+    e = engine(neighbor_capacity=48)
+    e.upload(types, pos, vel, mass, box)     # 77 entries an atom: grows at once
+    assert e.stats().neighbor_capacity > 77
+    assert launches(e) == WITH
+    want = engine()
+    want.upload(types, pos, vel, mass, box)
+    want.compute_forces()
+    a, b = e.download(), want.download()
+    for k in ("force", "potential", "temp"):
+        assert np.array_equal(a[k], b[k]), k
+    e.close()
+    want.close()
