@@ -325,7 +325,10 @@ int upload_pairs(mdgb_engine* e) {
 // The FP64 path's pair records for the current list capacity.  From
 // PAIR_MIN_ATOMS atoms on the pairs are computed once (kernels_pairs.cu);
 // below, where a step is a few launches of latency, and with several threads
-// per atom, k_force_fp64 evaluates both sides.  About 4 KB an atom in a
+// per atom, k_force_fp64 evaluates both sides.  The pair kernels walk the lists
+// in the layout of one thread per atom, so there are records only while every
+// size class has that layout: a state whose records found no room when it was
+// uploaded may since have been tuned to another one.  About 4 KB an atom in a
 // liquid, which only saves time: half of the device's memory is left to what
 // has to be there (other engines' states and lists), and a caller who wants
 // all of it sets MDGB_FLAG_NO_PAIR_RECORDS.
@@ -338,6 +341,8 @@ void alloc_pairs(mdgb_engine* e) {
     if (e->cfg.precision != MDGB_PRECISION_FP64 || e->ntot < PAIR_MIN_ATOMS || e->cfg.threads_per_atom > 1 ||
         (e->cfg.flags & MDGB_FLAG_NO_PAIR_RECORDS))
         return;
+    for (int c = 0; c < mdgb_engine::NCLASS; ++c)
+        if (e->class_ntiles[c] && e->class_tpa[c] != 1) return;
     const size_t N = e->ntot, room = pair_room(N, d.cap, d.single_type);
     if (room >= (size_t)PAIR_NEG) return;
     // sizes in whole 256 bytes, so that every array starts aligned
@@ -1114,6 +1119,10 @@ int autotune_tpa(mdgb_engine* e) {
         if (flags & E_NLIST) {
             rc = grow_list(e);
             if (!rc) rc = clear_err(e);
+            if (e->dev.pairs) {   // the larger list came with pair records: one thread per atom
+                for (int c = 0; c < NC; ++c) best_tpa[c] = 1;
+                break;
+            }
             --ci;  // same candidate again with the larger list
             continue;
         }
@@ -1402,6 +1411,15 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
     CU(cudaMemcpyAsync((void*)d.pair, pair_tab.data(), pair_tab.size() * sizeof(PairDev), cudaMemcpyHostToDevice,
                        e->stream));
 
+    // threads per atom: kept from the last tuning when the size classes are
+    // the same, else the configured (or default) value until the next tuning
+    // (before the list is allocated: the pair records go by it)
+    if (!same_classes) {
+        const int t0 = d.refmode ? 1 : (e->cfg.threads_per_atom > 0 ? e->cfg.threads_per_atom : 1);
+        for (int c = 0; c < NC; ++c) e->class_tpa[c] = t0;
+        e->tuned = false;
+    }
+
     // neighbour capacity from the densest replica (grows on overflow)
     int cap = e->cfg.neighbor_capacity;
     if (cap <= 0) {
@@ -1419,13 +1437,6 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
     e->st = mdgb_stats{};
     e->st.neighbor_capacity = e->cap;
 
-    // threads per atom: kept from the last tuning when the size classes are
-    // the same, else the configured (or default) value until the next tuning
-    if (!same_classes) {
-        const int t0 = d.refmode ? 1 : (e->cfg.threads_per_atom > 0 ? e->cfg.threads_per_atom : 1);
-        for (int c = 0; c < NC; ++c) e->class_tpa[c] = t0;
-        e->tuned = false;
-    }
     for (int r = 0; r < nrep; ++r) {
         e->rep_host[r].tpa = e->class_tpa[e->class_of[r]];
         e->rep_host[r].rlist = e->rcmax + class_skin_of(e, e->class_of[r]);

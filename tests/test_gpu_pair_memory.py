@@ -89,3 +89,49 @@ def test_a_longer_list_is_given_the_records_memory():
         assert np.array_equal(a[k], b[k]), k
     e.close()
     want.close()
+
+
+@pytest.mark.parametrize("how", ["another_upload", "a_longer_list"])
+def test_lists_of_several_threads_per_atom_get_no_records(how):
+    """Records that found no room at first, threads per atom tuned without them,
+    then room: the lists stay in the tuned layout, which the pair kernels do not
+    read."""
+    from moldyn_gb300.engine import Engine
+    types, pos, vel, mass, box = liquid()
+    two = types.copy()
+    two[::3] = 1
+    e = Engine(precision="fp64", trace=True)   # (phases are traced: single launches, tuned at any size)
+    for a, b in ((0, 0), (0, 1), (1, 1)):
+        e.set_potential(a, b, 1.0, 1.0)
+    held = hold_memory(0.45)
+    try:
+        if how == "another_upload":
+            e.upload(two, pos, vel, [1.0, 1.0], box)
+        else:
+            e.upload(types, pos, vel, mass, box)
+        e.compute_forces()
+    finally:
+        del held
+        give_back()
+    # (42 blocks of one thread per atom leave most of the chip idle)
+    assert max(e.stats().class_threads_per_atom) > 1
+    r_cut = 2.5
+    if how == "another_upload":
+        e.upload(types, pos, vel, mass, box)
+    else:
+        r_cut = 3.2
+        e.set_potential_raw(0, 0, 1.0, 1.0, r_cut, 0.0)
+        cap = e.stats().neighbor_capacity
+    e.compute_forces()
+    if how == "a_longer_list":
+        assert e.stats().neighbor_capacity > cap
+    want = engine(pair_records=False)
+    if r_cut != 2.5:
+        want.set_potential_raw(0, 0, 1.0, 1.0, r_cut, 0.0)
+    want.upload(types, pos, vel, mass, box)
+    want.compute_forces()
+    a, b = e.download(), want.download()
+    for k in ("force", "potential", "temp"):
+        assert np.abs(a[k] - b[k]).max() <= 1e-12 * np.abs(b[k]).max(), k
+    e.close()
+    want.close()
