@@ -97,8 +97,9 @@ constexpr int SORT_PER_LANE = 4;
 static __device__ __noinline__ void sort_lists_by_rank(const Dev& d, int s0, int n, long long rbeg, int rn) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+    __syncwarp();   // any lane may have written any entry (k_steps: one atom's list by all 32)
     if (n > 32 * SORT_PER_LANE) sort_list_by_rank(d, s0 + lane, n, 1, rbeg, rn);
-    __syncwarp();   // the lists are written by the lane of their atom
+    __syncwarp();
     unsigned todo = __ballot_sync(FULL, n > 1 && n <= 32 * SORT_PER_LANE);
     while (todo) {
         const int a = __ffs(todo) - 1;
