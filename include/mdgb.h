@@ -259,6 +259,8 @@ MDGB_API int mdgb_reset_stats(mdgb_engine* e);
  * returns MDGB_ERR_DEVICE_TIMEOUT and the state is restored to where the
  * chunk began, so the engine stays usable. */
 MDGB_API int mdgb_test_barrier_timeout(mdgb_engine* e, int hold_block, int64_t wait_cycles);
+/* The same in a later step (0, 1, ...) of that chunk. */
+MDGB_API int mdgb_test_barrier_timeout_at(mdgb_engine* e, int step, int hold_block, int64_t wait_cycles);
 MDGB_API int mdgb_synchronize(mdgb_engine* e);
 
 /* ---- allocation-free force evaluation -------------------------------- */

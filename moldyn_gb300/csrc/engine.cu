@@ -180,7 +180,7 @@ struct mdgb_engine {
     bool lists_fresh = false;
     // failure test of the bounded grid barrier (mdgb_test_barrier_timeout):
     // the next step call's first chunk holds this block back (-1: off)
-    int test_hold_block = -1;
+    int test_hold_block = -1, test_hold_step = 0;
     long long test_barrier_cycles = 0;
 
     // stats
@@ -787,6 +787,7 @@ int run_chunk_kernels(mdgb_engine* e, const StepParams& sp, int n) {
     for (int i = 0; i < n; ++i) {
         StepParams pre = sp;
         pre.predrifted = (i >= 1 && i <= nf) ? 1 : 0;
+        if (i != sp.hold_step) pre.hold_block = -1;
         int rc = launch_pre(e, pre);
         if (rc) return rc;
         StepParams frc = sp;
@@ -902,13 +903,15 @@ int step_impl(mdgb_engine* e, int64_t nsteps, double dt) {
     int retries = 0;
     while (done < nsteps) {
         const int n = (int)std::min<int64_t>(chunk, nsteps - done);
+        e->rep_fresh = false;   // until this chunk's steps stand
         int rc = begin_chunk(e);
         if (rc) return rc;
         if (e->test_hold_block >= 0) {
-            // the armed failure test: this chunk eager, its first step kernel
-            // with one block held back and a short wait limit
+            // the armed failure test: this chunk eager, one block of its first
+            // (or a later) step held back, and a short wait limit
             StepParams t = sp;
             t.hold_block = e->test_hold_block;
+            t.hold_step = e->test_hold_step;
             t.barrier_cycles = e->test_barrier_cycles;
             e->test_hold_block = -1;
             rc = run_chunk_kernels(e, t, n);
@@ -922,7 +925,6 @@ int step_impl(mdgb_engine* e, int64_t nsteps, double dt) {
         if (with_rep) CU(cudaMemcpyAsync(e->h_rep, e->dev.rep, sizeof(RepDev), cudaMemcpyDeviceToHost, e->stream));
         rc = read_err(e, &flags);
         if (rc) return rc;
-        e->rep_fresh = with_rep;
         if (flags & E_TIMEOUT) {
             // a grid barrier gave up: the rest of the chunk did nothing; put
             // the state back as the chunk found it, so the engine stays usable
@@ -948,6 +950,7 @@ int step_impl(mdgb_engine* e, int64_t nsteps, double dt) {
         }
         rc = check_flags(e, flags);
         if (rc) return rc;
+        e->rep_fresh = with_rep;
         done += n;
         e->st.steps += n;
     }
@@ -1982,7 +1985,12 @@ MDGB_API int mdgb_ensemble_prepare(mdgb_engine* e, int64_t nsteps, double dt) {
 }
 
 MDGB_API int mdgb_test_barrier_timeout(mdgb_engine* e, int hold_block, int64_t wait_cycles) {
-    if (!e || hold_block < 0 || wait_cycles <= 0) return MDGB_ERR_INVALID_ARGUMENT;
+    return mdgb_test_barrier_timeout_at(e, 0, hold_block, wait_cycles);
+}
+
+MDGB_API int mdgb_test_barrier_timeout_at(mdgb_engine* e, int step, int hold_block, int64_t wait_cycles) {
+    if (!e || step < 0 || hold_block < 0 || wait_cycles <= 0) return MDGB_ERR_INVALID_ARGUMENT;
+    e->test_hold_step = step;
     e->test_hold_block = hold_block;
     e->test_barrier_cycles = wait_cycles;
     return MDGB_OK;

@@ -233,9 +233,10 @@ class Engine:
                                                   C.byref(th) if th is not None else None,
                                                   C.byref(ba) if ba is not None else None))
 
-    def test_barrier_timeout(self, hold_block: int, wait_cycles: int):
-        """Arm the bounded-barrier failure test for the next step call."""
-        self._check(self._L.mdgb_test_barrier_timeout(self._h, int(hold_block), int(wait_cycles)))
+    def test_barrier_timeout(self, hold_block: int, wait_cycles: int, step: int = 0):
+        """Arm the bounded-barrier failure test for the next step call (its first
+        chunk's given step)."""
+        self._check(self._L.mdgb_test_barrier_timeout_at(self._h, int(step), int(hold_block), int(wait_cycles)))
 
     def download(self, out: dict | None = None, fields=("pos", "vel", "force", "potential", "temp")):
         """The state in the caller's atom order.  `out` may hold arrays to fill
