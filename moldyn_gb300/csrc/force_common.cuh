@@ -13,20 +13,6 @@ __device__ __forceinline__ void shift_table(float4* tab, const RepDev* R) {
     }
 }
 
-// The reference's FP64 displacement and distance (potential.rs:181-201).
-__device__ __forceinline__ double ref_distance(const double4_32a pi, const double4_32a pj, const double* box,
-                                               double& rx, double& ry, double& rz) {
-    rx = __dsub_rn(pj.x, pi.x);
-    ry = __dsub_rn(pj.y, pi.y);
-    rz = __dsub_rn(pj.z, pi.z);
-    const double hx = 0.5 * box[0], hy = 0.5 * box[1], hz = 0.5 * box[2];
-    if (rx < -hx) rx = __dadd_rn(rx, box[0]); else if (rx > hx) rx = __dsub_rn(rx, box[0]);
-    if (ry < -hy) ry = __dadd_rn(ry, box[1]); else if (ry > hy) ry = __dsub_rn(ry, box[1]);
-    if (rz < -hz) rz = __dadd_rn(rz, box[2]); else if (rz > hz) rz = __dsub_rn(rz, box[2]);
-    const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), __dmul_rn(rz, rz));
-    return __dsqrt_rn(r2);
-}
-
 // The reference's minimum image of one FP64 displacement component
 // (potential.rs:186-200: r < -L/2 -> r + L, r > L/2 -> r - L) with the
 // comparisons on the bit patterns (L/2 exact: exponent - 1): integer work

@@ -7,12 +7,11 @@
 // reference's single-shift rule (potential.rs:186-200).
 //
 // k_force_fp64  -- the plain path of systems without pair records
-//   (kernels_pairs.cu).  Every pair is evaluated with the reference's FP64
-//   operation sequence through explicit round-to-nearest intrinsics (no
-//   contraction), so each pair term carries the reference's bits; with
-//   MDGB_FLAG_REFERENCE_ORDER the list is in the reference's j order and the
-//   per-atom sums are bit-identical too.  An FP32 prefilter on the mirror
-//   skips candidates that are certainly outside r_cut.
+//   (kernels_pairs.cu), with the same pair terms (force_common.cuh): with
+//   MDGB_FLAG_REFERENCE_ORDER the bits of the reference's FP64 operation
+//   sequence, and the list in the reference's j order, so the per-atom sums are
+//   bit-identical too; in tree order functions of r^2.  An FP32 prefilter on
+//   the mirror skips candidates that are certainly outside r_cut.
 // k_force_mixed -- the chosen path.  FP32 pair maths from the float4 mirror
 //   (cell-relative coordinates, periodic cell shift from the list entry),
 //   force sums in deterministic 64-bit fixed point, potential/virial in FP32
@@ -115,25 +114,18 @@ __global__ void __launch_bounds__(TILE * TPA) k_force_fp64(Dev d, StepParams sp)
                     if (ex * ex + ey * ey + ez * ez > P.rc2f_hi * 1.0001f) continue;
                 }
                 const double4_32a pj = d.pos[j];
-                double rx, ry, rz;
-                const double r = ref_distance(pi, pj, box, rx, ry, rz);
-                if (r > P.rc) continue;                                          // :202-204
-                // potential.rs:57-75 get_potential_and_force
-                const double sr = __ddiv_rn(P.sigma, r);
-                const double s2 = __dmul_rn(sr, sr);
-                const double s4 = __dmul_rn(s2, s2);
-                const double s6 = __dmul_rn(s2, s4);
-                const double s12 = __dmul_rn(s6, s6);
-                const double u = __dsub_rn(__dmul_rn(P.eps4, __dsub_rn(s12, s6)), P.ucut);
-                const double dudr = __dmul_rn(__ddiv_rn(P.eps24, r), __dsub_rn(s6, __dmul_rn(2.0, s12)));
-                // :207-211
-                const double gx = __dmul_rn(__ddiv_rn(rx, r), dudr);
-                const double gy = __dmul_rn(__ddiv_rn(ry, r), dudr);
-                const double gz = __dmul_rn(__ddiv_rn(rz, r), dudr);
-                const double tt = __dadd_rn(__dadd_rn(__dmul_rn(gx, rx), __dmul_rn(gy, ry)), __dmul_rn(gz, rz));
-                fx = __dadd_rn(fx, gx); fy = __dadd_rn(fy, gy); fz = __dadd_rn(fz, gz);
-                pe = __dadd_rn(pe, u);
-                vr = __dadd_rn(vr, tt);
+                // the terms of k_pair_terms and k_steps: which of the three
+                // kernels runs (memory, size) moves no bit
+                const double rx = min_image_ref(__dsub_rn(pj.x, pi.x), box[0]);
+                const double ry = min_image_ref(__dsub_rn(pj.y, pi.y), box[1]);
+                const double rz = min_image_ref(__dsub_rn(pj.z, pi.z), box[2]);
+                const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), __dmul_rn(rz, rz));
+                PairTerms o;
+                if (!(d.refmode ? ref_terms<false>(rx, ry, rz, r2, P, o) : r2_terms<false>(rx, ry, rz, r2, P, o)))
+                    continue;
+                fx = __dadd_rn(fx, o.gx); fy = __dadd_rn(fy, o.gy); fz = __dadd_rn(fz, o.gz);
+                pe = __dadd_rn(pe, o.u);
+                vr = __dadd_rn(vr, o.t);
             }
         }
         if (TPA > 1) {
