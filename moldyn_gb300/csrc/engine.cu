@@ -123,6 +123,8 @@ struct mdgb_engine {
     void* nbr_alloc = nullptr;
     void* pair_alloc = nullptr;      // the FP64 path's pair records (Dev::pairs)
     int pair_single = 0;             // Dev::single_type they were sized for
+    bool pair_wanted = false;        // the last allocation's answer of pairs_wanted
+    double mean_density = 0.0;       // around an atom, at the upload
     // snapshot buffers (chunk retry)
     double4_32a* snap_pos = nullptr;
     double* snap_d = nullptr;   // [8][N]
@@ -332,17 +334,29 @@ int upload_pairs(mdgb_engine* e) {
 // liquid, which only saves time: half of the device's memory is left to what
 // has to be there (other engines' states and lists), and a caller who wants
 // all of it sets MDGB_FLAG_NO_PAIR_RECORDS.
+// Where an atom lists few others the four launches of the records cost more than
+// the pairs: 20 NVE steps with / without them, us, by the entries expected an
+// atom, 27,436 and 110,592 atoms in tree order: 2.8 811 / 578 and 1034 / 820, 4.6
+// 880 / 797 and 1202 / 1506, 7.4 988 / 1188 and 1526 / 2784; forces alone 28 / 17
+// at 1.8, 28 / 25 at 4.6, 52 / 115 at 7.4 (110,592).
 constexpr int PAIR_MIN_ATOMS = 4096;
+constexpr double PAIR_MIN_LISTED = 4.0;
+
+bool pairs_wanted(const mdgb_engine* e) {
+    if (e->cfg.precision != MDGB_PRECISION_FP64 || e->ntot < PAIR_MIN_ATOMS || e->cfg.threads_per_atom > 1 ||
+        (e->cfg.flags & MDGB_FLAG_NO_PAIR_RECORDS))
+        return false;
+    for (int c = 0; c < mdgb_engine::NCLASS; ++c)
+        if (e->class_ntiles[c] && e->class_tpa[c] != 1) return false;
+    return 4.0 / 3.0 * M_PI * std::pow(e->rlist, 3) * e->mean_density >= PAIR_MIN_LISTED;
+}
 
 void alloc_pairs(mdgb_engine* e) {
     Dev& d = e->dev;
     free_pairs(e);
     e->pair_single = d.single_type;
-    if (e->cfg.precision != MDGB_PRECISION_FP64 || e->ntot < PAIR_MIN_ATOMS || e->cfg.threads_per_atom > 1 ||
-        (e->cfg.flags & MDGB_FLAG_NO_PAIR_RECORDS))
-        return;
-    for (int c = 0; c < mdgb_engine::NCLASS; ++c)
-        if (e->class_ntiles[c] && e->class_tpa[c] != 1) return;
+    e->pair_wanted = pairs_wanted(e);
+    if (!e->pair_wanted) return;
     const size_t N = e->ntot, room = pair_room(N, d.cap, d.single_type);
     if (room >= (size_t)PAIR_NEG) return;
     // sizes in whole 256 bytes, so that every array starts aligned
@@ -1271,7 +1285,7 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
     const double rl_cells = e->rcmax + (auto_skin ? std::min(e->skin, SKIN_FRACTIONS[0] * e->rcmax) : e->skin);
     std::vector<int> cell_rep;
     int max_rep_n = 0;
-    double max_density = 0.0;
+    double max_density = 0.0, atom_density = 0.0;
     for (int r = 0; r < nrep; ++r) {
         RepDev& R = reps[r];
         const int nr = (int)(offsets[r + 1] - offsets[r]);
@@ -1284,6 +1298,7 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
         }
         const double vol = boxes[3 * r] * boxes[3 * r + 1] * boxes[3 * r + 2];
         max_density = std::max(max_density, nr / vol);
+        atom_density += nr * (nr / vol);
         // cell capacity: the grid at this box with room to grow (barostat), but
         // no finer than ~8 atoms a cell -- a dilute replica gets larger
         // cells, so its rebuild is not dominated by per-cell work
@@ -1423,6 +1438,7 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
         e->tuned = false;
     }
 
+    e->mean_density = atom_density / N;
     // neighbour capacity from the densest replica (grows on overflow)
     int cap = e->cfg.neighbor_capacity;
     if (cap <= 0) {
@@ -1434,8 +1450,9 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
     if (!e->nbr_alloc || cap > e->cap) {
         rc = alloc_nbr(e, cap);
         if (rc) return rc;
-    } else if (e->pair_single != d.single_type) {
-        alloc_pairs(e);   // as many records as list entries with several types
+    } else if (e->pair_single != d.single_type || e->pair_wanted != pairs_wanted(e)) {
+        // as many records as list entries with several types; none for a gas
+        alloc_pairs(e);
     }
     e->st = mdgb_stats{};
     e->st.neighbor_capacity = e->cap;

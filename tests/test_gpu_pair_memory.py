@@ -135,3 +135,15 @@ def test_lists_of_several_threads_per_atom_get_no_records(how):
         assert np.abs(a[k] - b[k]).max() <= 1e-12 * np.abs(b[k]).max(), k
     e.close()
     want.close()
+
+
+def test_records_go_with_the_length_of_the_lists():
+    """A gas of 1.4 entries an atom has no records; a liquid uploaded into the
+    same engine has them, and a gas after it gives them back."""
+    gas, dense = gs.fcc((11, 11, 11), rho=0.015, jitter=0.3, seed=4), gs.fcc((11, 11, 11), jitter=0.04, seed=3)
+    types = np.zeros(len(gas[0]), dtype=np.uint16)
+    e = engine()
+    for (pos, vel, box), want in ((gas, WITHOUT), (dense, WITH), (gas, WITHOUT)):
+        e.upload(types, pos, vel, [1.0], box)
+        assert launches(e) == want
+    e.close()
