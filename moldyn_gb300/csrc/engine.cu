@@ -768,9 +768,13 @@ int compute_forces_impl(mdgb_engine* e) {
 // atoms, 29 / 58 at 8,788, 43 / 60 at 23,328, 66 / 59 at 32,000; Berendsen T
 // and P 58 / 83, 75 / 83, 105 / 97 at 23,328 (the same crossing with
 // Nose-Hoover).
-constexpr int SMALL_MAX_ATOMS = 24576, SMALL_MAX_COUPLED = 12288;
+// An ensemble rebuilds some replica at nearly every step, and one block decides
+// for all of them: us for 20 NVE steps, one launch / launches, replicas of 64
+// atoms 2042 / 2760 at 64, 2748 / 3125 at 150, 3401 / 3365 at 300, 3642 / 3523 at
+// 380; of 27 atoms 2510 / 2602 at 300, 3865 / 3254 at 800.
+constexpr int SMALL_MAX_ATOMS = 24576, SMALL_MAX_COUPLED = 12288, SMALL_MAX_REPLICAS = 300;
 bool small_size(const mdgb_engine* e) {
-    return e->ntot <= SMALL_MAX_ATOMS && !e->dev.pairs && e->cfg.rebuild_every == 0 && e->steps_blocks_per_sm > 0 &&
+    return e->ntot <= SMALL_MAX_ATOMS && e->nrep <= SMALL_MAX_REPLICAS && !e->dev.pairs && e->cfg.rebuild_every == 0 && e->steps_blocks_per_sm > 0 &&
            e->cfg.threads_per_atom <= 1 &&
            !(e->cfg.flags & (MDGB_FLAG_PROFILE | MDGB_FLAG_TRACE | MDGB_FLAG_PERSISTENT));
 }

@@ -1537,10 +1537,9 @@ __device__ void phase_scan_a(const Dev& d, int chunk) {
     if (threadIdx.x == 0) d.bsum[blockIdx.x] = (int)v[0];
 }
 
-// Exclusive scan of the per-block sums by block 0 (each thread a contiguous run).
+// Exclusive scan of the per-block sums by one block (each thread a contiguous run).
 __device__ void phase_scan_b(const Dev& d) {
     __shared__ int part[TILE];
-    if (blockIdx.x != 0) return;
     const int G = gridDim.x;
     const int per = (G + blockDim.x - 1) / blockDim.x;
     const int b0 = threadIdx.x * per, b1 = min(b0 + per, G);
@@ -2086,7 +2085,7 @@ __device__ __forceinline__ void k_pre_rebuild(const Dev& d, const StepParams& sp
     phase_scan_a(d, chunk);
     if (grid_barrier(d)) return;
     clk.mark(TR_SCAN_A);
-    phase_scan_b(d);
+    if (blockIdx.x == 0) phase_scan_b(d);
     if (grid_barrier(d)) return;
     clk.mark(TR_SCAN_B);
     phase_scan_c(d, blockIdx.x * chunk, min((int)(blockIdx.x + 1) * chunk, d.ncells), __ldcg(d.bsum + blockIdx.x));
@@ -2452,9 +2451,16 @@ __device__ __noinline__ void steps_force_fp64(const Dev& d, const StepParams& sp
     }
 }
 
+// Cells up to which one block clears and scans them (a few round trips to L2 for
+// 128 cells); more, in ensembles of many replicas above all, take the whole grid
+// and three barriers more.  us for 20 NVE steps, one block / grid: 30 replicas of
+// 27 atoms (about 900 cells) 1576 / 1652, 64 of 64 atoms (2,240) 2055 / 2042, 128
+// (4,480) 2696 / 2450, 300 (10,500) 4406 / 3400.
+constexpr int STEPS_FEW_CELLS = 2048;
+
 // The rebuild decision of every replica (one block): decide_replica without
 // reading whole records where none is needed.  A rebuild's work list is made
-// and its cells are cleared here as well.
+// and its cells, where they are few, are cleared here as well.
 __device__ __noinline__ void steps_decide(const Dev& d, const StepParams& sp) {
     bool any = false;
     for (int r = threadIdx.x; r < d.nrep; r += blockDim.x) {
@@ -2470,7 +2476,7 @@ __device__ __noinline__ void steps_decide(const Dev& d, const StepParams& sp) {
     }
     if (__syncthreads_or(any)) {
         phase_work_list(d);
-        phase_zero_cells(d, 0, 1);
+        if (d.ncells <= STEPS_FEW_CELLS) phase_zero_cells(d, 0, 1);
     }
 }
 
@@ -2585,11 +2591,28 @@ __device__ __noinline__ void steps_lists(const Dev& d, uint32_t* smem) {
     }
 }
 
-// The rebuild of k_pre with the scans in the last block to arrive, then the
-// lists and the end of the rebuild.
-__device__ __noinline__ bool steps_rebuild(const Dev& d, uint32_t* st_smem) {
+// Clearing, binning and scanning of many cells by the whole grid, as k_pre does.
+__device__ __noinline__ bool steps_sort_many(const Dev& d) {
+    const int chunk = (d.ncells + gridDim.x - 1) / gridDim.x;
+    phase_zero_cells(d, blockIdx.x, gridDim.x);
+    if (grid_barrier(d)) return true;
     phase_bin(d);
-    if (grid_barrier_then(d, [&] { phase_scan_c(d, 0, d.ncells, 0); })) return true;
+    if (grid_barrier(d)) return true;
+    phase_scan_a(d, chunk);
+    if (grid_barrier_then(d, [&] { phase_scan_b(d); })) return true;
+    phase_scan_c(d, blockIdx.x * chunk, min((int)(blockIdx.x + 1) * chunk, d.ncells), __ldcg(d.bsum + blockIdx.x));
+    return grid_barrier(d);
+}
+
+// The rebuild of k_pre with the scan of few cells in the last block to arrive,
+// then the lists and the end of the rebuild.
+__device__ __noinline__ bool steps_rebuild(const Dev& d, uint32_t* st_smem) {
+    if (d.ncells > STEPS_FEW_CELLS) {
+        if (steps_sort_many(d)) return true;
+    } else {
+        phase_bin(d);
+        if (grid_barrier_then(d, [&] { phase_scan_c(d, 0, d.ncells, 0); })) return true;
+    }
     phase_scatter(d, false);
     if (grid_barrier(d)) return true;
     if (d.mixed) phase_sort_gather<true>(d, false); else phase_sort_gather<false>(d, false);
