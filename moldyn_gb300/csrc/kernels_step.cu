@@ -1237,10 +1237,15 @@ __device__ bool phase_serial(const Dev& d, const StepParams& sp, int sel, bool c
 }
 
 // The stages that follow a pass over the tiles: chunk sums, then a finalize
-// step.  With a few chunks (a few replicas of at most some ten thousand atoms)
+// step.  With up to four chunks (a replica has one for every 32,768 atoms)
 // the last block to arrive at the barrier does both; otherwise they are phases
 // of their own.  Returns true when the launch must stop.
-constexpr int THEN_MAX_CHUNKS = 16;
+// The block has a warp for each of four chunks, or replicas, at a time: us in the
+// last block / as phases, FP64 with both Berendsen couplings, 20 steps: replicas of
+// 4,096 atoms 3465 / 3588 at 4, 4376 / 4283 at 6, 8889 / 8339 at 16, one system of
+// 110,592 atoms (4 chunks) 10851 / 10999, of 442,368 (14) 31240 / 31007; mixed, 16
+// replicas of 512 atoms in one launch 2292 / 1775, Nose-Hoover 3311 / 2365.
+constexpr int THEN_MAX_CHUNKS = TILE / 32;
 template <int NS, class F>
 __device__ __forceinline__ bool sums_then(const Dev& d, F finalize) {
     if (d.nchunks <= THEN_MAX_CHUNKS)
