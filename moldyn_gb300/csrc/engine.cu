@@ -88,7 +88,7 @@ struct mdgb_engine {
     // the GPU reads the caller's pageable arrays itself (Grace: address
     // translation through the host's page tables), so uploads skip the copy
     bool host_direct = false;
-    int pre_blocks_per_sm = 0, steps_blocks_per_sm = 0;
+    int pre_blocks_per_sm = 0, macro_blocks_per_sm = 0, steps_blocks_per_sm = 0;
     int force_blocks_per_sm[4] = {0, 0, 0, 0};
     LJ pot[MAX_TYPES][MAX_TYPES];
     LJ pot_default;
@@ -433,8 +433,9 @@ void prof_collect(mdgb_engine* e) {
     e->prof.clear();
 }
 
-int pre_grid(const mdgb_engine* e) {
-    const int maxg = std::min(4096, std::max(1, e->num_sms * e->pre_blocks_per_sm));  // bsum holds 4096
+// Blocks of k_pre or k_macro: no more than are resident.
+int pre_grid(const mdgb_engine* e, int blocks_per_sm) {
+    const int maxg = std::min(4096, std::max(1, e->num_sms * blocks_per_sm));  // bsum holds 4096
     // reference order: one block per serial fold (six a replica at most)
     const int folds = e->dev.refmode ? 6 * std::min(e->nrep, maxg) : 1;
     const int want = std::max({e->ntiles, (e->ncells + 1023) / 1024, (e->nrep + TILE - 1) / TILE, folds});
@@ -445,7 +446,7 @@ int launch_pre(mdgb_engine* e, const StepParams& sp) {
     cudaEvent_t pe;
     prof_begin(e, 1, &pe);
     cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(pre_grid(e));
+    lc.gridDim = dim3(pre_grid(e, e->pre_blocks_per_sm));
     lc.blockDim = dim3(TILE);
     lc.stream = e->stream;
     cudaLaunchAttribute at[1];
@@ -1708,7 +1709,7 @@ int macro_impl(mdgb_engine* e, int type, mdgb_macro* out) {
     if (rc) return rc;
     StepParams sp = make_sp(e, 0.0, false);
     cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(pre_grid(e));
+    lc.gridDim = dim3(pre_grid(e, e->macro_blocks_per_sm));
     lc.blockDim = dim3(TILE);
     lc.stream = e->stream;
     cudaLaunchAttribute at[1];
@@ -1818,7 +1819,8 @@ MDGB_API int mdgb_create(const mdgb_config* cfg, mdgb_engine** out) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, (const void*)k_pre, TILE, 0);
     int bps2 = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps2, (const void*)k_macro, TILE, 0);
-    e->pre_blocks_per_sm = std::max(1, std::min(bps, bps2));
+    e->pre_blocks_per_sm = std::max(1, bps);
+    e->macro_blocks_per_sm = std::max(1, bps2);
     if (steps_init(&e->steps_blocks_per_sm) != cudaSuccess) { delete e; return MDGB_ERR_CUDA; }
     if (list_build_init() != cudaSuccess) { cudaGetLastError(); delete e; return MDGB_ERR_CUDA; }
     lj_finish(e->pot_default);

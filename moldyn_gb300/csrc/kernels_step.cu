@@ -2729,7 +2729,8 @@ cudaError_t launch_steps(const Dev& d, const StepParams& sp, int n, bool naive, 
 
 // Macro parameters of type `sel` (solver/src/macro_parameters): results land
 // in the replica records (vcm, mom, ke, pe, thermal, T, P, count).
-// 6 blocks per SM, as k_pre: the engine launches both on one grid size.
+// 6 blocks per SM (80 registers), on a grid of its own: at k_pre's five 1.6M atoms
+// took 204 us instead of 192.
 __global__ void __launch_bounds__(TILE, 6) k_macro(Dev d, StepParams sp, int sel) {
     barrier_setup(sp);
     tile_rep_reset();
