@@ -108,6 +108,11 @@ struct mdgb_engine {
     static constexpr int NCLASS = 3;
     std::vector<int> class_of;       // per replica
     int class_tpa[NCLASS] = {1, 1, 1};
+    // sizes of the one-launch kernel: whether the lists are in the timed layout,
+    // what the timing chose, and steps lately taken that the other layout suits
+    bool timed_layout = false, timed = false;
+    int timed_tpa[NCLASS] = {1, 1, 1};
+    int64_t off_layout = 0;
     int class_ntiles[NCLASS] = {0, 0, 0};
     int class_tile_off[NCLASS] = {0, 0, 0};   // offset into dev.tile_order
     int class_nrep[NCLASS] = {0, 0, 0};
@@ -773,14 +778,17 @@ int compute_forces_impl(mdgb_engine* e) {
 // for all of them: us for 20 NVE steps, one launch / launches, replicas of 64
 // atoms 2042 / 2760 at 64, 2748 / 3125 at 150, 3401 / 3365 at 300, 3642 / 3523 at
 // 380; of 27 atoms 2510 / 2602 at 300, 3865 / 3254 at 800.
+constexpr int TUNE_MIN_ATOMS = 4096;   // fewer: threads per atom are not worth measuring
 constexpr int SMALL_MAX_ATOMS = 24576, SMALL_MAX_COUPLED = 12288, SMALL_MAX_REPLICAS = 300;
 bool small_size(const mdgb_engine* e) {
     return e->ntot <= SMALL_MAX_ATOMS && e->nrep <= SMALL_MAX_REPLICAS && !e->dev.pairs && e->cfg.rebuild_every == 0 && e->steps_blocks_per_sm > 0 &&
            e->cfg.threads_per_atom <= 1 &&
            !(e->cfg.flags & (MDGB_FLAG_PROFILE | MDGB_FLAG_TRACE | MDGB_FLAG_PERSISTENT));
 }
+// Steps of such a size that run as launches all the same.
+bool steps_as_launches(const mdgb_engine* e, bool coupled) { return coupled && e->ntot > SMALL_MAX_COUPLED; }
 bool small_system(const mdgb_engine* e, const StepParams& sp) {
-    if (!small_size(e) || ((sp.coupled || sp.thermo_nh) && e->ntot > SMALL_MAX_COUPLED)) return false;
+    if (!small_size(e) || steps_as_launches(e, sp.coupled || sp.thermo_nh)) return false;
     for (int c = 0; c < mdgb_engine::NCLASS; ++c)
         if (e->class_ntiles[c] && e->class_tpa[c] != 1) return false;
     return true;
@@ -901,14 +909,14 @@ int run_chunk(mdgb_engine* e, const StepParams& sp, int n) {
 // Chunk lengths a call of nsteps steps runs: full chunks, then the rest.
 int chunk_steps(const mdgb_engine* e) { return e->cfg.graph_steps > 1 ? e->cfg.graph_steps : 64; }
 
-int autotune_tpa(mdgb_engine* e);
+int settle_tpa(mdgb_engine* e, bool launches, int64_t steps);
 int autotune_skin(mdgb_engine* e, double dt);
 
 int step_impl(mdgb_engine* e, int64_t nsteps, double dt) {
     if (!e->has_state) return fail(e, MDGB_ERR_NO_STATE, "no state uploaded");
     if (nsteps < 0 || !(dt == dt)) return fail(e, MDGB_ERR_INVALID_ARGUMENT, "bad nsteps or dt");
-    if (!e->tuned) {
-        int rc = autotune_tpa(e);
+    {
+        const int rc = settle_tpa(e, steps_as_launches(e, e->thermo_on || e->baro_on), nsteps);
         if (rc) return rc;
     }
     if (nsteps > 0 && !e->skin_tuned && skin_auto(e)) {
@@ -990,9 +998,13 @@ int prepare_impl(mdgb_engine* e, int64_t nsteps, double dt, bool thermo_on, bool
     if (!e->has_state) return fail(e, MDGB_ERR_NO_STATE, "no state uploaded");
     if (nsteps < 0 || !(dt == dt)) return fail(e, MDGB_ERR_INVALID_ARGUMENT, "bad nsteps or dt");
     if (!(e->cfg.graph_steps > 1)) return MDGB_OK;   // eager engine: nothing to capture
-    if (!e->tuned) {
-        int rc = autotune_tpa(e);
+    {
+        // the layout that call will choose, without counting its steps here
+        const int64_t off = e->off_layout;
+        const bool layout = e->timed_layout;
+        const int rc = settle_tpa(e, steps_as_launches(e, thermo_on || baro_on), nsteps);
         if (rc) return rc;
+        if (layout == e->timed_layout) e->off_layout = off;
     }
     const bool t0 = e->thermo_on, b0 = e->baro_on, n0 = e->thermo_nh;
     if (nsteps > 0 && !e->skin_tuned && skin_auto(e)) {
@@ -1089,19 +1101,63 @@ int autotune_skin(mdgb_engine* e, double dt) {
     return rc;
 }
 
+// The lists in the layout of these threads per atom for each size class.
+int use_tpa(mdgb_engine* e, const int (&tpa)[mdgb_engine::NCLASS]) {
+    const int NC = mdgb_engine::NCLASS;
+    for (int c = 0; c < NC; ++c) e->class_tpa[c] = tpa[c];
+    e->tpa = tpa[0];
+    for (int c = NC - 1; c >= 0; --c)
+        if (e->class_ntiles[c]) { e->tpa = tpa[c]; break; }
+    e->st.threads_per_atom = e->tpa;
+    const int rc = apply_class_tpa(e);
+    if (rc) return rc;
+    return e->lists_fresh ? MDGB_OK : rebuild_lists(e);
+}
+
+int autotune_tpa(mdgb_engine* e);
+
+// Threads per atom for the calls to come.  Sizes of the one-launch kernel take
+// one (it shares an atom's list out itself), but what runs as launches there,
+// coupled steps of the larger ones and forces alone, is faster with what a timing
+// chooses (us, mixed path, one thread / timed: forces of 13,500 atoms 41 / 31, a
+// step with both Berendsen couplings 77 / 66).  Changing the layout costs a
+// rebuild and the first timing about a millisecond, so it waits for PATIENCE steps
+// (a force evaluation is one) that the other layout suits.
+constexpr int PATIENCE = 32;
+int settle_tpa(mdgb_engine* e, bool launches, int64_t steps) {
+    const bool fixed = e->dev.refmode || e->dev.pairs || e->cfg.threads_per_atom > 0;
+    if (fixed || small_size(e)) {
+        if (!e->tuned) {
+            const int t = e->cfg.threads_per_atom > 0 && !e->dev.refmode ? e->cfg.threads_per_atom : 1;
+            e->tuned = true;
+            e->timed_layout = false;
+            e->off_layout = 0;
+            const int rc = use_tpa(e, {t, t, t});
+            if (rc) return rc;
+        }
+        if (fixed || e->ntot < TUNE_MIN_ATOMS || launches == e->timed_layout) {
+            e->off_layout = 0;
+            return MDGB_OK;
+        }
+        e->off_layout += steps;
+        if (e->off_layout < PATIENCE) return MDGB_OK;
+        e->off_layout = 0;
+        e->timed_layout = launches;
+        if (!launches) return use_tpa(e, {1, 1, 1});
+        return e->timed ? use_tpa(e, e->timed_tpa) : autotune_tpa(e);
+    }
+    return e->tuned ? MDGB_OK : autotune_tpa(e);
+}
+
 // Threads per atom for each size class: every candidate is timed on every
 // class at once (each class's launch bracketed by its own events), and each
 // class keeps its fastest.
 int autotune_tpa(mdgb_engine* e) {
     e->tuned = true;
     const int NC = mdgb_engine::NCLASS;
-    if (e->dev.refmode || e->dev.pairs || e->cfg.threads_per_atom > 0 || small_size(e)) {
-        const int t = e->cfg.threads_per_atom > 0 && !e->dev.refmode ? e->cfg.threads_per_atom : 1;
-        for (int c = 0; c < NC; ++c) e->class_tpa[c] = t;
-        e->tpa = t;
-        int rc = apply_class_tpa(e);
+    if (!e->lists_fresh) {   // the tuning's rebuilds then keep the atoms' order, and with it the forces'
+        const int rc = rebuild_lists(e);
         if (rc) return rc;
-        return e->lists_fresh ? MDGB_OK : rebuild_lists(e);
     }
     e->lists_fresh = false;
     // Keep the caller's forces: tuning evaluates forces into scratch.
@@ -1121,7 +1177,7 @@ int autotune_tpa(mdgb_engine* e) {
     int rc = MDGB_OK;
     for (int ci = 0; ci < 4 && !rc; ++ci) {
         const int cand = cands[ci];
-        if (e->ntot < 4096 && cand > 1) break;  // tiny systems: not worth measuring
+        if (e->ntot < TUNE_MIN_ATOMS && cand > 1) break;
         for (int c = 0; c < NC; ++c) e->class_tpa[c] = cand;
         rc = apply_class_tpa(e);
         if (!rc) rc = clear_err(e);
@@ -1158,17 +1214,13 @@ int autotune_tpa(mdgb_engine* e) {
     e->cfg.flags = saved_flags;
     for (int c = 0; c < NC; ++c) { cudaEventDestroy(ev[c][0]); cudaEventDestroy(ev[c][1]); }
     if (rc) return rc;
-    for (int c = 0; c < NC; ++c) e->class_tpa[c] = best_tpa[c];
-    e->tpa = best_tpa[0];
-    for (int c = NC - 1; c >= 0; --c)
-        if (e->class_ntiles[c]) { e->tpa = best_tpa[c]; break; }
-    e->st.threads_per_atom = e->tpa;
+    for (int c = 0; c < NC; ++c) e->timed_tpa[c] = best_tpa[c];
+    e->timed = true;
     CU(cudaMemcpyAsync(e->dev.frc, e->snap_d, 3 * N * sizeof(double), cudaMemcpyDeviceToDevice, e->stream));
     CU(cudaMemcpyAsync(e->dev.epot, e->snap_d + 3 * N, N * sizeof(double), cudaMemcpyDeviceToDevice, e->stream));
     CU(cudaMemcpyAsync(e->dev.evir, e->snap_d + 4 * N, N * sizeof(double), cudaMemcpyDeviceToDevice, e->stream));
-    rc = apply_class_tpa(e);
-    if (rc) return rc;
-    return rebuild_lists(e);  // lists in the chosen layouts
+    e->lists_fresh = false;
+    return use_tpa(e, best_tpa);
 }
 
 // Counts of every type per tile (exclusive over the tiles of a replica when
@@ -1457,7 +1509,7 @@ int upload_impl(mdgb_engine* e, int nrep, const int64_t* offsets, const uint16_t
     if (!same_classes) {
         const int t0 = d.refmode ? 1 : (e->cfg.threads_per_atom > 0 ? e->cfg.threads_per_atom : 1);
         for (int c = 0; c < NC; ++c) e->class_tpa[c] = t0;
-        e->tuned = false;
+        e->tuned = e->timed = false;
     }
 
     e->mean_density = atom_density / N;
@@ -1990,11 +2042,9 @@ MDGB_API int mdgb_compute_forces(mdgb_engine* e) {
     if (!e) return MDGB_ERR_INVALID_ARGUMENT;
     if (!e->has_state) return fail(e, MDGB_ERR_NO_STATE, "no state uploaded");
     cudaSetDevice(e->device);
-    if (!e->tuned) {
-        int rc = autotune_tpa(e);
-        if (rc) return rc;
-    }
-    int rc = compute_forces_impl(e);
+    int rc = settle_tpa(e, true, 1);
+    if (rc) return rc;
+    rc = compute_forces_impl(e);
     if (!rc) e->forces_valid = true;
     return rc;
 }
