@@ -1,6 +1,6 @@
 """The two Verlet-list builds (kernels_list.cu) give the same lists.
 
-The paired build (replicas of at least 32,768 atoms) tests each pair of
+The paired build (large replicas, and smaller ones with room in their cells) tests each pair of
 neighbouring cells once and expands per-(atom, shift code) hit words; the
 direct build (smaller replicas, MDGB_FLAG_DIRECT_LIST, and the engine's own
 choice for a rebuild with a cell of more than 32 atoms) tests every cell
