@@ -804,8 +804,16 @@ int run_chunk_kernels(mdgb_engine* e, const StepParams& sp, int n) {
         Dev d = e->dev;
         d.pos_next = e->pos_alt;
         d.mir_next = e->mir_alt;
-        CU(launch_steps(d, sp, n, e->cfg.precision == MDGB_PRECISION_FP32_NAIVE, e->num_sms * e->steps_blocks_per_sm,
-                        e->stream));
+        const bool naive = e->cfg.precision == MDGB_PRECISION_FP32_NAIVE;
+        const int blocks = e->num_sms * e->steps_blocks_per_sm;
+        // (the failure test in a later step: the steps before it by themselves)
+        const int before = sp.hold_block >= 0 ? std::min(sp.hold_step, n - 1) : 0;
+        if (before > 0) {
+            StepParams clean = sp;
+            clean.hold_block = -1;
+            CU(launch_steps(d, clean, before, naive, blocks, e->stream));
+        }
+        CU(launch_steps(d, sp, n - before, naive, blocks, e->stream));
         e->st.kernel_launches++;
         return MDGB_OK;
     }

@@ -2647,16 +2647,15 @@ __global__ void __launch_bounds__(TILE, 4) k_steps(Dev d_in, StepParams sp_in, i
     StepParams sp = sp_in;
     barrier_setup(sp, true);
     tile_rep_reset();
+    if (sp.hold_block == (int)blockIdx.x && threadIdx.x == 0) {   // failure test, as in k_pre
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2 * g_bar_limit) __nanosleep(1000);
+    }
     __syncthreads();
     const int row = STEPS_SMEM / 4 / (TILE / lanes);   // list words shared memory holds per atom
     const bool fusable = !sp.coupled && !sp.thermo_nh;
     const int nf = fusable ? ((n - 1) & ~1) : 0;
-    const int hold_at = sp_in.hold_block == (int)blockIdx.x ? sp_in.hold_step : -1;
     for (int i = 0; i < n; ++i) {
-        if (i == hold_at && threadIdx.x == 0) {   // failure test, as in k_pre
-            const long long t0 = clock64();
-            while (clock64() - t0 < 2 * g_bar_limit) __nanosleep(1000);
-        }
         const bool predrifted = i >= 1 && i <= nf;
         if (!predrifted && steps_motion(d, sp)) return;
         if (grid_barrier_then(d, [&] { steps_decide(d, sp); })) return;

@@ -136,7 +136,7 @@ struct StepParams {
     int fused;                 // force pass: also the next step's kick and drift (into pos_next/mir_next)
     int hold_block;            // >= 0: that block of the step kernel enters its first grid barrier late
                                //   (failure test of the bounded barrier; -1 in every normal step)
-    int hold_step, pad_hs;     // in that step of the chunk
+    int hold_step, pad_hs;     // in that step of the chunk (read by the host)
     long long barrier_cycles;  // > 0: the grid barrier's wait limit in clock cycles (0: the default, ~2 s)
 };
 
