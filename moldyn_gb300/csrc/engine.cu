@@ -621,13 +621,6 @@ int clear_err(mdgb_engine* e) {
     return MDGB_OK;
 }
 
-// What a chunk needs to be run again, copied aside, and the error words and the
-// barrier cleared, in one launch: for small states the eleven copies and two
-// clears were most of a step call's launches.  (From 262,144 atoms on the
-// copies themselves are what counts.)
-constexpr int SNAP_KERNEL_MAX = 262144;
-int begin_chunk(mdgb_engine* e);
-
 int snapshot(mdgb_engine* e, bool restore) {
     const size_t N = e->ntot;
     auto cp = [&](void* dst, const void* src, size_t bytes) {
@@ -662,11 +655,11 @@ int snapshot(mdgb_engine* e, bool restore) {
     return MDGB_OK;
 }
 
+// What a chunk needs to be run again, copied aside, and the error words and the
+// barrier cleared, in one launch instead of eleven copies and two clears.  us a
+// call of one step, copies / one launch: 70,304 atoms 133 / 79, 256,000 167 / 135,
+// 442,368 228 / 188, 1M 432 / 358, 4M 1245 / 1206.
 int begin_chunk(mdgb_engine* e) {
-    if (e->ntot >= SNAP_KERNEL_MAX) {
-        const int rc = clear_err(e);
-        return rc ? rc : snapshot(e, false);
-    }
     const size_t N = e->ntot;
     Dev& d = e->dev;
     const SnapArrays a{{e->snap_pos, e->snap_d, e->snap_d + 3 * N, e->snap_d + 6 * N, e->snap_d + 7 * N, e->snap_i,
