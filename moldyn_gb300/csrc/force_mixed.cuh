@@ -41,22 +41,21 @@ struct FixAcc {
 };
 
 // One term per accumulator pair, with the term already divided by 2^23
-// (t = v / 2^23; the scaling is exact) and not rounded before it is split: a =
-// fma(d, g, M) holds M + rint(t) = M + h, l' = fma(d, g, -h) is t - h rounded
-// once, and fma(l', 2^23, M) = M + rint(v - h 2^23).  The x and y components go
-// through the paired instructions together, with -l' (no negation to issue: 60
-// steps of 1M atoms 16187 -> 16120 us).  Written as a product and sums, the
-// assembler fused the paired ones, in a unit without contraction as well.
+// (t = v / 2^23; the scaling is exact): a = t + M holds M + rint(t) = M + h,
+// l' = t - h is exact (Sterbenz) and fma(l', 2^23, M) = M + rint(v - h 2^23).
+// The x and y components go through the paired instructions together.
 __device__ __forceinline__ void fix_add_xyz(FixAcc& ax, FixAcc& ay, FixAcc& az, f2_t dxy, float dz, float g) {
     const f2_t M2 = f2(FIX_MAGIC, FIX_MAGIC);
-    const f2_t a2 = fma2(dxy, f2(g, g), M2);
-    const f2_t n2 = fma2(dxy, f2(-g, -g), sub2(a2, M2));
-    const f2_t b2 = fma2(n2, f2(-8388608.0f, -8388608.0f), M2);
+    const f2_t K2 = f2(8388608.0f, 8388608.0f);
+    const f2_t t2 = mul2(dxy, f2(g, g));
+    const f2_t a2 = add2(t2, M2);
+    const f2_t l2 = sub2(t2, sub2(a2, M2));
+    const f2_t b2 = fma2(l2, K2, M2);
     ax.hi += (unsigned)a2 - FIX_MAGIC_BITS;
     ay.hi += (unsigned)(a2 >> 32) - FIX_MAGIC_BITS;
     ax.lo += (unsigned)b2 - FIX_MAGIC_BITS;
     ay.lo += (unsigned)(b2 >> 32) - FIX_MAGIC_BITS;
-    const float az_ = fmaf(dz, g, FIX_MAGIC);
+    const float az_ = fmaf(dz, g, FIX_MAGIC);   // one rounding: dz g is not rounded before
     const float lz = fmaf(dz, g, -__fsub_rn(az_, FIX_MAGIC));
     const float bz = fmaf(lz, 8388608.0f, FIX_MAGIC);
     az.hi += __float_as_uint(az_) - FIX_MAGIC_BITS;

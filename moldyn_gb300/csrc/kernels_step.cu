@@ -2264,8 +2264,8 @@ __device__ __noinline__ void steps_force_mixed(const Dev& d, const StepParams& s
                     lj_f32(P, r2, fs, uu);
                     if (!NAIVE) acc.add(dxy, dz, r2, fs, uu, fscale_t);
                     if (NOE && !NAIVE) {
-                        // (there dx g is rounded before it is split;
-                        // fix_add_xyz does not round it)
+                        // (there dx g is rounded before it is split; here
+                        // the paired instructions fuse the two)
                         const float g = __fmul_rn(fs, fscale_t), dd[3] = {f2_lo(dxy), f2_hi(dxy), dz};
 #pragma unroll
                         for (int c = 0; c < 3; ++c) {
