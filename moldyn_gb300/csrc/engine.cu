@@ -330,9 +330,12 @@ int upload_pairs(mdgb_engine* e) {
 }
 
 // The FP64 path's pair records for the current list capacity.  From
-// PAIR_MIN_ATOMS atoms on the pairs are computed once (kernels_pairs.cu);
-// below, where a step is a few launches of latency, and with several threads
-// per atom, k_force_fp64 evaluates both sides.  The pair kernels walk the lists
+// PAIR_MIN_ATOMS atoms on the pairs are computed once (kernels_pairs.cu); below,
+// steps run as one launch, and with several threads per atom k_force_fp64
+// evaluates both sides.  20 NVE steps with records / as one launch, us: tree order
+// 1630 / 1245 at 4,000 atoms, 1700 / 1442 at 5,324, 1762 / 2487 at 8,788, reference
+// order 1955 / 1762, 2077 / 2192, 2249 / 3966; forces alone 65 / 165 and 78 / 275 at
+// 4,000.  The pair kernels walk the lists
 // in the layout of one thread per atom, so there are records only while every
 // size class has that layout: a state whose records found no room when it was
 // uploaded may since have been tuned to another one.  About 4 KB an atom in a
@@ -763,10 +766,11 @@ int compute_forces_impl(mdgb_engine* e) {
 // Whether a chunk of this state's steps runs as one launch (k_steps): few
 // enough atoms that the step is launch latency and a mostly idle chip, one
 // thread per atom in the list layout, and nothing that looks at single
-// launches.  us a step, one launch / launches, mixed path: NVE 20 / 55 at 2,016
-// atoms, 29 / 58 at 8,788, 43 / 60 at 23,328, 66 / 59 at 32,000; Berendsen T
-// and P 58 / 83, 75 / 83, 105 / 97 at 23,328 (the same crossing with
-// Nose-Hoover).
+// launches.  us a step, one launch / launches, mixed path: NVE 19 / 51 at 4,000
+// atoms, 23 / 51 at 8,788, 35 / 51 at 23,328, 66 / 59 at 32,000; Berendsen T
+// and P 55 / 74, 66 / 75, 68 / 74 at 10,976, 70 / 77 (66 in the timed layout) at
+// 13,500, 84 / 76 at 16,384; Nose-Hoover 93 / 97 at 10,976, 98 / 100 (90) at 13,500,
+// 107 / 98 at 16,384.
 // An ensemble rebuilds some replica at nearly every step, and one block decides
 // for all of them: us for 20 NVE steps, one launch / launches, replicas of 64
 // atoms 2042 / 2760 at 64, 2748 / 3125 at 150, 3401 / 3365 at 300, 3642 / 3523 at
@@ -774,8 +778,8 @@ int compute_forces_impl(mdgb_engine* e) {
 constexpr int TUNE_MIN_ATOMS = 4096;   // fewer: threads per atom are not worth measuring
 constexpr int SMALL_MAX_ATOMS = 24576, SMALL_MAX_COUPLED = 12288, SMALL_MAX_REPLICAS = 300;
 bool small_size(const mdgb_engine* e) {
-    return e->ntot <= SMALL_MAX_ATOMS && e->nrep <= SMALL_MAX_REPLICAS && !e->dev.pairs && e->cfg.rebuild_every == 0 && e->steps_blocks_per_sm > 0 &&
-           e->cfg.threads_per_atom <= 1 &&
+    return e->ntot <= SMALL_MAX_ATOMS && e->nrep <= SMALL_MAX_REPLICAS && !e->dev.pairs &&
+           e->cfg.rebuild_every == 0 && e->steps_blocks_per_sm > 0 && e->cfg.threads_per_atom <= 1 &&
            !(e->cfg.flags & (MDGB_FLAG_PROFILE | MDGB_FLAG_TRACE | MDGB_FLAG_PERSISTENT));
 }
 // Steps of such a size that run as launches all the same.

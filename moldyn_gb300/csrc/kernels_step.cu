@@ -1028,6 +1028,9 @@ __device__ double serial_sum(const double* x, long long n, double c) {
         const bool ok = !near && ez > 0 && ez < 0x7FF && climb <= 3 && deep < 24;
         r.mask = ok && climb > 0 ? (1 << climb) - 1 : 0;
         r.base = zb & ~(long long)r.mask;
+        // (a start lies a multiple of mask + 1 from the run it is taken over from, and
+        // so does lim, a power of two: less than lim from z, too, whose running
+        // values were looked at)
         r.lim = ok ? (int)(SS_NEAR >> deep) : 0;
         r.shift = (int)((eb >> 52) & 0x7FF) - ez;
         r.flip = (int)((unsigned long long)(zb ^ eb) >> 63);
@@ -1132,8 +1135,7 @@ __device__ void phase_serial_terms1(const Dev& d, int sel, bool coupling) {
     }
 }
 
-// Centre-of-mass velocity of replica r from the pass-1 folds.
-// Pass 2: row 0 thermal energy, rows 1-3 (as one) the pressure's three terms
+// Pass 2, with the centre-of-mass velocity from the pass-1 folds: row 0 thermal energy, rows 1-3 (as one) the pressure's three terms
 // of every atom, row 4 the negated virial.
 __device__ void phase_serial_terms2(const Dev& d, int sel) {
     const int N = d.ntot;

@@ -243,9 +243,6 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// The rebuild work list (Dev::rb): replica ids and prefix offsets of their
-// cells and tiles.  Work item w (a cell or a tile of a rebuilding replica,
-// counted over the list) -> the list position i with off[i] <= w < off[i+1].
 // Which replicas take the paired list build.  The list phase of a step by the
 // lower limit (512 replicas of 64 to 64,000 atoms, 74 of them rebuilt a step):
 // 4,096 568 us, 6,144 525, 8,192 521, 16,384 536, 32,768 561; one system of
@@ -259,6 +256,10 @@ __host__ __device__ __forceinline__ bool list_paired(int atoms, int cells) {
     return atoms >= LIST_PAIRED_ANY_ATOMS ||
            (atoms >= LIST_PAIRED_MIN_ATOMS && atoms <= LIST_PAIRED_CELL_ATOMS * cells);
 }
+
+// The rebuild work list (Dev::rb): replica ids and prefix offsets of their
+// cells and tiles.  Work item w (a cell or a tile of a rebuilding replica,
+// counted over the list) -> the list position i with off[i] <= w < off[i+1].
 __device__ __forceinline__ const int* rb_rep(const Dev& d) { return d.rb + 2; }
 __device__ __forceinline__ const int* rb_cell_off(const Dev& d) { return d.rb + 2 + d.nrep; }
 __device__ __forceinline__ const int* rb_tile_off(const Dev& d) { return d.rb + 3 + 2 * d.nrep; }
