@@ -2555,25 +2555,19 @@ __device__ __noinline__ void steps_lists(const Dev& d, uint32_t* smem) {
             x.y = __fadd_rn(x.y, __fmul_rn((float)((lo / 3) % 3 - 1), cs[1]));
             x.z = __fadd_rn(x.z, __fmul_rn((float)(lo / 9 - 1), cs[2]));
         };
-        const bool held = total <= STEPS_WIN;
-        if (held)
-            for (int p = threadIdx.x; p < total; p += blockDim.x) candidate(p, ce[p], cx[p]);
-        __syncthreads();
-        int cmax = 0;
-        for (int a = w; a < in; a += TILE / 32) {
-            const int s = ib + a;
+        // atom s against the n candidates held, self its own place among them; cnt:
+        // its entries so far
+        auto scan = [&](int s, int self, int n, int cnt) {
             const float4 xi = d.mir[s];
             const int ti = type_of(xi);
             uint32_t* list = d.nbr + list_index(s, 0, 1, rbeg, rn, d.cap);
-            const int self = nb_off[CODE_ZERO] + a;
-            int cnt = 0;
-            for (int q = 0; q < total; q += 32) {
+            for (int q = 0; q < n; q += 32) {
                 const int p = q + lane;
                 bool hit = false;
                 uint32_t e = 0u;
-                if (p < total) {
-                    float4 x;
-                    if (held) { e = ce[p]; x = cx[p]; } else candidate(p, e, x);
+                if (p < n) {
+                    e = ce[p];
+                    const float4 x = cx[p];
                     const float ex = __fsub_rn(x.x, xi.x), ey = __fsub_rn(x.y, xi.y), ez = __fsub_rn(x.z, xi.z);
                     hit = fmaf(ez, ez, fmaf(ey, ey, fmaf(ex, ex, -__fmul_rn(rl, rl)))) < 0.f && type_of(x) >= ti &&
                           p != self;
@@ -2583,6 +2577,10 @@ __device__ __noinline__ void steps_lists(const Dev& d, uint32_t* smem) {
                 if (hit && k < d.cap) list[(size_t)k * rn] = e;
                 cnt += __popc(got);
             }
+            return cnt;
+        };
+        int cmax = 0;
+        auto finish = [&](int s, int cnt) {
             const int nfill = min(cnt, d.cap);
             if (d.refmode) sort_lists_by_rank(d, s, lane == 0 ? nfill : 0, rbeg, rn);
             if (lane == 0) {
@@ -2593,6 +2591,27 @@ __device__ __noinline__ void steps_lists(const Dev& d, uint32_t* smem) {
                 }
             }
             cmax = max(cmax, cnt);
+        };
+        if (total <= STEPS_WIN) {
+            for (int p = threadIdx.x; p < total; p += blockDim.x) candidate(p, ce[p], cx[p]);
+            __syncthreads();
+            for (int a = w; a < in; a += TILE / 32) finish(ib + a, scan(ib + a, nb_off[CODE_ZERO] + a, total, 0));
+        } else {
+            // crowded cells: a window of the stream at a time, an atom's count so far
+            // in nn
+            for (int w0 = 0; w0 < total; w0 += STEPS_WIN) {
+                const int wn = min(STEPS_WIN, total - w0);
+                __syncthreads();   // the last window's readers are done
+                for (int p = threadIdx.x; p < wn; p += blockDim.x) candidate(w0 + p, ce[p], cx[p]);
+                __syncthreads();
+                for (int a = w; a < in; a += TILE / 32) {
+                    const int s = ib + a;
+                    const int cnt = scan(s, nb_off[CODE_ZERO] + a - w0, wn, w0 ? d.nn[s] : 0);
+                    __syncwarp();   // every lane has read the count
+                    if (w0 + wn == total) finish(s, cnt);
+                    else if (lane == 0) d.nn[s] = cnt;
+                }
+            }
         }
         if (lane == 0 && cmax > 0) atomicMax(&d.rep[r].max_nn, cmax);
     }
