@@ -3,8 +3,7 @@
 //
 // GB300's FP64 pipe takes 64 cycles of a scheduler per warp instruction,
 // however few lanes are active, so k_force_fp64 (a thread per atom, both sides
-// of every pair, about 86 FP64 instructions each, lanes idle where a candidate
-// is outside r_cut) is bound by it.  Here a force pass is two kernels:
+// of every pair, lanes idle where a candidate is outside r_cut) is bound by it.  Here a force pass is two kernels:
 //
 //   k_pair_terms  one thread per pair record: the pair's force, potential and
 //                 virial terms once, from the side of its owner.  Candidates
@@ -26,8 +25,9 @@
 // by binary search in its (ascending) list.  A pair listed by the later atom
 // only (within rounding of the list radius, far outside r_cut) has none.
 //
-// 256,000 atoms, one NVE pass: 3.66 ms with k_force_fp64; 0.39 + 0.21 ms in
-// tree order here, and 0.41 ms more at a rebuild (every ninth step).  23,256
+// 256,000 atoms, one NVE pass in tree order: 3.66 ms with k_force_fp64 as the
+// reference writes the terms, 1.47 with the terms used here; 0.39 + 0.21 ms
+// here, and 0.41 ms more at a rebuild (every ninth step).  23,256
 // atoms in reference order: 0.53 -> 0.14 ms.  k_pair_terms keeps the FP64 pipe
 // busy over 80 % of the time; k_pair_sums waits for its record gathers.
 // (Summing runs of tiles on a second stream beside the next run's terms was
