@@ -774,11 +774,15 @@ int compute_forces_impl(mdgb_engine* e) {
 // An ensemble rebuilds some replica at nearly every step, and one block decides
 // for all of them: us for 20 NVE steps, one launch / launches, replicas of 64
 // atoms 2042 / 2760 at 64, 2748 / 3125 at 150, 3401 / 3365 at 300, 3642 / 3523 at
-// 380; of 27 atoms 2510 / 2602 at 300, 3865 / 3254 at 800.
+// 380; of 27 atoms 2510 / 2602 at 300, 3865 / 3254 at 800.  Against launches in the
+// timed layout, where threads per atom are the engine's choice: of 64 atoms 1947 /
+// 2673 at 60, 2220 / 2292 at 100 (Berendsen T and P 3122 / 2839), 2755 / 2515 at 150.
 constexpr int TUNE_MIN_ATOMS = 4096;   // fewer: threads per atom are not worth measuring
-constexpr int SMALL_MAX_ATOMS = 24576, SMALL_MAX_COUPLED = 12288, SMALL_MAX_REPLICAS = 300;
+constexpr int SMALL_MAX_ATOMS = 24576, SMALL_MAX_COUPLED = 12288, SMALL_MAX_REPLICAS = 300,
+              SMALL_MAX_TUNABLE = 96;
 bool small_size(const mdgb_engine* e) {
-    return e->ntot <= SMALL_MAX_ATOMS && e->nrep <= SMALL_MAX_REPLICAS && !e->dev.pairs &&
+    const bool tunable = e->cfg.threads_per_atom == 0 && e->ntot >= TUNE_MIN_ATOMS && !e->dev.refmode;
+    return e->ntot <= SMALL_MAX_ATOMS && e->nrep <= (tunable ? SMALL_MAX_TUNABLE : SMALL_MAX_REPLICAS) && !e->dev.pairs &&
            e->cfg.rebuild_every == 0 && e->steps_blocks_per_sm > 0 && e->cfg.threads_per_atom <= 1 &&
            !(e->cfg.flags & (MDGB_FLAG_PROFILE | MDGB_FLAG_TRACE | MDGB_FLAG_PERSISTENT));
 }
